@@ -78,15 +78,14 @@ __global__ void __launch_bounds__(kThreads) k_histogram(SampleSource src, GridGe
 constexpr int kScanPer = 4;               // keys (or chunks) per thread and tile
 constexpr int kScanTile = kScanPer * 1024;
 
-// Inclusive block-wide scan (sum or max) of one value per thread of a 1024-thread block; `tmp`
-// holds 32 words of shared memory. Returns this thread's inclusive result and the block total.
-template <bool kMax>
+// Inclusive block-wide sum scan of one value per thread of a 1024-thread block; `tmp` holds 32 words
+// of shared memory. Returns this thread's inclusive result and the block total.
 __device__ __forceinline__ unsigned int block_scan(unsigned int v, unsigned int* tmp, unsigned int& total) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const unsigned int u = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v = kMax ? max(v, u) : v + u;
+        if (lane >= o) v += u;
     }
     if (lane == 31) tmp[w] = v;
     __syncthreads();
@@ -95,17 +94,68 @@ __device__ __forceinline__ unsigned int block_scan(unsigned int v, unsigned int*
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const unsigned int u = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x = kMax ? max(x, u) : x + u;
+            if (lane >= o) x += u;
         }
         tmp[lane] = x;
     }
     __syncthreads();
-    if (w > 0) v = kMax ? max(v, tmp[w - 1]) : v + tmp[w - 1];
+    if (w > 0) v += tmp[w - 1];
     total = tmp[31];
     __syncthreads();
     return v;
 }
 
+// The key whose records hold the start of each chunk: every key writes the chunks that start inside
+// its records [run, run + c).
+__device__ __forceinline__ void mark_chunks(unsigned int* chunk_key, unsigned int chunk_size, unsigned int run,
+                                            unsigned int c, unsigned int key) {
+    for (unsigned long long ch = ((unsigned long long)run + chunk_size - 1) / chunk_size;
+         ch * chunk_size < (unsigned long long)run + c; ++ch)
+        chunk_key[ch] = key;
+}
+
+// Scan of the kScanTile keys from `base`, whose records and K-blocks follow `carry` and `kcarry`
+// earlier ones; returns the tile's totals.
+__device__ __forceinline__ void scan_tile(const unsigned int* __restrict__ counts, int base, int n_keys,
+                                          unsigned int* __restrict__ offsets, unsigned int* __restrict__ cursor,
+                                          unsigned int* __restrict__ kb_offsets, int kb_size,
+                                          unsigned int* __restrict__ chunk_key, int chunk_size, unsigned int carry,
+                                          unsigned int kcarry, unsigned int* tile, unsigned int* ktile,
+                                          unsigned int* tmp, unsigned int& tot, unsigned int& ktot) {
+    const int t = threadIdx.x;
+    const int n = min(kScanTile, n_keys - base);
+    for (int i = t; i < kScanTile; i += 1024) tile[i] = i < n ? counts[base + i] : 0u;
+    __syncthreads();
+    unsigned int c[kScanPer], s = 0, ks = 0;
+#pragma unroll
+    for (int k = 0; k < kScanPer; ++k) {
+        c[k] = tile[kScanPer * t + k];
+        s += c[k];
+        ks += (c[k] + kb_size - 1) / kb_size;
+    }
+    tot = ktot = 0;
+    const unsigned int incl = block_scan(s, tmp, tot);
+    const unsigned int kincl = kb_offsets ? block_scan(ks, tmp, ktot) : 0u;
+    unsigned int run = carry + incl - s, krun = kcarry + kincl - ks;
+#pragma unroll
+    for (int k = 0; k < kScanPer; ++k) {
+        if (chunk_key && c[k])
+            mark_chunks(chunk_key, (unsigned int)chunk_size, run, c[k], (unsigned int)(base + kScanPer * t + k));
+        tile[kScanPer * t + k] = run;
+        run += c[k];
+        ktile[kScanPer * t + k] = krun;
+        krun += (c[k] + kb_size - 1) / kb_size;
+    }
+    __syncthreads();
+    for (int i = t; i < n; i += 1024) {
+        offsets[base + i] = tile[i];
+        cursor[base + i] = tile[i];
+        if (kb_offsets) kb_offsets[base + i] = ktile[i];
+    }
+    __syncthreads();
+}
+
+// One block over all keys.
 __global__ void __launch_bounds__(1024) k_scan(const unsigned int* __restrict__ counts, int n_keys,
                                               unsigned int* __restrict__ offsets,
                                               unsigned int* __restrict__ cursor,
@@ -114,83 +164,66 @@ __global__ void __launch_bounds__(1024) k_scan(const unsigned int* __restrict__ 
     __shared__ __align__(16) unsigned int tile[kScanTile];
     __shared__ __align__(16) unsigned int ktile[kScanTile];
     __shared__ unsigned int tmp[32];
-    const int t = threadIdx.x;
     unsigned int carry = 0, kcarry = 0;
-    if (chunk_key) {  // chunks are marked below: clear the table first (needs the record total)
-        unsigned int sum = 0, total = 0;
-        for (int k = t; k < n_keys; k += 1024) sum += counts[k];
-        block_scan<false>(sum, tmp, total);
-        const unsigned int n_chunks = (total + chunk_size - 1) / chunk_size;
-        for (unsigned int ch = t; ch < n_chunks; ch += 1024) chunk_key[ch] = 0u;
-        __syncthreads();
-    }
     for (int base = 0; base < n_keys; base += kScanTile) {
-        const int n = min(kScanTile, n_keys - base);
-        for (int i = t; i < kScanTile; i += 1024) tile[i] = i < n ? counts[base + i] : 0u;
-        __syncthreads();
-        unsigned int c[kScanPer], s = 0, ks = 0;
-#pragma unroll
-        for (int k = 0; k < kScanPer; ++k) {
-            c[k] = tile[kScanPer * t + k];
-            s += c[k];
-            ks += (c[k] + kb_size - 1) / kb_size;
-        }
-        unsigned int tot = 0, ktot = 0;
-        const unsigned int incl = block_scan<false>(s, tmp, tot);
-        const unsigned int kincl = kb_offsets ? block_scan<false>(ks, tmp, ktot) : 0u;
-        unsigned int run = carry + incl - s, krun = kcarry + kincl - ks;
-#pragma unroll
-        for (int k = 0; k < kScanPer; ++k) {
-            const int key = base + kScanPer * t + k;
-            if (chunk_key && c[k] && key < n_keys) {  // the first chunk that starts inside this key's records
-                const unsigned int ch = (run + chunk_size - 1) / chunk_size;
-                if ((unsigned long long)ch * chunk_size < (unsigned long long)run + c[k]) chunk_key[ch] = (unsigned int)key;
-            }
-            tile[kScanPer * t + k] = run;
-            run += c[k];
-            ktile[kScanPer * t + k] = krun;
-            krun += (c[k] + kb_size - 1) / kb_size;
-        }
-        __syncthreads();
-        for (int i = t; i < n; i += 1024) {
-            offsets[base + i] = tile[i];
-            cursor[base + i] = tile[i];
-            if (kb_offsets) kb_offsets[base + i] = ktile[i];
-        }
+        unsigned int tot, ktot;
+        scan_tile(counts, base, n_keys, offsets, cursor, kb_offsets, kb_size, chunk_key, chunk_size, carry, kcarry, tile,
+                  ktile, tmp, tot, ktot);
         carry += tot;
         kcarry += ktot;
-        __syncthreads();
     }
-    if (t == 0) {
+    if (threadIdx.x == 0) {
         offsets[n_keys] = carry;
         if (kb_offsets) kb_offsets[n_keys] = kcarry;
     }
-    if (!chunk_key) return;
-    // chunks without a mark start inside the key of the last mark before them: a running maximum
-    // (keys increase along the records), in tiles with a carry
-    __syncthreads();
-    const unsigned int n_chunks = (carry + chunk_size - 1) / chunk_size;
-    unsigned int mcarry = 0;
-    for (unsigned int base = 0; base < n_chunks; base += kScanTile) {
-        const unsigned int n = min((unsigned int)kScanTile, n_chunks - base);
-        for (unsigned int i = t; i < (unsigned int)kScanTile; i += 1024) tile[i] = i < n ? chunk_key[base + i] : 0u;
-        __syncthreads();
-        unsigned int v[kScanPer], m = 0;
+}
+
+// Many keys: a block per kScanTile keys, in two launches. The first writes each block's record and
+// K-block totals; in the second every block adds up its predecessors' totals and scans its own tile.
+// (147,456 keys of a 3072^2 grid at 8 x 8 tiles: 36 tiles one after another would take ~60 us.)
+__global__ void __launch_bounds__(1024) k_scan_sums(const unsigned int* __restrict__ counts, int n_keys, int kb_size,
+                                                   unsigned int* __restrict__ sums) {
+    __shared__ unsigned int tmp[32];
+    const int base = blockIdx.x * kScanTile;
+    unsigned int s = 0, ks = 0;
 #pragma unroll
-        for (int k = 0; k < kScanPer; ++k) {
-            m = max(m, tile[kScanPer * t + k]);
-            v[k] = m;
-        }
-        unsigned int tot = 0;
-        ktile[t] = block_scan<true>(m, tmp, tot);  // inclusive maximum over threads 0..t
-        __syncthreads();
-        const unsigned int before = max(mcarry, t ? ktile[t - 1] : 0u);
-#pragma unroll
-        for (int k = 0; k < kScanPer; ++k) tile[kScanPer * t + k] = max(before, v[k]);
-        __syncthreads();
-        for (unsigned int i = t; i < n; i += 1024) chunk_key[base + i] = tile[i];
-        mcarry = max(mcarry, tot);
-        __syncthreads();
+    for (int k = 0; k < kScanPer; ++k) {
+        const int i = base + k * 1024 + (int)threadIdx.x;
+        const unsigned int c = i < n_keys ? counts[i] : 0u;
+        s += c;
+        ks += (c + kb_size - 1) / kb_size;
+    }
+    unsigned int tot = 0, ktot = 0;
+    block_scan(s, tmp, tot);
+    block_scan(ks, tmp, ktot);
+    if (threadIdx.x == 0) {
+        sums[2 * blockIdx.x] = tot;
+        sums[2 * blockIdx.x + 1] = ktot;
+    }
+}
+
+__global__ void __launch_bounds__(1024) k_scan_tiles(const unsigned int* __restrict__ counts, int n_keys,
+                                                    const unsigned int* __restrict__ sums,
+                                                    unsigned int* __restrict__ offsets,
+                                                    unsigned int* __restrict__ cursor,
+                                                    unsigned int* __restrict__ kb_offsets, int kb_size,
+                                                    unsigned int* __restrict__ chunk_key, int chunk_size) {
+    __shared__ __align__(16) unsigned int tile[kScanTile];
+    __shared__ __align__(16) unsigned int ktile[kScanTile];
+    __shared__ unsigned int tmp[32];
+    unsigned int s = 0, ks = 0, carry = 0, kcarry = 0;
+    for (int b = threadIdx.x; b < (int)blockIdx.x; b += 1024) {
+        s += sums[2 * b];
+        ks += sums[2 * b + 1];
+    }
+    block_scan(s, tmp, carry);
+    block_scan(ks, tmp, kcarry);
+    unsigned int tot, ktot;
+    scan_tile(counts, blockIdx.x * kScanTile, n_keys, offsets, cursor, kb_offsets, kb_size, chunk_key, chunk_size, carry,
+              kcarry, tile, ktile, tmp, tot, ktot);
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+        offsets[n_keys] = carry + tot;
+        if (kb_offsets) kb_offsets[n_keys] = kcarry + ktot;
     }
 }
 
@@ -476,10 +509,21 @@ int launch_histogram(const SampleSource& src, const GridGeom& g, const SlabParam
     return SVDI_OK;
 }
 
+size_t scan_sums_words(long long n_keys) { return 2 * (size_t)((n_keys + kScanTile - 1) / kScanTile); }
+
 int launch_scan(const unsigned int* d_counts, int n_keys, unsigned int* d_offsets,
                 unsigned int* d_cursor, cudaStream_t st, unsigned int* d_kb_offsets, int kb_size,
-                unsigned int* d_chunk_key, int chunk_size) {
-    k_scan<<<1, 1024, 0, st>>>(d_counts, n_keys, d_offsets, d_cursor, d_kb_offsets, kb_size, d_chunk_key, chunk_size);
+                unsigned int* d_chunk_key, int chunk_size, unsigned int* d_sums) {
+    if (!d_sums || n_keys <= kScanTile) {
+        k_scan<<<1, 1024, 0, st>>>(d_counts, n_keys, d_offsets, d_cursor, d_kb_offsets, kb_size, d_chunk_key, chunk_size);
+        SVDI_LAUNCHED();
+        return SVDI_OK;
+    }
+    const int blocks = (n_keys + kScanTile - 1) / kScanTile;
+    k_scan_sums<<<blocks, 1024, 0, st>>>(d_counts, n_keys, kb_size, d_sums);
+    SVDI_LAUNCHED();
+    k_scan_tiles<<<blocks, 1024, 0, st>>>(d_counts, n_keys, d_sums, d_offsets, d_cursor, d_kb_offsets, kb_size,
+                                          d_chunk_key, chunk_size);
     SVDI_LAUNCHED();
     return SVDI_OK;
 }

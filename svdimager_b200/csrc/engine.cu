@@ -165,7 +165,7 @@ struct svdi_engine {
     // intermediates
     svdi::DevBuf vr, vi, q, s, vin64, vin32, stats, partial, counts, offsets, cursor, dropped, rec,
         rec_s, planes, corr, image, cheb_err, bin_out, grid_keep, tc_status, kb_offsets, acc, chunk_key, keymax,
-        plan_buf;
+        plan_buf, scan_sums;
     size_t sz_vr = 0, sz_q = 0, sz_s = 0, sz_off = 0, sz_rec = 0, sz_rec_s = 0, sz_grid = 0, sz_mom = 0;
     const float* cur_vr = nullptr;
     const float* cur_vi = nullptr;
@@ -522,6 +522,21 @@ void tc_tiles(int gridder, GridGeom& g) {
     }
 }
 
+// Whether the FP32 gridder of an automatic tile size runs as the matrix-instruction form
+// (gridder_mma.cu, 8 x 8 tiles): supports its footprint registers hold, and tile keys within the
+// engine's limit.
+bool use_mma_gridder(const svdi_options& o, long long G, int nslab) {
+    if (o.gridder != SVDI_GRIDDER_FP32 && !is_tc_gridder(o.gridder)) return false;
+    const long long nt = (G + kMmaTile - 1) / kMmaTile;
+    return o.tile == 0 && o.support <= 8 && (long long)nslab * nt * nt <= (1LL << 26);
+}
+
+// Tile geometry of the FP32 gridder forms (the grid size g.G set).
+void fp32_tiles(int T, GridGeom& g) {
+    g.T = g.T2 = T;
+    g.ntile = g.ntile2 = (int)((g.G + T - 1) / T);
+}
+
 long long grid_size(long long N, double sigma) {
     if (sigma == 1.5) return (3 * N + 1) / 2;  // ceil(1.5 N), SVDIntegratedImager.cu:1510
     return next_nice_even((long long)std::ceil(sigma * (double)N - 1e-9));
@@ -675,13 +690,12 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
     // the integer form scales each key by its own max |value| from the scatter
     const bool use_tc = is_tc_gridder(o.gridder) && (sp.K == 1 || o.gridder == SVDI_GRIDDER_TC_I8) && g.W <= 8;
     const bool use_i8 = use_tc && o.gridder == SVDI_GRIDDER_TC_I8;
+    const bool use_mma = !use_tc && use_mma_gridder(o, g.G, sp.nslab);
+    const int chunk = use_mma ? mma_chunk(n) : kGridChunk;  // records per chunk of the scan's table
     if (use_tc) {
         tc_tiles(o.gridder, g);
     } else {
-        g.T = o.tile ? o.tile : (sp.K == 1 ? 64 : 32);
-        g.ntile = (int)((g.G + g.T - 1) / g.T);
-        g.T2 = g.T;
-        g.ntile2 = g.ntile;
+        fp32_tiles(use_mma ? kMmaTile : (o.tile ? o.tile : (sp.K == 1 ? 64 : 32)), g);
     }
     g.edge_mode = o.edge_mode;
     g.coord_mode = o.coord_mode;
@@ -718,10 +732,11 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
                               e->dropped.as<unsigned long long>(), st, dplan));
     if (use_tc) {
         SVDI_TRY(e->kb_offsets.ensure((size_t)(n_keys + 1) * 4));
-    } else {  // the FP32 gridder's chunk table
-        SVDI_TRY(e->chunk_key.ensure(((size_t)std::max<long long>(n, 1) / kGridChunk + 2) * 4));
+    } else {  // the FP32 gridders' chunk table, then the work counter
+        SVDI_TRY(e->chunk_key.ensure(((size_t)std::max<long long>(n, 1) / chunk + 2) * 4));
     }
-    const bool need_keymax = !use_tc || use_i8;  // per-key max |value| (FP32 and integer gridders)
+    SVDI_TRY(e->scan_sums.ensure(scan_sums_words(n_keys) * 4));
+    const bool need_keymax = use_i8 || (!use_tc && !use_mma);  // per-key max |value| (fixed-point gridders)
     if (need_keymax) {
         SVDI_TRY(e->keymax.ensure((size_t)n_keys * 4));
         SVDI_CUDA(cudaMemsetAsync(e->keymax.p, 0, (size_t)n_keys * 4, st));
@@ -729,7 +744,8 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
     SVDI_TRY(launch_scan(e->counts.as<unsigned int>(), n_keys, e->offsets.as<unsigned int>(),
                          e->cursor.as<unsigned int>(), st,
                          use_tc ? e->kb_offsets.as<unsigned int>() : nullptr, kTcKBlock,
-                         use_tc ? nullptr : e->chunk_key.as<unsigned int>(), kGridChunk));
+                         use_tc ? nullptr : e->chunk_key.as<unsigned int>(), chunk,
+                         e->scan_sums.as<unsigned int>()));
     // tensor-core gridder: [0] give-up status, [1] max |record value| (float bits) from the scatter
     if (use_tc) {
         SVDI_TRY(e->tc_status.ensure(4 * sizeof(unsigned int)));
@@ -787,11 +803,17 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
                                     s1 * tiles2, s0, g, e->poly, e->planes.as<float2>(),
                                     e->tc_status.as<unsigned int>() + 1, e->tc_status.as<unsigned int>(),
                                     e->sm_count, st, o.gridder == SVDI_GRIDDER_TC_BF16));
+        } else if (use_mma) {
+            SVDI_TRY(launch_grid_mma(e->rec.as<SampleRec>(), need_s ? e->rec_s.as<float>() : nullptr,
+                                     e->offsets.as<unsigned int>(), e->chunk_key.as<unsigned int>(), chunk,
+                                     e->chunk_key.as<unsigned int>() + (size_t)std::max<long long>(n, 1) / chunk + 1,
+                                     n_keys, s0 * tiles2, s1 * tiles2, g, sp.K, e->poly, e->planes.as<float2>(),
+                                     e->sm_count, st));
         } else {
             SVDI_TRY(launch_grid_fp32(e->rec.as<SampleRec>(), need_s ? e->rec_s.as<float>() : nullptr,
                                       e->offsets.as<unsigned int>(), e->chunk_key.as<unsigned int>(),
                                       e->keymax.as<unsigned int>(),
-                                      e->chunk_key.as<unsigned int>() + (size_t)std::max<long long>(n, 1) / kGridChunk + 1,
+                                      e->chunk_key.as<unsigned int>() + (size_t)std::max<long long>(n, 1) / chunk + 1,
                                       n_keys, s0 * tiles2, s1 * tiles2, s0, g,
                                       sp, e->poly, e->planes.as<float2>(), e->sm_count, st));
         }
@@ -1441,7 +1463,7 @@ struct svdi_batch {
     // per Chebyshev order over the keys of all snapshots, one FFT over all moment planes).
     bool wide = false;
     svdi::DevBuf vr, vi, q, s, vin64, vin32, stats, partial, counts, offsets, cursor, keymax, chunk_key,
-        kb_offsets, rec, rec_s, planes, dropped, work, corr;
+        kb_offsets, rec, rec_s, planes, dropped, work, corr, scan_sums;
     svdi::FftPlan fft;
     std::vector<cudaStream_t> lanes;
     std::vector<cudaEvent_t> lane_ev;
@@ -1475,7 +1497,7 @@ namespace svdi {
 namespace {
 
 // Grid geometry of an imaging call (the same rules as image_core).
-GridGeom geom_for(const svdi_options& o, long long N, float cell_f, int K, bool use_tc) {
+GridGeom geom_for(const svdi_options& o, long long N, float cell_f, int K, bool use_tc, bool use_mma) {
     GridGeom g{};
     g.G = grid_size(N, o.sigma);
     g.gmin = -(g.G / 2);
@@ -1484,10 +1506,7 @@ GridGeom geom_for(const svdi_options& o, long long N, float cell_f, int K, bool 
     if (use_tc) {
         tc_tiles(o.gridder, g);
     } else {
-        g.T = o.tile ? o.tile : (K == 1 ? 64 : 32);
-        g.ntile = (int)((g.G + g.T - 1) / g.T);
-        g.T2 = g.T;
-        g.ntile2 = g.ntile;
+        fp32_tiles(use_mma ? kMmaTile : (o.tile ? o.tile : (K == 1 ? 64 : 32)), g);
     }
     g.edge_mode = o.edge_mode;
     g.coord_mode = o.coord_mode;
@@ -1526,7 +1545,7 @@ int wide_capture(svdi_batch* b) {
     const int NG = (int)group_k.size();
     struct Group {
         int K = 1;
-        bool tc = false;
+        bool tc = false, mma = false;
         GridGeom g{};
         long long key_lo = 0, key_hi = 0, slab_lo = 0, plane_lo = 0;
     };
@@ -1534,11 +1553,16 @@ int wide_capture(svdi_batch* b) {
     std::vector<long long> key_base(B), plane_base(B), samp_off(B), row_off(B), chan_off(B);
     long long nkeys = 0, nplanes = 0, ntot = 0, rtot = 0, ctot = 0;
     bool need_s = false, any_tc = false;
+    // one scan table serves all groups, so the FP32 groups use one gridder form
+    long long slabs = 0;
+    for (const auto& p : b->plans) slabs += p.sp.nslab;
+    const bool mma_batch = slabs < (1 << 20) && use_mma_gridder(o, grid_size(N, o.sigma), (int)slabs);
     for (int gi = 0; gi < NG; ++gi) {
         Group& G = groups[gi];
         G.K = group_k[gi];
         G.tc = tc_opt && (G.K == 1 || o.gridder == SVDI_GRIDDER_TC_I8) && o.support <= 8;
-        G.g = geom_for(o, N, cell_f, G.K, G.tc);
+        G.mma = !G.tc && mma_batch;
+        G.g = geom_for(o, N, cell_f, G.K, G.tc, G.mma);
         // the gridders take a key's slab as key / (tiles per slab): start the group on a multiple of
         // its tiles per slab (the keys skipped stay empty)
         const long long tiles2 = (long long)G.g.ntile * G.g.ntile2;
@@ -1567,6 +1591,7 @@ int wide_capture(svdi_batch* b) {
         ctot += (long long)b->snaps[s].num_channels;
     }
     if (nkeys > (1LL << 28) || ntot >= (1LL << 32) - 1) return SVDI_ERR_UNSUPPORTED;
+    const int chunk = mma_batch ? mma_chunk(ntot) : kGridChunk;
     const long long Gs = groups[0].g.G, GG = Gs * Gs;
     size_t free_b = 0, total_b = 0;
     SVDI_CUDA(cudaMemGetInfo(&free_b, &total_b));
@@ -1587,7 +1612,8 @@ int wide_capture(svdi_batch* b) {
     SVDI_TRY(b->offsets.ensure((size_t)(nkeys + 1) * 4));
     SVDI_TRY(b->cursor.ensure((size_t)nkeys * 4));
     SVDI_TRY(b->keymax.ensure((size_t)nkeys * 4));
-    SVDI_TRY(b->chunk_key.ensure(((size_t)std::max<long long>(ntot, 1) / kGridChunk + 2) * 4));
+    SVDI_TRY(b->chunk_key.ensure(((size_t)std::max<long long>(ntot, 1) / chunk + 2) * 4));
+    SVDI_TRY(b->scan_sums.ensure(scan_sums_words(nkeys) * 4));
     if (any_tc) SVDI_TRY(b->kb_offsets.ensure((size_t)(nkeys + 1) * 4));
     SVDI_TRY(b->rec.ensure((size_t)std::max<long long>(ntot, 1) * sizeof(SampleRec)));
     if (need_s) SVDI_TRY(b->rec_s.ensure((size_t)std::max<long long>(ntot, 1) * 4));
@@ -1676,7 +1702,7 @@ int wide_capture(svdi_batch* b) {
         SVDI_TRY(join());
         SVDI_TRY(launch_scan(b->counts.as<unsigned int>(), (int)nkeys, b->offsets.as<unsigned int>(),
                              b->cursor.as<unsigned int>(), st, any_tc ? b->kb_offsets.as<unsigned int>() : nullptr,
-                             kTcKBlock, b->chunk_key.as<unsigned int>(), kGridChunk));
+                             kTcKBlock, b->chunk_key.as<unsigned int>(), chunk, b->scan_sums.as<unsigned int>()));
         // per snapshot: scatter into the global record order
         SVDI_TRY(fork());
         for (size_t s = 0; s < B; ++s) {
@@ -1686,7 +1712,8 @@ int wide_capture(svdi_batch* b) {
             const int nk = (int)((long long)sp.nslab * G.g.ntile * G.g.ntile2);
             SVDI_TRY(launch_scatter(source(s), G.g, sp, b->cursor.as<unsigned int>() + key_base[s], nk,
                                     b->rec.as<SampleRec>(), need_s ? b->rec_s.as<float>() : nullptr,
-                                    G.tc ? vmax : nullptr, ls, b->keymax.as<unsigned int>() + key_base[s]));
+                                    G.tc ? vmax : nullptr, ls,
+                                    G.mma ? nullptr : b->keymax.as<unsigned int>() + key_base[s]));
         }
         SVDI_TRY(join());
         // one gridder launch per Chebyshev order over the records of all its snapshots
@@ -1711,6 +1738,11 @@ int wide_capture(svdi_batch* b) {
                                         b->kb_offsets.as<unsigned int>(), (int)nkeys, (int)G.key_lo, (int)G.key_hi,
                                         (int)G.slab_lo, G.g, e->poly, pl, vmax, stw, e->sm_count, st,
                                         o.gridder == SVDI_GRIDDER_TC_BF16));
+            } else if (G.mma) {
+                SVDI_TRY(launch_grid_mma(b->rec.as<SampleRec>(), need_s ? b->rec_s.as<float>() : nullptr,
+                                         b->offsets.as<unsigned int>(), b->chunk_key.as<unsigned int>(), chunk,
+                                         b->work.as<unsigned int>() + gi, (int)nkeys, (int)G.key_lo, (int)G.key_hi,
+                                         G.g, G.K, e->poly, pl, e->sm_count, st));
             } else {
                 SVDI_TRY(launch_grid_fp32(b->rec.as<SampleRec>(), need_s ? b->rec_s.as<float>() : nullptr,
                                           b->offsets.as<unsigned int>(), b->chunk_key.as<unsigned int>(),

@@ -191,9 +191,13 @@ int launch_histogram(const SampleSource& src, const GridGeom& g, const SlabParam
 // d_kb_offsets (optional): exclusive scan of ceil(count / kb_size) per key, n_keys + 1 entries.
 // d_chunk_key (optional): for every chunk c of chunk_size records, the last key whose records
 // start at or before c * chunk_size (ceil(total / chunk_size) entries, total = offsets[n_keys]).
+// d_sums (optional, scan_sums_words(n_keys) words of scratch): lets several blocks scan a large
+// number of keys; without it one block scans them all.
+size_t scan_sums_words(long long n_keys);
 int launch_scan(const unsigned int* d_counts, int n_keys, unsigned int* d_offsets,
                 unsigned int* d_cursor, cudaStream_t st, unsigned int* d_kb_offsets = nullptr,
-                int kb_size = 32, unsigned int* d_chunk_key = nullptr, int chunk_size = 512);
+                int kb_size = 32, unsigned int* d_chunk_key = nullptr, int chunk_size = 512,
+                unsigned int* d_sums = nullptr);
 // d_vmax (optional, zeroed by the caller): receives max(|vre|, |vim|) over the records as float bits
 // d_keymax (optional, n_keys entries zeroed by the caller): the same maximum per key
 int launch_scatter(const SampleSource& src, const GridGeom& g, const SlabParams& sp,
@@ -288,6 +292,17 @@ int launch_grid_fp32(const SampleRec* d_rec, const float* d_rec_s, const unsigne
                      const SlabParams& sp, const EsPoly& poly, float2* d_planes, int sm_count,
                      cudaStream_t st);
 void build_es_poly(int W, double beta, EsPoly* out);
+
+// gridder_mma.cu: the FP32 gridder on warp-level matrix instructions (support <= 8, 8 x 8 tiles)
+constexpr int kMmaTile = 8;
+// records per chunk of the scan's table for n records (a power of two, at least kMmaChunkMin)
+constexpr int kMmaChunkMin = 64;
+int mma_chunk(long long n);
+// key_lo: the first tile of a slab; its planes come first in d_planes
+int launch_grid_mma(const SampleRec* d_rec, const float* d_rec_s, const unsigned int* d_offsets,
+                    const unsigned int* d_chunk_key, int chunk, unsigned int* d_work, int n_keys, int key_lo,
+                    int key_hi, const GridGeom& g, int K, const EsPoly& poly, float2* d_planes,
+                    int sm_count, cudaStream_t st);
 
 // image.cu
 // d_acc (N x N doubles, zeroed before the first batch) when the slabs are split over several

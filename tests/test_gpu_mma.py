@@ -1,0 +1,75 @@
+"""The matrix-instruction gridder (8 x 8 tiles, automatic tile size, support 6 and 8) against the oracle.
+
+Positions cover what its dispatch and its edges can get wrong: tiles that the grid cuts (G not a
+multiple of 8, odd G), footprints clipped at both grid edges, exactly integer positions, tiles of one
+record and of many (chunks shared by several warps, a tile split over several), neighbouring and
+distant tiles, and every split of the Chebyshev terms over its 4-, 2- and 1-term variants.
+
+Tolerance: a contribution is off by at most (2 * 1.2e-7 + 3 * 2^-22) of the kernel's peak times |v|
+(FP32 piecewise polynomials of both axes; FP16 hi + lo splits of both factors and the dropped lo * lo
+product), about 1e-6; the planes are held to the 4e-6 relative L2 of the other gridders' tests."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from svdimager_b200 import api
+
+pytestmark = pytest.mark.gpu
+
+GRID_TOL = 4e-6
+W_BETA = {8: O.REF_BETA, 6: O.REF_BETA * 0.75}
+
+
+def _samples(rng, n, G, spread):
+    """n positions in grid cells: a dense core, rows of neighbouring tiles, the whole grid and beyond its
+    edges, and some exactly integer ones."""
+    p = np.empty((n, 2))
+    a, b, c = n // 3, n // 2, (9 * n) // 10
+    p[:a] = rng.normal(0.0, spread, (a, 2))
+    p[a:b, 0] = rng.uniform(-1.0, 1.0, b - a)
+    p[a:b, 1] = rng.uniform(-G / 2, G / 2, b - a)
+    p[b:c] = rng.uniform(-1.0, 1.0, (c - b, 2)) * (G / 2 + 3)
+    p[c:] = rng.uniform(-1.0, 1.0, (n - c, 2)) * (G / 2 + 3)
+    p[c::3, 0] = np.round(p[c::3, 0])
+    p[c::4] = np.round(p[c::4])
+    return p
+
+
+def _run(n, N, W, K, seed=3, spread=3.0):
+    cell, G = 2e-3, (3 * N + 1) // 2
+    scale = float(np.float32(cell)) * G
+    rng = np.random.default_rng(seed)
+    b = np.concatenate([_samples(rng, n, G, spread) / scale, rng.uniform(-40.0, 40.0, (n, 1))], axis=1)
+    b = b.astype(np.float32)
+    vr, vi = (rng.normal(size=n).astype(np.float32) for _ in range(2))
+    v = np.eye(3, dtype=np.float32)
+    v[0], v[1] = [0.8, 0.6, 0.0], [-0.6, 0.8, 0.0]
+    opt = dict(coord_mode=api.COORD_REF32, keep_grid=1, k_rule=api.KRULE_FIXED, fixed_k=K, support=W, beta=W_BETA[W])
+    with api.Engine(api.archive_options(**opt)) as e:
+        e.fipipe(vr, vi, b, v, N, cell)
+        st = e.stats()
+        grid = e.buffer(api.BUF_GRID).reshape(K, G, G)
+    assert st["tile"] == 8 and st["num_terms"] == K
+    sc = O.SlabConfig(st["slab_r3_min"], st["r3_max"], st["max_abs_t3"], st["alpha_max"], 1, st["slab_width"],
+                      st["slab_half"], 1.0 / st["slab_half"], st["slab_alpha_max"], K)
+    ref = O.grid(b.astype(np.float64), vr, vi, scale, G, sc, 1.0 / (0.8 * 0.8 + 0.6 * 0.6), W=W, beta=W_BETA[W],
+                 coord_mode=1)
+    return grid, ref
+
+
+@pytest.mark.parametrize("n,N,W,K", [
+    (1, 16, 8, 1), (33, 16, 8, 2), (700, 37, 8, 1), (5000, 100, 8, 3), (5000, 90, 6, 1), (4000, 99, 6, 2),
+    (20000, 64, 8, 4), (9000, 61, 8, 5), (6000, 85, 6, 7), (300, 255, 8, 1)])
+def test_planes_match_oracle(cuda_device, n, N, W, K):
+    grid, ref = _run(n, N, W, K)
+    for k in range(K):
+        den = np.linalg.norm(ref[k])
+        err = np.linalg.norm(grid[k] - ref[k])
+        assert err <= GRID_TOL * den, (k, err, den)
+
+
+@pytest.mark.parametrize("n", [600_000, 2_100_000])
+def test_long_runs_match_oracle(cuda_device, n):
+    """Both chunk sizes (64 and 256 records), most tiles split over many chunks."""
+    grid, ref = _run(n, 48, 8, 1, spread=12.0)
+    assert np.linalg.norm(grid[0] - ref[0]) <= GRID_TOL * np.linalg.norm(ref[0])
