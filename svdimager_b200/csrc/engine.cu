@@ -196,6 +196,8 @@ struct svdi_engine {
     std::map<std::tuple<long long, long long, int, double>, std::vector<float>> corr_cache;
     std::tuple<long long, long long, int, double> corr_key{-1, -1, -1, 0.0};
     std::map<std::tuple<double, int, int>, std::vector<double>> cheb_cache;
+    svdi::EsPoly wpoly{};                // the w axis' kernel and its correction (w planes)
+    double wcorr[svdi::kWCorrTerms] = {};
     svdi::EsPoly poly{};
     int poly_W = -1;
     double poly_beta = 0.0;
@@ -208,7 +210,8 @@ struct svdi_engine {
     long long last_N = 0;
     double last_cell = 0.0;
     bool have_last = false;
-    svdi::DevBuf probe;
+    bool last_w = false;       // it went through w planes: no records or moments of it are held yet
+    svdi::DevBuf probe, remade;
     // pageable host uploads and image downloads of the archive entry and the host-input call
     svdi::HostStager stager;
     bool batch_bound = false;  // a batch's captured graph refers to this engine's buffers
@@ -299,21 +302,22 @@ int cheb_errors(svdi_engine* e, double amax, int na, int ns, std::vector<double>
     return SVDI_OK;
 }
 
-// Upper bound of the Jacobi-Anger truncation error on |s| <= 1 when K terms are kept:
-// 2 sum_{n >= K} |J_n(a)| (|T_n| <= 1).
-double truncation_bound(double a, int K) {
-    double j[200];
-    const int nmax = std::min(199, K + 60 + (int)std::fabs(a));
-    bessel_jn(a, nmax, j);
-    double s = 0.0;
-    for (int n = K; n <= nmax; ++n) s += std::fabs(j[n]);
-    return 2.0 * s;
-}
-
+// Smallest K whose Jacobi-Anger truncation error on |s| <= 1, bounded by 2 sum_{n >= K} |J_n(a)| (|T_n| <=
+// 1), is at most `target`; -1 when more than kMaxTerms are needed. One Bessel evaluation: the tail sums from
+// the largest order down (one per K made the wide-field decision 30 times as long).
 int k_for_target(double a, double target) {
-    for (int K = 1; K <= kMaxTerms; ++K)
-        if (truncation_bound(a, K) <= target) return K;
-    return -1;
+    double j[200];
+    const int nmax = std::min(199, kMaxTerms + 60 + (int)std::fabs(a));
+    bessel_jn(a, nmax, j);
+    int K = -1;
+    double s = 0.0;
+    for (int n = nmax; n >= 1; --n) {
+        s += std::fabs(j[n]);
+        if (n > kMaxTerms) continue;
+        if (2.0 * s > target) break;
+        K = n;
+    }
+    return K;
 }
 
 // Slab / Chebyshev configuration from the device statistics.
@@ -330,7 +334,7 @@ int choose_slabs(svdi_engine* e, bool archive, double r3min, double r3max, doubl
             // equal plane counts take the smallest K (a sample is gridded into K planes of its slab,
             // so fewer terms and more slabs grid the same planes with less work)
             int best_n = 1, best_p = 1 << 30;
-            for (int n = 1; n <= 64; ++n) {
+            for (int n = 1; n <= std::min(64, best_p); ++n) {  // n slabs need at least n planes
                 const double h = std::max(0.5 * r3_range / n, 1.0e-6);
                 const int K = k_for_target(2.0 * kPi * mt3 * h, o.target_error);
                 if (K < 0) continue;
@@ -567,6 +571,71 @@ size_t batch_slabs_for(svdi_engine* e, int nslab, int K, long long G) {
     return b;
 }
 
+// Moment planes from which the error-target rule images through w planes instead (wplanes.cu).
+constexpr int kWPlanesMin = 48;
+
+// ES transform psi^(k) = integral of psi(x / (W / 2)) cos(2 pi k x) over the support, composite
+// Gauss-Legendre quadrature.
+double es_transform(int W, double beta, double k) {
+    static const double x8[4] = {0.1834346424956498, 0.5255324099163290, 0.7966664774136267, 0.9602898564975363};
+    static const double w8[4] = {0.3626837833783620, 0.3137066458778873, 0.2223810344533745, 0.1012285362903763};
+    const double hw = 0.5 * W;
+    auto f = [&](double x) {
+        return std::exp(-beta * x * x / (1.0 + std::sqrt((1.0 - x) * (1.0 + x)))) * std::cos(2.0 * kPi * k * hw * x);
+    };
+    const int panels = 48;  // 384 nodes on [0, 1]
+    double acc = 0.0;
+    for (int p = 0; p < panels; ++p) {
+        const double mid = (p + 0.5) / panels, h = 0.5 / panels;
+        for (int j = 0; j < 4; ++j) acc += w8[j] * h * (f(mid - h * x8[j]) + f(mid + h * x8[j]));
+    }
+    return 2.0 * hw * acc;
+}
+
+// The w-plane geometry of a call with r3 in [r3min, r3max] and |t3| <= mt3, or false when the call
+// images through Chebyshev moments: other rules than the error target (their truncation is part of the
+// result), other gridders, few moment planes (measured: at 48 and more the w planes are faster on every
+// grid tried, from 1.2x at 48 to 2.5x at 236), no fewer w planes than 3/4 of them, odd grid sizes (the
+// reference's indexing of those does not commute with the mirrored samples).
+bool plan_wplanes(svdi_engine* e, const SampleSource& src, long long G, const SlabParams& sp, double r3min,
+                  double r3max, double mt3, WPlanes& wp) {
+    const svdi_options& o = e->opt;
+    if (o.k_rule != SVDI_KRULE_TARGET || o.target_error < 1e-8 || o.gridder != SVDI_GRIDDER_FP32 || o.tile != 0 ||
+        (o.support != 6 && o.support != 8) || o.keep_grid || src.bin || (G & 1) || sp.nslab * sp.K < kWPlanesMin ||
+        !(mt3 > 0.0) || src.R <= 0 || src.n % src.R || G < 32)
+        return false;
+    // largest error over the band of kernels with beta = 2.06 W at sigma = 1.5 (|t3| dw <= 1/3): 2e-7
+    // at W = 10, 7e-9 at W = 12
+    wp.W = o.target_error >= 2e-7 ? 10 : 12;
+    wp.beta_xy = (float)o.beta;
+    const double hi = std::max(std::fabs(r3min), std::fabs(r3max));
+    wp.lo = (r3min <= 0.0 && r3max >= 0.0) ? 0.0 : std::min(std::fabs(r3min), std::fabs(r3max));
+    wp.dw = 1.0 / (2.0 * 1.5 * mt3);
+    wp.inv_dw = 1.0 / wp.dw;
+    const double span = std::floor((hi - wp.lo) * wp.inv_dw * (1.0 + 1e-12)) + wp.W;
+    if (!(span <= 0.75 * sp.nslab * sp.K)) return false;
+    wp.P = (int)span;
+    wp.kmax = mt3 * wp.dw;
+    const double beta = 2.06 * wp.W;
+    if (e->wpoly.W != wp.W) {
+        build_es_poly(wp.W, beta, &e->wpoly);
+        // Chebyshev coefficients of 1 / psi^ in 2 (k / kmax)^2 - 1 (kmax = 1/3)
+        const int n = kWCorrTerms;
+        double v[kWCorrTerms];
+        for (int i = 0; i < n; ++i) {
+            const double z = std::cos(kPi * (i + 0.5) / n);
+            v[i] = 1.0 / es_transform(wp.W, beta, wp.kmax * std::sqrt(0.5 * (z + 1.0)));
+        }
+        for (int j = 0; j < n; ++j) {
+            double c = 0.0;
+            for (int i = 0; i < n; ++i) c += v[i] * std::cos(kPi * j * (i + 0.5) / n);
+            e->wcorr[j] = (j ? 2.0 : 1.0) * c / n;
+        }
+    }
+    std::memcpy(wp.corr, e->wcorr, sizeof(wp.corr));
+    return true;
+}
+
 // The host decisions of one snapshot: everything image_core reads back from the device before
 // it can launch the gridding (basis determinant, w range, slab and Chebyshev configuration,
 // slabs per batch). With a fixed plan image_core issues device work only (no synchronisation,
@@ -630,11 +699,124 @@ int host_decision(svdi_engine* e, bool archive, SampleSource& src, SlabParams& s
     return choose_slabs(e, archive, r3min, r3max, mt3, sp, alpha_max, slab_alpha);
 }
 
+// The statistics of a call that both forms of image_core report.
+void record_call(svdi_engine* e, const SampleSource& src, const GridGeom& g, const SlabParams& sp, long long N,
+                 double cell) {
+    e->last_src = src;
+    e->last_g = g;
+    e->last_sp = sp;
+    e->last_N = N;
+    e->last_cell = cell;
+    e->have_last = true;
+}
+void record_stats(svdi_engine* e, const SampleSource& src, const GridGeom& g, const SlabParams& sp, int n_keys,
+                  bool use_tc, double alpha_max, double slab_alpha, double r3min, double r3max, double mt3) {
+    e->cur_vr = src.vr;
+    e->cur_vi = src.vi;
+    e->sz_vr = (size_t)src.n * 4;
+    e->cur_q = src.q;
+    e->cur_s = src.s;
+    svdi_stats& L = e->last;
+    L.tile = g.T;
+    L.tile_cols = g.T2;
+    L.used_tc = use_tc ? 1 : 0;
+    L.num_keys = n_keys;
+    L.slab_r3_min = sp.r3_min;
+    L.slab_width = sp.slab_width;
+    L.slab_half = sp.slab_half;
+    L.num_samples = (size_t)src.n;
+    L.grid_size = (size_t)g.G;
+    L.num_slabs = sp.nslab;
+    L.num_terms = sp.K;
+    L.num_planes = sp.nslab * sp.K;
+    L.r3_min = r3min;
+    L.r3_max = r3max;
+    L.max_abs_t3 = mt3;
+    L.valid_pixels = (size_t)e->h_stats[ST_VALID_PIX];
+    L.alpha_max = alpha_max;
+    L.slab_alpha_max = slab_alpha;
+}
+
+// The imaging of one call through w planes (plan_wplanes), as many planes at a time as the memory rule of
+// the Chebyshev batches allows. The statistics report the Chebyshev configuration that the error target
+// asks for (sp); the records, the grid and the moments of it are made when they are asked for
+// (materialise_moments).
+int image_wplanes(svdi_engine* e, SampleSource src, const GridGeom& g, const SlabParams& sp, const WPlanes& wp,
+                  long long N, double cell, float* d_out, cudaEvent_t vis_ready, double alpha_max, double slab_alpha,
+                  double r3min, double r3max, double mt3) {
+    cudaStream_t st = e->stream;
+    e->spec_valid = false;
+    if (e->poly_W != g.W || e->poly_beta != e->opt.beta) {
+        build_es_poly(g.W, e->opt.beta, &e->poly);
+        e->poly_W = g.W;
+        e->poly_beta = e->opt.beta;
+    }
+    const size_t plane_bytes = (size_t)g.G * g.G * sizeof(float2);
+    const size_t bslabs = batch_slabs_for(e, sp.nslab, sp.K, g.G);
+    const int per = (int)std::min<size_t>((size_t)wp.P, bslabs * (size_t)sp.K);
+    SVDI_TRY(e->planes.ensure(plane_bytes * per));
+    SVDI_TRY(e->dropped.ensure(16));
+    SVDI_CUDA(cudaEventRecord(e->ev[1], st));
+    SVDI_CUDA(cudaMemsetAsync(e->dropped.p, 0, 16, st));
+    src.nonfinite = e->dropped.as<unsigned long long>() + 1;
+    SVDI_CUDA(cudaEventRecord(e->ev[2], st));
+    SVDI_TRY(ensure_corr(e, N, g.G, g.W, e->opt.beta));
+    SVDI_CUDA(cudaMemsetAsync(d_out, 0, (size_t)N * N * sizeof(float), st));
+    const bool multi = per < wp.P;
+    if (multi) {
+        SVDI_TRY(e->acc.ensure((size_t)N * N * sizeof(double)));
+        SVDI_CUDA(cudaMemsetAsync(e->acc.p, 0, (size_t)N * N * sizeof(double), st));
+    }
+    float ms[3] = {0, 0, 0};  // gridding, FFT, recombination
+    for (int lo = 0; lo < wp.P; lo += per) {
+        const int hi = std::min(wp.P, lo + per);
+        FftPlan plan;
+        SVDI_TRY(get_plan(e, g.G, N, hi - lo, plan));
+        SVDI_CUDA(cudaEventRecord(e->ev[3], st));
+        SVDI_CUDA(cudaMemsetAsync(e->planes.p, 0, plane_bytes * (hi - lo), st));
+        if (lo == 0 && vis_ready) SVDI_CUDA(cudaStreamWaitEvent(st, vis_ready, 0));
+        SVDI_TRY(launch_grid_w(src, g, wp, e->poly, e->wpoly, lo, hi, e->planes.as<float2>(),
+                               lo == 0 ? e->dropped.as<unsigned long long>() : nullptr, st));
+        SVDI_CUDA(cudaEventRecord(e->ev[4], st));
+        SVDI_TRY(exec_fft(plan, e->planes.as<cufftComplex>(), hi - lo));
+        SVDI_CUDA(cudaEventRecord(e->ev[5], st));
+        SVDI_TRY(launch_recombine_w(e->planes.as<float2>(), g, N, cell, e->vin64.as<double>(), wp, lo, hi,
+                                    e->corr.as<float>(), 1.0 / (double)src.n, e->opt.reprojection, e->opt.presplat,
+                                    d_out, st, multi ? e->acc.as<double>() : nullptr, hi == wp.P, src.nonfinite));
+        SVDI_CUDA(cudaEventRecord(e->ev[6], st));
+        if (!multi) continue;  // one batch: its stage times are read when the call completes
+        SVDI_CUDA(cudaEventSynchronize(e->ev[6]));
+        for (int k = 0; k < 3; ++k) {
+            float t = 0;
+            cudaEventElapsedTime(&t, e->ev[3 + k], e->ev[4 + k]);
+            ms[k] += t;
+        }
+    }
+    SVDI_CUDA(cudaMemcpyAsync(e->h_ndrop, e->dropped.p, 8, cudaMemcpyDeviceToHost, st));
+    record_call(e, src, g, sp, N, cell);
+    record_stats(e, src, g, sp, sp.nslab * g.ntile * g.ntile2, false, alpha_max, slab_alpha, r3min, r3max, mt3);
+    e->pending = true;
+    e->pending_times = !multi;
+    if (multi) {
+        e->last.ms_bin = 0;
+        e->last.ms_grid = ms[0];
+        e->last.ms_fft = ms[1];
+        e->last.ms_image = ms[2];
+    }
+    e->pending_total = false;
+    e->pending_need_s = sp.K > 1;
+    e->pending_n = src.n;
+    e->sz_off = (size_t)(sp.nslab * g.ntile * g.ntile2 + 1) * 4;
+    e->sz_mom = plane_bytes * bslabs * (size_t)sp.K;
+    return SVDI_OK;
+}
+
 // vis_ready (optional): event after which src.vr / src.vi hold the collapsed visibilities; only
 // the scatter reads them.
 int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, float cell_f,
                float* d_out, const ExecPlan* fixed = nullptr, ExecPlan* record = nullptr,
-               unsigned int* d_status_out = nullptr, cudaEvent_t vis_ready = nullptr, bool allow_spec = true) {
+               unsigned int* d_status_out = nullptr, cudaEvent_t vis_ready = nullptr, bool allow_spec = true,
+               bool allow_w = true) {
     cudaStream_t st = e->stream;
     const svdi_options& o = e->opt;
     const double cell = (double)cell_f;
@@ -713,6 +895,11 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
         e->poly_W = g.W;
         e->poly_beta = o.beta;
     }
+
+    WPlanes wp{};
+    e->last_w = timed && !record && !dplan && allow_w && !use_tc && plan_wplanes(e, src, g.G, sp, r3min, r3max, mt3, wp);
+    if (e->last_w)
+        return image_wplanes(e, src, g, sp, wp, N, cell, d_out, vis_ready, alpha_max, slab_alpha, r3min, r3max, mt3);
 
     // binning
     if (timed) SVDI_CUDA(cudaEventRecord(e->ev[1], st));
@@ -855,7 +1042,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
         }
         if (real.nslab != sp.nslab || real.K != sp.K) {  // other counts: image again with them
             e->spec_valid = false;
-            return image_core(e, archive, src, N, cell_f, d_out, nullptr, nullptr, d_status_out, vis_ready, false);
+            return image_core(e, archive, src, N, cell_f, d_out, nullptr, nullptr, d_status_out, vis_ready, false, allow_w);
         }
         sp = real;  // the same bits as the device plan (slab_params_for, basis_det)
     }
@@ -869,12 +1056,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
         e->spec_R = src.R;
         e->spec_sp = sp;
     }
-    e->last_src = src;
-    e->last_g = g;
-    e->last_sp = sp;
-    e->last_N = N;
-    e->last_cell = cell;
-    e->have_last = true;
+    record_call(e, src, g, sp, N, cell);
     if (!timed) {
         if (d_status_out) {
             if (use_tc)
@@ -912,30 +1094,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
 
     e->sz_off = (size_t)(n_keys + 1) * 4;
     e->sz_mom = plane_bytes * (size_t)planes_per_batch;
-    e->cur_vr = src.vr;
-    e->cur_vi = src.vi;
-    e->sz_vr = (size_t)n * 4;
-    e->cur_q = src.q;
-    e->cur_s = src.s;
-    svdi_stats& L = e->last;
-    L.tile = g.T;
-    L.tile_cols = g.T2;
-    L.used_tc = use_tc ? 1 : 0;
-    L.num_keys = n_keys;
-    L.slab_r3_min = sp.r3_min;
-    L.slab_width = sp.slab_width;
-    L.slab_half = sp.slab_half;
-    L.num_samples = (size_t)n;
-    L.grid_size = (size_t)g.G;
-    L.num_slabs = sp.nslab;
-    L.num_terms = sp.K;
-    L.num_planes = sp.nslab * sp.K;
-    L.r3_min = r3min;
-    L.r3_max = r3max;
-    L.max_abs_t3 = mt3;
-    L.valid_pixels = (size_t)e->h_stats[ST_VALID_PIX];
-    L.alpha_max = alpha_max;
-    L.slab_alpha_max = slab_alpha;
+    record_stats(e, src, g, sp, n_keys, use_tc, alpha_max, slab_alpha, r3min, r3max, mt3);
     return SVDI_OK;
 }
 
@@ -1257,6 +1416,20 @@ int svdi_engine_last_stats(const svdi_engine* e, svdi_stats* out) {
     return SVDI_OK;
 }
 
+// The records and moment planes of a last call that went through w planes: its Chebyshev form, run again on
+// the inputs that are still resident (into a scratch image).
+static int materialise_moments(svdi_engine* e, int which) {
+    if (!e->last_w || which < SVDI_BUF_OFFSETS || which == SVDI_BUF_GRID) return SVDI_OK;
+    const svdi_stats kept = e->last;
+    const size_t N = (size_t)e->last_N;
+    SVDI_TRY(e->remade.ensure(N * N * sizeof(float)));
+    SVDI_TRY(image_core(e, false, e->last_src, (long long)N, (float)e->last_cell, e->remade.as<float>(), nullptr, nullptr,
+                        nullptr, nullptr, false, false));
+    SVDI_TRY(finish_pending(e));
+    e->last = kept;
+    return SVDI_OK;
+}
+
 static int buffer_of(const svdi_engine* e, int which, const void** p, size_t* bytes) {
     switch (which) {
         case SVDI_BUF_VIS_REAL: *p = e->cur_vr; *bytes = e->cur_vr ? e->sz_vr : 0; return SVDI_OK;
@@ -1284,6 +1457,7 @@ int svdi_engine_buffer_size(const svdi_engine* e, int which, size_t* bytes) {
     std::lock_guard<std::mutex> lk(m->mu);
     SVDI_CUDA(cudaSetDevice(m->device));
     SVDI_TRY(finish_pending(m));
+    SVDI_TRY(materialise_moments(m, which));
     const void* p = nullptr;
     return buffer_of(e, which, &p, bytes);
 }
@@ -1296,6 +1470,7 @@ int svdi_engine_copy_buffer(svdi_engine* e, int which, void* host_dst, size_t by
     std::lock_guard<std::mutex> lk(e->mu);
     SVDI_CUDA(cudaSetDevice(e->device));
     SVDI_TRY(finish_pending(e));
+    SVDI_TRY(materialise_moments(e, which));
     const void* p = nullptr;
     size_t have = 0;
     SVDI_TRY(buffer_of(e, which, &p, &have));

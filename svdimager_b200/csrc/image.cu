@@ -109,6 +109,47 @@ __device__ inline SplatTarget reproject_fipk(long long idx, long long idy, long 
     return {oi0 - (double)half, oi1 - (double)half, true};
 }
 
+// From the sum over planes at pixel (x, y) to the image: checkerboard, grid correction, slab batches,
+// |.| / N_s, reprojection and bilinear splat.
+__device__ __forceinline__ void finish_pixel(long long x, long long y, double sum, long long N, double cell,
+                                             const double* V, const float* __restrict__ corr, double inv_n,
+                                             int reprojection, int presplat, float* __restrict__ out,
+                                             double* __restrict__ acc, int final_batch, bool bad,
+                                             const ReprojConst& kc) {
+    const long long half = N / 2;
+    const long long xr = x - half, yr = y - half;
+    if ((xr + yr) & 1) sum = -sum;
+    const long long ax = xr < 0 ? -xr : xr, ay = yr < 0 ? -yr : yr;
+    double signed_sum = sum * (double)corr[ax] * (double)corr[ay];
+    if (acc) {  // slab batches: the signed sums add up, |.| is taken once, in the last batch
+        signed_sum += acc[y * N + x];
+        if (!final_batch) {
+            acc[y * N + x] = signed_sum;
+            return;
+        }
+    }
+    double value = fabs(signed_sum) * inv_n;
+    // a NaN or Inf among the gridded values: every moment cell would be NaN after the FFT, so every
+    // valid pixel is NaN (the reference's float atomics, SVDIntegratedImager.cu:1276-1290, carry it)
+    if (bad) value = __longlong_as_double(0x7ff8000000000000LL);
+    if (presplat) {
+        out[y * N + x] = (float)value;
+        return;
+    }
+
+    const SplatTarget tg = reprojection == SVDI_REPROJ_FIPK ? reproject_fipk(x, y, N, cell, V)
+                                                            : reproject_sii(x, y, N, kc, V);
+    if (!tg.ok) return;
+    const double LL = tg.LL, MM = tg.MM;
+    if (!(fabs(LL) < (double)(half - 1) && fabs(MM) < (double)(half - 1))) return;
+    const double Lf = floor(LL), Mf = floor(MM), Lc = ceil(LL), Mc = ceil(MM);
+    float* d = out + half * N + half;
+    atomicAdd(&d[(long long)Mf * N + (long long)Lf], (float)((1 - LL + Lf) * (1 - MM + Mf) * value));
+    atomicAdd(&d[(long long)Mc * N + (long long)Lf], (float)((1 - LL + Lf) * (0 + MM - Mf) * value));
+    atomicAdd(&d[(long long)Mf * N + (long long)Lc], (float)((0 + LL - Lf) * (1 - MM + Mf) * value));
+    atomicAdd(&d[(long long)Mc * N + (long long)Lc], (float)((0 + LL - Lf) * (0 + MM - Mf) * value));
+}
+
 // One pixel (x, y) of the rotated frame: moments -> |Re sum| -> grid correction -> reprojection.
 template <int KMAX>
 __device__ __forceinline__ void recombine_pixel(long long x, long long y, const float2* __restrict__ moments,
@@ -182,36 +223,7 @@ __device__ __forceinline__ void recombine_pixel(long long x, long long y, const 
         }
         sum += (s4[0] + s4[1]) + (s4[2] + s4[3]);
     }
-    if ((xr + yr) & 1) sum = -sum;
-    const long long ax = xr < 0 ? -xr : xr, ay = yr < 0 ? -yr : yr;
-    double signed_sum = sum * (double)corr[ax] * (double)corr[ay];
-    if (acc) {  // slab batches: the signed sums add up, |.| is taken once, in the last batch
-        signed_sum += acc[y * N + x];
-        if (!final_batch) {
-            acc[y * N + x] = signed_sum;
-            return;
-        }
-    }
-    double value = fabs(signed_sum) * inv_n;
-    // a NaN or Inf among the gridded values: every moment cell would be NaN after the FFT, so every
-    // valid pixel is NaN (the reference's float atomics, SVDIntegratedImager.cu:1276-1290, carry it)
-    if (bad) value = __longlong_as_double(0x7ff8000000000000LL);
-    if (presplat) {
-        out[y * N + x] = (float)value;
-        return;
-    }
-
-    const SplatTarget tg = reprojection == SVDI_REPROJ_FIPK ? reproject_fipk(x, y, N, cell, V)
-                                                            : reproject_sii(x, y, N, kc, V);
-    if (!tg.ok) return;
-    const double LL = tg.LL, MM = tg.MM;
-    if (!(fabs(LL) < (double)(half - 1) && fabs(MM) < (double)(half - 1))) return;
-    const double Lf = floor(LL), Mf = floor(MM), Lc = ceil(LL), Mc = ceil(MM);
-    float* d = out + half * N + half;
-    atomicAdd(&d[(long long)Mf * N + (long long)Lf], (float)((1 - LL + Lf) * (1 - MM + Mf) * value));
-    atomicAdd(&d[(long long)Mc * N + (long long)Lf], (float)((1 - LL + Lf) * (0 + MM - Mf) * value));
-    atomicAdd(&d[(long long)Mf * N + (long long)Lc], (float)((0 + LL - Lf) * (1 - MM + Mf) * value));
-    atomicAdd(&d[(long long)Mc * N + (long long)Lc], (float)((0 + LL - Lf) * (0 + MM - Mf) * value));
+    finish_pixel(x, y, sum, N, cell, V, corr, inv_n, reprojection, presplat, out, acc, final_batch, bad, kc);
 }
 
 // Persistent over 32 x 8 pixel tiles: the per-launch constants (slab geometry, reprojection
@@ -244,6 +256,67 @@ __global__ void __launch_bounds__(256, 4) k_recombine(const float2* __restrict__
     }
 }
 
+// One pixel from w planes: Re sum_p e^{2 pi i w_p t3} M_p / psi^(dw t3). The phases advance by one
+// rotation per plane in FP64 (two chains of every other plane).
+__global__ void __launch_bounds__(256, 4) k_recombine_w(const float2* __restrict__ planes, GridGeom g, long long N,
+                                                    double cell, const double* __restrict__ vin, WPlanes wp,
+                                                    int plane_lo, int plane_hi, const float* __restrict__ corr,
+                                                    double inv_n, int reprojection, int presplat,
+                                                    float* __restrict__ out, double* __restrict__ acc,
+                                                    int final_batch, const unsigned long long* __restrict__ nonfinite) {
+    __shared__ ReprojConst kc;
+    if (threadIdx.x == 0 && threadIdx.y == 0) kc = reproj_const(vin, cell);
+    __syncthreads();
+    const bool bad = nonfinite && *nonfinite;
+    double V[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) V[k] = vin[k];
+    const long long half = N / 2, G = g.G, GG = G * G;
+    const long long ntx = (N + 31) / 32, nty = (N + 7) / 8;
+    for (long long t = blockIdx.x; t < ntx * nty; t += gridDim.x) {
+        const long long ty = t / ntx, tx = t - ty * ntx;
+        const long long x = tx * 32 + threadIdx.x, y = ty * 8 + threadIdx.y;
+        if (x >= N || y >= N) continue;
+        const long long xr = x - half, yr = y - half;
+        const double t1 = cell * (double)yr, t2 = cell * (double)xr;
+        const double ra = 1.0 - (t1 + V[2]) * (t1 + V[2]) - (t2 + V[5]) * (t2 + V[5]);
+        if (ra < 0.0) {
+            if (presplat && final_batch) out[y * N + x] = __int_as_float(0x7fc00000);  // NaN
+            continue;
+        }
+        const double t3 = -V[8] + (V[8] >= 0.0 ? 1.0 : -1.0) * sqrt(ra);
+        const double w0 = wp.lo + (double)(plane_lo - (wp.W / 2 - 1)) * wp.dw;
+        double si, co, dsi, dco;
+        sincospi(2.0 * t3 * w0, &si, &co);
+        sincospi(2.0 * t3 * wp.dw, &dsi, &dco);
+        const float2* mp = planes + GG / 2 + G / 2 + yr * G + xr;
+        double sum0 = 0.0, sum1 = 0.0;
+        int n = plane_hi - plane_lo;
+#pragma unroll 4
+        for (; n >= 2; n -= 2) {
+            const float2 m0 = mp[0], m1 = mp[GG];
+            mp += 2 * GG;
+            sum0 += co * (double)m0.x - si * (double)m0.y;
+            double c1 = co * dco - si * dsi, s1 = si * dco + co * dsi;
+            sum1 += c1 * (double)m1.x - s1 * (double)m1.y;
+            co = c1 * dco - s1 * dsi;
+            si = s1 * dco + c1 * dsi;
+        }
+        if (n) sum0 += co * (double)mp[0].x - si * (double)mp[0].y;
+        // 1 / psi^ by Clenshaw's recurrence in 2 (t3 / max|t3|)^2 - 1
+        const double kk = t3 * wp.dw / wp.kmax, z = 2.0 * kk * kk - 1.0;
+        double b1 = 0.0, b2 = 0.0;
+#pragma unroll
+        for (int i = kWCorrTerms - 1; i > 0; --i) {
+            const double b = fma(2.0 * z, b1, wp.corr[i] - b2);
+            b2 = b1;
+            b1 = b;
+        }
+        finish_pixel(x, y, (sum0 + sum1) * fma(z, b1, wp.corr[0] - b2), N, cell, V, corr, inv_n, reprojection,
+                     presplat, out, acc, final_batch, bad, kc);
+    }
+}
+
 }  // namespace
 
 int launch_recombine(const float2* d_moments, const GridGeom& g, long long N, double cell,
@@ -263,6 +336,19 @@ int launch_recombine(const float2* d_moments, const GridGeom& g, long long N, do
         set_error("recombine: too many Chebyshev terms");
         return SVDI_ERR_UNSUPPORTED;
     }
+    SVDI_LAUNCHED();
+    return SVDI_OK;
+}
+
+int launch_recombine_w(const float2* d_planes, const GridGeom& g, long long N, double cell, const double* d_vin64,
+                       const WPlanes& wp, int plane_lo, int plane_hi, const float* d_corr, double inv_n_total,
+                       int reprojection, int presplat, float* d_out, cudaStream_t st, double* d_acc, bool final_batch,
+                       const unsigned long long* d_nonfinite) {
+    const dim3 block(32, 8);
+    const long long tiles = ((N + 31) / 32) * ((N + 7) / 8);
+    const dim3 grid((unsigned)std::min<long long>(tiles, 8LL * current_sm_count()));
+    k_recombine_w<<<grid, block, 0, st>>>(d_planes, g, N, cell, d_vin64, wp, plane_lo, plane_hi, d_corr, inv_n_total,
+                                          reprojection, presplat, d_out, d_acc, final_batch ? 1 : 0, d_nonfinite);
     SVDI_LAUNCHED();
     return SVDI_OK;
 }

@@ -304,7 +304,26 @@ int launch_grid_mma(const SampleRec* d_rec, const float* d_rec_s, const unsigned
                     int key_hi, const GridGeom& g, int K, const EsPoly& poly, float2* d_planes,
                     int sm_count, cudaStream_t st);
 
+// wplanes.cu: imaging through P w planes w_p = lo + (p - (W / 2 - 1)) dw (even grid sizes, support 6 or 8)
+constexpr int kWCorrTerms = 16;
+struct WPlanes {
+    int P, W;             // planes; planes per sample
+    double lo, dw, inv_dw;
+    double kmax;          // max |t3| dw
+    double corr[kWCorrTerms];  // 1 / psi^(k) = sum_i corr[i] T_i(2 (k / kmax)^2 - 1)
+    float beta_xy;
+};
+// Grids the samples of a separable source into planes [plane_lo, plane_hi); pxy and pz: the kernels of
+// the image axes and of the w axis. Dropped and non-finite samples are counted as the binning does.
+int launch_grid_w(const SampleSource& src, const GridGeom& g, const WPlanes& wp, const EsPoly& pxy, const EsPoly& pz,
+                  int plane_lo, int plane_hi, float2* d_planes, unsigned long long* d_dropped, cudaStream_t st);
+
 // image.cu
+// The planes [plane_lo, plane_hi) of a w-plane call; d_acc and final_batch as below.
+int launch_recombine_w(const float2* d_planes, const GridGeom& g, long long N, double cell, const double* d_vin64,
+                       const WPlanes& wp, int plane_lo, int plane_hi, const float* d_corr, double inv_n_total,
+                       int reprojection, int presplat, float* d_out, cudaStream_t st, double* d_acc, bool final_batch,
+                       const unsigned long long* d_nonfinite);
 // d_acc (N x N doubles, zeroed before the first batch) when the slabs are split over several
 // batches: every batch adds its signed sum, the final batch takes |.| and writes the image.
 int launch_recombine(const float2* d_moments, const GridGeom& g, long long N, double cell,

@@ -1,0 +1,132 @@
+"""Imaging through w planes (error-target rule, 48 and more moment planes) against the FP64 DFT of the same
+samples and against the Chebyshev form of the same call (an explicit tile size keeps that form).
+
+Tolerance: the w kernel's largest error is 2e-7 (10 planes per sample) or 7e-9 (12), below the error target
+1e-6 of either form; the images are held to the 1e-5 relative RMS of the other parity tests."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from svdimager_b200 import api
+from tests.conftest import snapshot
+
+pytestmark = pytest.mark.gpu
+
+IMG_TOL = 1e-5
+
+
+def _snap(N, nchan, rows, shift=0.0):
+    """A wide-field snapshot of `rows` baselines whose w range needs many moment planes; `shift` adds a
+    constant w (metres), so that all r3 have one sign."""
+    s = snapshot("widefield", nchan=nchan, n_rows_limit=rows, image_size=N, cell_size=0.3 / N)
+    if not shift:
+        return s
+    uvw = s.uvw.copy()
+    uvw[:, 2] += np.float32(shift)
+    return dataclasses.replace(s, uvw=uvw)
+
+
+def _images(s, **kw):
+    opt = dict(k_rule=api.KRULE_TARGET, target_error=1e-6, presplat=1)
+    opt.update(kw)
+    rng = np.random.default_rng(4)
+    px, py = rng.integers(0, s.image_size, 400), rng.integers(0, s.image_size, 400)
+    with api.Engine(**opt) as e:
+        img = e.image(s)
+        st = e.stats()
+        dft = e.dft_pixels(px, py)
+    with api.Engine(**dict(opt, tile=32)) as e:
+        ref = e.image(s)
+        rst = e.stats()
+    return img, st, img[py, px], dft, ref, rst
+
+
+@pytest.mark.parametrize("N,nchan,rows,kw", [
+    (512, 4, 6000, dict(edge_mode=api.EDGE_STRICT)),
+    (512, 4, 6000, dict(edge_mode=api.EDGE_STRICT, max_batch_slabs=1)),
+    (256, 33, 700, dict(edge_mode=api.EDGE_STRICT, support=6, beta=0.75 * O.REF_BETA)),
+    (500, 1, 9001, dict(edge_mode=api.EDGE_STRICT, target_error=1e-7)),
+    (384, 5, 5000, dict(edge_mode=api.EDGE_STRICT, support=6, beta=0.75 * O.REF_BETA, target_error=1e-7)),
+    (512, 7, 3000, dict()),
+])
+def test_matches_dft_and_chebyshev_form(cuda_device, N, nchan, rows, kw):
+    s = _snap(N, nchan, rows)
+    img, st, at, dft, ref, rst = _images(s, **kw)
+    assert st["num_planes"] >= 48 and st["num_planes"] == rst["num_planes"]
+    assert st["num_gridded"] == rst["num_gridded"]
+    m = np.isfinite(ref)
+    assert np.array_equal(m, np.isfinite(img))
+    tol = IMG_TOL if kw.get("support", 8) == 8 else 2e-4  # six taps at sigma 1.5 alias at 1e-4
+    assert O.rel_rms(img[m], ref[m]) < IMG_TOL
+    if kw.get("edge_mode") == api.EDGE_STRICT:  # clipped footprints are no samples of the DFT
+        f = np.isfinite(dft)
+        assert O.rel_rms(at[f], dft[f]) < tol
+
+
+def test_one_signed_w_range(cuda_device):
+    s = _snap(512, 4, 6000, shift=400.0)
+    img, st, at, dft, ref, rst = _images(s, edge_mode=api.EDGE_STRICT)
+    assert st["num_planes"] >= 48
+    f = np.isfinite(dft)
+    assert O.rel_rms(at[f], dft[f]) < IMG_TOL
+
+
+def test_exactly_integer_positions_and_both_edges(cuda_device):
+    """Baselines on exact grid cells and on the outermost cells that the clip rule keeps, on both sides (the
+    mirrored ones wrap from +G/2 to -G/2)."""
+    N = 128
+    s = _snap(N, 1, 2000)
+    cell = float(np.float32(s.cell_size))
+    G = (3 * N + 1) // 2
+    with api.Engine(k_rule=api.KRULE_TARGET, target_error=1e-6) as e:
+        e.image(s)
+        vin = np.array(e.stats()["vin"]).reshape(3, 3)
+    q = s.uvw.astype(np.float64) @ vin.T
+    sc = float(s.frequencies_hz[0]) / 299792458.0
+    scale = cell * G * sc
+    rng = np.random.default_rng(8)
+    cells = rng.integers(-G // 2 - 3, G // 2 + 4, (2000, 2))
+    q[:, :2] = cells / scale
+    q[::2, :2] += rng.uniform(0, 1, (1000, 2)) / scale
+    t = dataclasses.replace(s, uvw=(q @ vin).astype(np.float32))
+    img, st, _, _, ref, rst = _images(t)
+    assert st["num_gridded"] == rst["num_gridded"] and st["num_planes"] == rst["num_planes"] >= 48
+    m = np.isfinite(ref)
+    assert O.rel_rms(img[m], ref[m]) < IMG_TOL
+
+
+def test_buffers_and_next_calls(cuda_device):
+    """The records and moments of a w-plane call are those of its Chebyshev form; asking for them changes
+    neither the statistics nor the calls that follow."""
+    s = _snap(256, 4, 3000)
+    opt = dict(k_rule=api.KRULE_TARGET, target_error=1e-6, edge_mode=api.EDGE_STRICT)
+    with api.Engine(**opt) as e, api.Engine(keep_grid=1, **opt) as c:
+        img = e.image(s)
+        st = e.stats()
+        ref = c.image(s)
+        assert np.array_equal(e.buffer(api.BUF_OFFSETS), c.buffer(api.BUF_OFFSETS))
+        a, b = e.buffer(api.BUF_RECORDS), c.buffer(api.BUF_RECORDS)
+        order = ("vim", "vre", "yq", "xq")
+        assert np.array_equal(np.sort(a, order=order), np.sort(b, order=order))
+        assert len(e.buffer(api.BUF_RECORDS_S)) == len(a)
+        ma, mb = e.buffer(api.BUF_MOMENTS), c.buffer(api.BUF_MOMENTS)
+        assert ma.shape == mb.shape and np.linalg.norm(ma - mb) < 1e-5 * np.linalg.norm(mb)
+        assert e.stats() == st
+        again = e.image(s)
+        assert O.rel_rms(again, img) < 1e-6 and O.rel_rms(img, ref) < IMG_TOL
+        flat = snapshot("small")
+        assert O.rel_rms(e.image(flat), c.image(flat)) < 1e-6  # a Chebyshev call after it
+
+
+def test_non_finite_visibility(cuda_device):
+    s = _snap(256, 4, 3000)
+    v = s.vis0_real.copy()
+    row = np.argmin(np.hypot(s.uvw[:, 0], s.uvw[:, 1]) + 1e9 * (s.flag0[:s.num_rows] != 0))
+    v[row] = np.nan  # channel 0 of an unflagged short baseline
+    t = dataclasses.replace(s, vis0_real=v)
+    with api.Engine(k_rule=api.KRULE_TARGET, target_error=1e-6, edge_mode=api.EDGE_CLIP) as e:
+        img = e.image(t)
+        ok = e.image(s)
+    assert np.isnan(img).any() and np.array_equal(np.isnan(img), ok != 0)
