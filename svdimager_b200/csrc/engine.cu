@@ -84,6 +84,9 @@ constexpr int kPartialCap = 4096;
         }                                                                                 \
     } while (0)
 
+// Frees the idle engines of the two-step entry's pool; true when there were any.
+bool drop_idle_engines();
+
 // Grow-only device buffer.
 struct DevBuf {
     void* p = nullptr;
@@ -100,6 +103,10 @@ struct DevBuf {
         }
         const size_t want = std::max<size_t>(bytes, 256);
         cudaError_t e = cudaMalloc(&p, want);
+        if (e == cudaErrorMemoryAllocation && drop_idle_engines()) {  // memory that only the idle pool holds
+            cudaGetLastError();
+            e = cudaMalloc(&p, want);
+        }
         if (e != cudaSuccess) {
             cudaGetLastError();
             set_error(std::string("device allocation of ") + std::to_string(want) + " bytes failed: " +
@@ -215,6 +222,17 @@ struct svdi_engine {
     // pageable host uploads and image downloads of the archive entry and the host-input call
     svdi::HostStager stager;
     bool batch_bound = false;  // a batch's captured graph refers to this engine's buffers
+
+    size_t device_bytes() const {
+        size_t n = 0;
+        for (const svdi::DevBuf* b :
+             {&in_uvw, &in_freq, &in_v0r, &in_v0i, &in_v3r, &in_v3i, &in_f0, &in_f3, &in_w0, &in_w3, &in_bin, &in_vin, &vr,
+              &vi, &q, &s, &vin64, &vin32, &stats, &partial, &counts, &offsets, &cursor, &dropped, &rec, &rec_s, &planes,
+              &corr, &image, &cheb_err, &bin_out, &grid_keep, &tc_status, &kb_offsets, &acc, &chunk_key, &keymax,
+              &plan_buf, &scan_sums, &probe, &remade})
+            n += b->cap;
+        return n;
+    }
 
     ~svdi_engine() {
         if (device >= 0) cudaSetDevice(device);
@@ -594,9 +612,12 @@ double es_transform(int W, double beta, double k) {
 
 // The w-plane geometry of a call with r3 in [r3min, r3max] and |t3| <= mt3, or false when the call
 // images through Chebyshev moments: other rules than the error target (their truncation is part of the
-// result), other gridders, few moment planes (measured: at 48 and more the w planes are faster on every
-// grid tried, from 1.2x at 48 to 2.5x at 236), no fewer w planes than 3/4 of them, odd grid sizes (the
-// reference's indexing of those does not commute with the mirrored samples).
+// result), other gridders, odd grid sizes (the reference's indexing of those does not commute with the
+// mirrored samples), few moment planes, or when the moments are estimated to be faster. The estimate, fitted
+// to B200 times: a sample and w plane 0.17 ns (its reductions in the L2), a sample and Chebyshev term 0.018
+// ns, a plane's clearing, FFT and recombination 10 ps a cell (12 ps for moments). Measured (w planes against
+// moments): 2.9 M samples, 1536^2 grid, 53 moments 5.5 / 4.1 ms; 0.64 M, 1536^2, 144 moments 2.4 / 4.5 ms;
+// 0.32 M, 3072^2, 43 moments 3.2 / 6.5 ms; 89 k, 384^2, 92 moments 0.40 / 0.55 ms.
 bool plan_wplanes(svdi_engine* e, const SampleSource& src, long long G, const SlabParams& sp, double r3min,
                   double r3max, double mt3, WPlanes& wp) {
     const svdi_options& o = e->opt;
@@ -613,7 +634,9 @@ bool plan_wplanes(svdi_engine* e, const SampleSource& src, long long G, const Sl
     wp.dw = 1.0 / (2.0 * 1.5 * mt3);
     wp.inv_dw = 1.0 / wp.dw;
     const double span = std::floor((hi - wp.lo) * wp.inv_dw * (1.0 + 1e-12)) + wp.W;
-    if (!(span <= 0.75 * sp.nslab * sp.K)) return false;
+    const double n = (double)src.n, cells = (double)G * (double)G;
+    if (!(n * wp.W * 1.7e-7 + span * cells * 1.0e-8 < n * sp.K * 1.8e-8 + (double)sp.nslab * sp.K * cells * 1.2e-8))
+        return false;
     wp.P = (int)span;
     wp.kmax = mt3 * wp.dw;
     const double beta = 2.06 * wp.W;
@@ -1260,6 +1283,46 @@ svdi_options archive_defaults() {
 std::mutex g_default_mu;
 std::map<int, std::unique_ptr<svdi_engine>> g_default_engines;
 
+// Idle engines of the two-step entry (svdi_preprocess_measurement_set ... svdi_free_device_buffers): the
+// entry used to make and destroy an engine per snapshot -- streams, some 25 allocations, a cuFFT plan --
+// which took 7 of the 8.5 ms of a 512^2 call with 130 k samples. A freed engine waits here for the next
+// call, at most kIdleEngines of them and kIdleBytes of their device memory in all; beyond that it is
+// destroyed as before, and a failing allocation of this library destroys them all and tries again. An engine
+// is owned by one descriptor at a time; the pool itself is guarded by a mutex.
+constexpr size_t kIdleEngines = 2;
+constexpr size_t kIdleBytes = (size_t)1 << 30;
+std::mutex g_idle_mu;
+std::vector<std::unique_ptr<svdi_engine>> g_idle;
+
+std::unique_ptr<svdi_engine> take_idle_engine(int device) {
+    std::lock_guard<std::mutex> lk(g_idle_mu);
+    for (size_t i = 0; i < g_idle.size(); ++i)
+        if (g_idle[i]->device == device) {
+            std::unique_ptr<svdi_engine> e = std::move(g_idle[i]);
+            g_idle.erase(g_idle.begin() + (long)i);
+            return e;
+        }
+    return nullptr;
+}
+
+void give_idle_engine(std::unique_ptr<svdi_engine> e) {
+    // a new descriptor decides its slab batches by the memory that is free then, and starts without a plan
+    e->bslab_cache.clear();
+    e->spec_valid = false;
+    e->have_last = false;
+    e->last_w = false;
+    {
+        std::lock_guard<std::mutex> lk(g_idle_mu);
+        size_t held = e->device_bytes();
+        for (const auto& other : g_idle) held += other->device_bytes();
+        if (g_idle.size() < kIdleEngines && held <= kIdleBytes) {
+            g_idle.push_back(std::move(e));
+            return;
+        }
+    }
+    e.reset();  // outside the lock: freeing device memory waits for the device
+}
+
 int default_engine(svdi_engine** out) {
     int dev = 0;
     SVDI_CUDA(cudaGetDevice(&dev));
@@ -1273,6 +1336,20 @@ int default_engine(svdi_engine** out) {
     }
     *out = it->second.get();
     return SVDI_OK;
+}
+
+bool drop_idle_engines() {
+    std::vector<std::unique_ptr<svdi_engine>> gone;
+    int dev = 0;
+    const bool have = cudaGetDevice(&dev) == cudaSuccess;
+    {
+        std::lock_guard<std::mutex> lk(g_idle_mu);
+        gone.swap(g_idle);
+    }
+    const bool any = !gone.empty();
+    gone.clear();
+    if (have) cudaSetDevice(dev);  // an engine's destructor selects its own device
+    return any;
 }
 
 }  // namespace
@@ -1511,21 +1588,26 @@ int svdi_preprocess_measurement_set(const svdi_host_ms* h, svdi_device_buffers* 
     svdi_options o;
     svdi_default_options(&o);
     SVDI_CUDA(cudaGetDevice(&o.device));
-    svdi_engine* e = nullptr;
-    SVDI_TRY(svdi_engine_create(&o, &e));
-    std::unique_ptr<svdi_engine> guard(e);
+    std::unique_ptr<svdi_engine> guard = take_idle_engine(o.device);
+    if (!guard) {
+        svdi_engine* made = nullptr;
+        SVDI_TRY(svdi_engine_create(&o, &made));
+        guard.reset(made);
+    }
+    svdi_engine* e = guard.get();
+    SVDI_CUDA(cudaSetDevice(e->device));
     cudaStream_t st = e->stream;
     const size_t n = h->num_samples, R = h->num_rows, C = h->num_channels;
     SVDI_TRY(upload(e->in_uvw, h->uvw, R * 3, st));
     SVDI_TRY(upload(e->in_freq, h->frequencies_hz, C, st));
-    SVDI_TRY(upload(e->in_v0r, h->vis0_real, n, st));
-    SVDI_TRY(upload(e->in_v0i, h->vis0_imag, n, st));
-    SVDI_TRY(upload(e->in_v3r, h->vis3_real, n, st));
-    SVDI_TRY(upload(e->in_v3i, h->vis3_imag, n, st));
-    SVDI_TRY(upload(e->in_f0, h->flag0, n, st));
-    SVDI_TRY(upload(e->in_f3, h->flag3, n, st));
-    SVDI_TRY(upload(e->in_w0, h->weight0, n, st));
-    SVDI_TRY(upload(e->in_w3, h->weight3, n, st));
+    SVDI_TRY(upload_staged(e, e->in_v0r, h->vis0_real, n, st));
+    SVDI_TRY(upload_staged(e, e->in_v0i, h->vis0_imag, n, st));
+    SVDI_TRY(upload_staged(e, e->in_v3r, h->vis3_real, n, st));
+    SVDI_TRY(upload_staged(e, e->in_v3i, h->vis3_imag, n, st));
+    SVDI_TRY(upload_staged(e, e->in_f0, h->flag0, n, st));
+    SVDI_TRY(upload_staged(e, e->in_f3, h->flag3, n, st));
+    SVDI_TRY(upload_staged(e, e->in_w0, h->weight0, n, st));
+    SVDI_TRY(upload_staged(e, e->in_w3, h->weight3, n, st));
     SVDI_TRY(e->vr.ensure(n * 4));
     SVDI_TRY(e->vi.ensure(n * 4));
     SVDI_TRY(e->q.ensure(R * 24));
@@ -1584,8 +1666,7 @@ int svdi_fipipe_device(const svdi_device_buffers* dev, float* dirty_image, size_
     src.vi = dev->d_vis_imag;
     src.n = (long long)dev->num_samples;
     SVDI_TRY(image_core(e, false, src, (long long)N, cell, e->image.as<float>()));
-    SVDI_CUDA(cudaMemcpyAsync(dirty_image, e->image.p, N * N * 4, cudaMemcpyDeviceToHost, e->stream));
-    SVDI_CUDA(cudaStreamSynchronize(e->stream));
+    SVDI_TRY(e->stager.d2h(dirty_image, e->image.p, N * N * 4, e->stream));
     SVDI_TRY(finish_pending(e));
     return SVDI_OK;
 }
@@ -1604,7 +1685,7 @@ void svdi_free_device_buffers(svdi_device_buffers* dev) {
     if (!dev) return;
     if (dev->internal) {
         auto* in = static_cast<svdi_pre_internal*>(dev->internal);
-        delete in->engine;
+        give_idle_engine(std::unique_ptr<svdi_engine>(in->engine));
         delete in;
     }
     memset(dev, 0, sizeof(*dev));

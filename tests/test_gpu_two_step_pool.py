@@ -1,0 +1,71 @@
+"""The two-step entry's idle engines: buffers taken over from an earlier descriptor give the images of a fresh
+engine, whatever the shapes in between, with several descriptors live at once and from several threads.
+
+Tolerance 1e-6 relative RMS: the order of floating-point atomic adds (as in the other repeat tests)."""
+import threading
+
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from svdimager_b200 import api
+from tests.conftest import snapshot
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = ((16, 8128, 256), (2, 500, 64), (16, 8128, 256), (5, 3000, 128))
+
+
+def _two_step(s, want_bin=False):
+    b = api.preprocess_measurement_set_gpu(s, want_bin=want_bin)
+    assert bool(b.buf.d_bin) == want_bin
+    img = api.FIpipeDevice(b, s.image_size, s.cell_size)
+    api.free_device_preprocess_buffers(b)
+    return img
+
+
+@pytest.fixture(scope="module")
+def cases():
+    out = []
+    for nchan, rows, N in SHAPES:
+        s = snapshot("small", nchan=nchan, n_rows_limit=rows, image_size=N, cell_size=0.1 / N)
+        with api.Engine() as e:
+            out.append((s, e.image(s)))
+    return out
+
+
+def test_taken_over_engines_match_fresh_ones(cuda_device, cases):
+    for i, (s, ref) in enumerate(cases * 2):
+        assert O.rel_rms(_two_step(s, want_bin=i % 3 == 0), ref) < 1e-6, i
+
+
+def test_live_descriptors_keep_their_buffers(cuda_device, cases):
+    """More descriptors than idle engines, imaged after all of them were filled, twice over."""
+    for _ in range(2):
+        live = [(api.preprocess_measurement_set_gpu(s), s, ref) for s, ref in cases]
+        assert len({b.buf.d_vis_real for b, _, _ in live}) == len(live)
+        for b, s, ref in live:
+            assert O.rel_rms(api.FIpipeDevice(b, s.image_size, s.cell_size), ref) < 1e-6
+        for b, _, _ in live:
+            b.free()
+
+
+def test_threads(cuda_device, cases):
+    errors = []
+
+    def work(k):
+        try:
+            for i in range(6):
+                s, ref = cases[(k + i) % len(cases)]
+                err = O.rel_rms(_two_step(s), ref)
+                if not err < 1e-6:
+                    errors.append((k, i, err))
+        except Exception as ex:  # noqa: BLE001
+            errors.append((k, repr(ex)))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors

@@ -1,4 +1,5 @@
-"""Imaging through w planes (error-target rule, 48 and more moment planes) against the FP64 DFT of the same
+"""Imaging through w planes (error-target rule, 48 and more moment planes, not too many
+samples per plane cell) against the FP64 DFT of the same
 samples and against the Chebyshev form of the same call (an explicit tile size keeps that form).
 
 Tolerance: the w kernel's largest error is 2e-7 (10 planes per sample) or 7e-9 (12), below the error target
