@@ -315,18 +315,20 @@ __global__ void __launch_bounds__(kThreads) k_scatter(SampleSource src, GridGeom
     }
 }
 
-// Separable sources (r = s[chan] q[row], idx = row + chan R). A warp takes units of kUnitRows
-// rows x one chunk of `lpr` channels (lpr a power of two <= 32): lane -> (row kUnitRows-subset
+// Separable sources (r = s[chan] q[row], idx = row + chan R). A warp takes units of UR
+// rows x one chunk of `lpr` channels (lpr a power of two <= 32): lane -> (row subset
 // lane / lpr, channel lane % lpr), so consecutive lanes hold consecutive channels of one row. The
 // channels of a baseline mostly share a tile, so match groups are large: one shared-memory or
 // global atomic per group, and a group's records land in consecutive slots. No 64-bit division.
-constexpr int kUnitRows = 16;
-static_assert(32 / 2 <= kUnitRows, "every lane must take part in each row step");
+// UR = 16, or 4 where 16 would leave most of the chip idle: a unit is a serial chain of row steps (FP64 key
+// rule, match, a returning cursor atomic in the scatter). 130 k samples: histogram 11 -> 6 us, scatter 18 ->
+// 9 us; 8.4 M samples keep 16, whose staging loads are whole 64-byte pieces.
+constexpr int kUnitRows = 16, kUnitRowsSmall = 4;
 
 struct SepMap {
     int lpr;       // lanes per row (channels per chunk)
     int nch;       // channel chunks
-    int nrt;       // row tiles of kUnitRows
+    int nrt;       // row tiles of UR
     int C;
 };
 
@@ -335,6 +337,7 @@ __device__ inline void unit_of(long long u, const SepMap& m, int& rt, int& ch) {
     ch = (int)(u - (long long)rt * m.nch);
 }
 
+template <int UR>
 __global__ void __launch_bounds__(kThreads) k_histogram_sep(SampleSource src, SepMap m, GridGeom g, SlabParams sp,
                                                            unsigned int* __restrict__ counts, int n_keys,
                                                            unsigned long long* __restrict__ dropped,
@@ -357,10 +360,12 @@ __global__ void __launch_bounds__(kThreads) k_histogram_sep(SampleSource src, Se
         const int c = ch * m.lpr + coff;
         const bool cvalid = c < m.C;
         const double sc = cvalid ? src.s[c] : 0.0;
-        for (int i = sub; i < kUnitRows; i += rps) {
-            const long long row = (long long)rt * kUnitRows + i;
+        // every lane takes every step (the match needs the whole warp); rows past the unit have no key
+        for (int i0 = 0; i0 < UR; i0 += rps) {
+            const int i = i0 + sub;
+            const long long row = (long long)rt * UR + i;
             int key = -2;
-            if (cvalid && row < src.R) {
+            if (cvalid && i < UR && row < src.R) {
                 const double* q = src.q + row * 3;
                 key = row_chan_key(sc, q[0], q[1], q[2], g, sp).key;
                 if (key < 0) ++ndrop;
@@ -384,8 +389,7 @@ __global__ void __launch_bounds__(kThreads) k_histogram_sep(SampleSource src, Se
 // Scatter for separable sources: per unit, the warp stages the unit's collapsed visibilities in
 // shared memory with row-contiguous loads, then writes each group's records to the slots one
 // global atomic on the key's cursor reserved.
-constexpr int kVisPitch = kUnitRows + 1;   // float2 pitch of a staged channel (bank-conflict free)
-
+template <int UR>
 __global__ void __launch_bounds__(kThreads) k_scatter_sep(SampleSource src, SepMap m, GridGeom g, SlabParams sp,
                                                          unsigned int* __restrict__ cursor,
                                                          SampleRec* __restrict__ rec, float* __restrict__ rec_s,
@@ -396,6 +400,7 @@ __global__ void __launch_bounds__(kThreads) k_scatter_sep(SampleSource src, SepM
         sp = plan->sp;
         src.inv_det = plan->inv_det;
     }
+    constexpr int kVisPitch = UR + 1;   // float2 pitch of a staged channel (bank-conflict free)
     __shared__ float2 stage[kThreads / 32][32 * kVisPitch];
     float2* my = stage[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -408,29 +413,30 @@ __global__ void __launch_bounds__(kThreads) k_scatter_sep(SampleSource src, SepM
     for (long long u = (long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); u < nunits; u += nwarps) {
         int rt, ch;
         unit_of(u, m, rt, ch);
-        const long long row0 = (long long)rt * kUnitRows;
+        const long long row0 = (long long)rt * UR;
         const int c0 = ch * m.lpr;
-        // stage: lanes 0-15 and 16-31 read kUnitRows consecutive rows of two channels
+        // stage: UR lanes read UR consecutive rows of a channel, 32 / UR channels at a time
         __syncwarp();
-        for (int k = 0; k < m.lpr; k += 2) {
-            const int cc = k + (lane >> 4);
-            const long long row = row0 + (lane & 15);
+        for (int k = 0; k < m.lpr; k += 32 / UR) {
+            const int cc = k + lane / UR;
+            const long long row = row0 + lane % UR;
             float2 v = make_float2(0.0f, 0.0f);
             if (c0 + cc < m.C && row < R) {
                 const long long idx = row + (long long)(c0 + cc) * R;
                 v = make_float2(src.vr[idx], src.vi[idx]);
             }
-            my[cc * kVisPitch + (lane & 15)] = v;
+            my[cc * kVisPitch + lane % UR] = v;
         }
         __syncwarp();
         const int c = c0 + coff;
         const bool cvalid = c < m.C;
         const double sc = cvalid ? src.s[c] : 0.0;
-        for (int i = sub; i < kUnitRows; i += rps) {
+        for (int i0 = 0; i0 < UR; i0 += rps) {  // every lane takes every step
+            const int i = i0 + sub;
             const long long row = row0 + i;
             KeyRec kr;
             kr.key = -2;
-            if (cvalid && row < R) {
+            if (cvalid && i < UR && row < R) {
                 const double* q = src.q + row * 3;
                 kr = row_chan_key(sc, q[0], q[1], q[2], g, sp);
             }
@@ -467,14 +473,20 @@ __global__ void __launch_bounds__(kThreads) k_scatter_sep(SampleSource src, SepM
     }
 }
 
-SepMap sep_map(const SampleSource& src) {
+SepMap sep_map(const SampleSource& src, int unit_rows) {
     SepMap m{};
     m.C = (int)(src.n / src.R);
-    m.lpr = 2;   // >= 2: then 32 / lpr <= kUnitRows and every lane runs the same row loop
+    m.lpr = 2;
     while (m.lpr < 32 && m.lpr < m.C) m.lpr <<= 1;
     m.nch = (m.C + m.lpr - 1) / m.lpr;
-    m.nrt = (int)((src.R + kUnitRows - 1) / kUnitRows);
+    m.nrt = (int)((src.R + unit_rows - 1) / unit_rows);
     return m;
+}
+
+// Rows per unit: short units until they fill four 8-warp blocks per SM.
+int unit_rows(const SampleSource& src) {
+    const long long chunks = (src.n / src.R + 31) / 32;
+    return (src.R + kUnitRows - 1) / kUnitRows * chunks < 32LL * current_sm_count() ? kUnitRowsSmall : kUnitRows;
 }
 
 // Separable kernels need whole rows x channels and 32-bit unit and row counts.
@@ -490,13 +502,15 @@ int launch_histogram(const SampleSource& src, const GridGeom& g, const SlabParam
                      cudaStream_t st, const DevPlan* d_plan) {
     const size_t smem = n_keys <= kSmemKeyLimit ? (size_t)n_keys * 4 : 0;
     if (use_sep(src)) {
-        SVDI_TRY(ensure_dynamic_smem((const void*)k_histogram_sep, smem));
-        const SepMap m = sep_map(src);
+        const int ur = unit_rows(src);
+        auto kern = ur == kUnitRows ? k_histogram_sep<kUnitRows> : k_histogram_sep<kUnitRowsSmall>;
+        SVDI_TRY(ensure_dynamic_smem((const void*)kern, smem));
+        const SepMap m = sep_map(src, ur);
         const long long units = (long long)m.nrt * m.nch;
         long long blocks = (units + kThreads / 32 - 1) / (kThreads / 32);
         if (blocks > 4LL * current_sm_count()) blocks = 4LL * current_sm_count();   // a few units per warp: the shared histogram is flushed once
         if (blocks < 1) blocks = 1;
-        k_histogram_sep<<<(int)blocks, kThreads, smem, st>>>(src, m, g, sp, d_counts, n_keys, d_dropped, d_plan);
+        kern<<<(int)blocks, kThreads, smem, st>>>(src, m, g, sp, d_counts, n_keys, d_dropped, d_plan);
         SVDI_LAUNCHED();
         return SVDI_OK;
     }
@@ -532,12 +546,14 @@ int launch_scatter(const SampleSource& src, const GridGeom& g, const SlabParams&
                    unsigned int* d_cursor, int n_keys, SampleRec* d_rec, float* d_rec_s,
                    unsigned int* d_vmax, cudaStream_t st, unsigned int* d_keymax, const DevPlan* d_plan) {
     if (use_sep(src)) {
-        const SepMap m = sep_map(src);
+        const int ur = unit_rows(src);
+        auto kern = ur == kUnitRows ? k_scatter_sep<kUnitRows> : k_scatter_sep<kUnitRowsSmall>;
+        const SepMap m = sep_map(src, ur);
         const long long units = (long long)m.nrt * m.nch;
         long long blocks = (units + kThreads / 32 - 1) / (kThreads / 32);
         if (blocks > 8LL * current_sm_count()) blocks = 8LL * current_sm_count();
         if (blocks < 1) blocks = 1;
-        k_scatter_sep<<<(int)blocks, kThreads, 0, st>>>(src, m, g, sp, d_cursor, d_rec, d_rec_s, d_vmax, d_keymax,
+        kern<<<(int)blocks, kThreads, 0, st>>>(src, m, g, sp, d_cursor, d_rec, d_rec_s, d_vmax, d_keymax,
                                                         d_plan);
         SVDI_LAUNCHED();
         return SVDI_OK;

@@ -73,6 +73,11 @@ constexpr int kChebMaxMoments = 32;          // SVDIntegratedImager.cu:35
 constexpr double kChebTargetError = 1.0e-2;  // SVDIntegratedImager.cu:36
 constexpr double kChebTargetAlpha = 10.0;    // SVDIntegratedImager.cu:37
 constexpr int kPartialCap = 4096;
+// `counters`: block tickets of the two preprocessing kernels and of the t3 statistics
+constexpr int kCounterWords = 4;
+// `zero`, cleared before a call's binning: dropped and non-finite samples (64 bits each), the gridder's work
+// counters, then the key counts
+constexpr int kZeroWork = 4, kZeroCounts = 8;
 
 #define SVDI_CUFFT(call)                                                                  \
     do {                                                                                  \
@@ -164,13 +169,15 @@ struct svdi_engine {
     bool own_stream = true;
     // the flag/weight collapse runs on `side`, beside the rotation, statistics and histogram
     cudaStream_t side = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_vis = nullptr;
+    // (ev_vis), with max |t3| (after ev_basis), the read-back of the statistics (after ev_rows) and the
+    // clearing of the planes and the image (ev_clear); `zero` and `counters` are cleared on the main stream
+    cudaEvent_t ev_fork = nullptr, ev_vis = nullptr, ev_basis = nullptr, ev_rows = nullptr, ev_clear = nullptr;
     std::mutex mu;
     // staging for host inputs
     svdi::DevBuf in_uvw, in_freq, in_v0r, in_v0i, in_v3r, in_v3i, in_f0, in_f3, in_w0, in_w3;
     svdi::DevBuf in_bin, in_vin;
     // intermediates
-    svdi::DevBuf vr, vi, q, s, vin64, vin32, stats, partial, counts, offsets, cursor, dropped, rec,
+    svdi::DevBuf vr, vi, q, s, vin64, vin32, stats, partial, zero, offsets, cursor, counters, rec,
         rec_s, planes, corr, image, cheb_err, bin_out, grid_keep, tc_status, kb_offsets, acc, chunk_key, keymax,
         plan_buf, scan_sums;
     size_t sz_vr = 0, sz_q = 0, sz_s = 0, sz_off = 0, sz_rec = 0, sz_rec_s = 0, sz_grid = 0, sz_mom = 0;
@@ -227,7 +234,7 @@ struct svdi_engine {
         size_t n = 0;
         for (const svdi::DevBuf* b :
              {&in_uvw, &in_freq, &in_v0r, &in_v0i, &in_v3r, &in_v3i, &in_f0, &in_f3, &in_w0, &in_w3, &in_bin, &in_vin, &vr,
-              &vi, &q, &s, &vin64, &vin32, &stats, &partial, &counts, &offsets, &cursor, &dropped, &rec, &rec_s, &planes,
+              &vi, &q, &s, &vin64, &vin32, &stats, &partial, &zero, &offsets, &cursor, &counters, &rec, &rec_s, &planes,
               &corr, &image, &cheb_err, &bin_out, &grid_keep, &tc_status, &kb_offsets, &acc, &chunk_key, &keymax,
               &plan_buf, &scan_sums, &probe, &remade})
             n += b->cap;
@@ -243,7 +250,8 @@ struct svdi_engine {
         if (h_ndrop) cudaFreeHost(h_ndrop);
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_stats) cudaEventDestroy(ev_stats);
-        if (ev_vis) cudaEventDestroy(ev_vis);
+        for (cudaEvent_t ev : {ev_vis, ev_basis, ev_rows, ev_clear})
+            if (ev) cudaEventDestroy(ev);
         if (side) cudaStreamDestroy(side);
         if (stream && own_stream) cudaStreamDestroy(stream);
     }
@@ -266,6 +274,10 @@ int engine_init(svdi_engine* e, const svdi_options* opt) {
     SVDI_CUDA(cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming));
     SVDI_CUDA(cudaEventCreateWithFlags(&e->ev_vis, cudaEventDisableTiming));
     SVDI_CUDA(cudaEventCreateWithFlags(&e->ev_stats, cudaEventDisableTiming));
+    for (cudaEvent_t* ev : {&e->ev_basis, &e->ev_rows, &e->ev_clear})
+        SVDI_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
+    SVDI_TRY(e->counters.ensure(kCounterWords * sizeof(unsigned int)));
+    SVDI_CUDA(cudaMemsetAsync(e->counters.p, 0, kCounterWords * sizeof(unsigned int), e->stream));
     SVDI_CUDA(cudaMallocHost(&e->h_stats, (ST_COUNT + 9) * sizeof(double)));
     SVDI_CUDA(cudaMallocHost(&e->h_ndrop, 2 * sizeof(unsigned long long)));
     for (auto& ev : e->ev) SVDI_CUDA(cudaEventCreate(&ev));
@@ -659,6 +671,63 @@ bool plan_wplanes(svdi_engine* e, const SampleSource& src, long long G, const Sl
     return true;
 }
 
+// Gridder form, tiles and keys of a call with slab configuration sp.
+struct CallGeom {
+    GridGeom g{};
+    bool use_tc = false, use_i8 = false, use_mma = false;
+    int chunk = kGridChunk;  // records per chunk of the scan's table
+    int n_keys = 0;
+    size_t zero_words() const { return (size_t)kZeroCounts + (size_t)n_keys; }
+};
+int call_geom(const svdi_options& o, long long N, float cell_f, const SlabParams& sp, long long n, CallGeom& c) {
+    GridGeom& g = c.g;
+    g.G = grid_size(N, o.sigma);
+    g.gmin = -(g.G / 2);
+    g.gmax = (g.G - 1) / 2;
+    g.W = o.support;
+    // the tensor-core gridders accumulate one moment plane at a time in TMEM: the FP16 / BF16 form
+    // (K == 1) bins into 56 x 8 tiles (64 x 16 accumulator window, gridder_tc.cu), the integer form
+    // (any K, one launch per Chebyshev term) into 24 x 8 tiles (32 x 16 window, gridder_i8.cu);
+    // the integer form scales each key by its own max |value| from the scatter
+    c.use_tc = is_tc_gridder(o.gridder) && (sp.K == 1 || o.gridder == SVDI_GRIDDER_TC_I8) && g.W <= 8;
+    c.use_i8 = c.use_tc && o.gridder == SVDI_GRIDDER_TC_I8;
+    c.use_mma = !c.use_tc && use_mma_gridder(o, g.G, sp.nslab);
+    c.chunk = c.use_mma ? mma_chunk(n) : kGridChunk;
+    if (c.use_tc) {
+        tc_tiles(o.gridder, g);
+    } else {
+        fp32_tiles(c.use_mma ? kMmaTile : (o.tile ? o.tile : (sp.K == 1 ? 64 : 32)), g);
+    }
+    g.edge_mode = o.edge_mode;
+    g.coord_mode = o.coord_mode;
+    g.scale = (double)cell_f * (double)g.G;
+    g.scale32 = cell_f * (float)g.G;
+    const long long n_keys = (long long)sp.nslab * g.ntile * g.ntile2;
+    if (n_keys > (1LL << 26)) {
+        set_error("too many tile keys");
+        return SVDI_ERR_UNSUPPORTED;
+    }
+    c.n_keys = (int)n_keys;
+    return SVDI_OK;
+}
+
+// Whether a call can run on the previous call's slab and Chebyshev counts (`bslabs`: its slabs per batch).
+bool spec_usable(svdi_engine* e, bool archive, long long N, float cell_f, const SampleSource& src, size_t& bslabs) {
+    if (!(e->spec_valid && e->spec_archive == archive && e->spec_N == N && e->spec_cell == cell_f && e->spec_n == src.n &&
+          e->spec_R == src.R && e->spec_bin == (src.bin != nullptr)))
+        return false;
+    bslabs = batch_slabs_for(e, e->spec_sp.nslab, e->spec_sp.K, grid_size(N, e->opt.sigma));
+    return (int)bslabs >= e->spec_sp.nslab;  // one batch of all slabs only
+}
+
+// What main_path_device has queued before image_core: the decision to speculate (the device plan made by the
+// projection of the rows) and the clearing of `zero`.
+struct Prep {
+    bool spec = false, zeroed = false;
+    bool uploads = false;  // the side stream uploads the visibilities: nothing else waits behind them there
+    size_t bslabs = 0;
+};
+
 // The host decisions of one snapshot: everything image_core reads back from the device before
 // it can launch the gridding (basis determinant, w range, slab and Chebyshev configuration,
 // slabs per batch). With a fixed plan image_core issues device work only (no synchronisation,
@@ -778,10 +847,11 @@ int image_wplanes(svdi_engine* e, SampleSource src, const GridGeom& g, const Sla
     const size_t bslabs = batch_slabs_for(e, sp.nslab, sp.K, g.G);
     const int per = (int)std::min<size_t>((size_t)wp.P, bslabs * (size_t)sp.K);
     SVDI_TRY(e->planes.ensure(plane_bytes * per));
-    SVDI_TRY(e->dropped.ensure(16));
+    SVDI_TRY(e->zero.ensure(kZeroCounts * 4));
+    unsigned long long* const dropped = e->zero.as<unsigned long long>();
     SVDI_CUDA(cudaEventRecord(e->ev[1], st));
-    SVDI_CUDA(cudaMemsetAsync(e->dropped.p, 0, 16, st));
-    src.nonfinite = e->dropped.as<unsigned long long>() + 1;
+    SVDI_CUDA(cudaMemsetAsync(dropped, 0, 16, st));
+    src.nonfinite = dropped + 1;
     SVDI_CUDA(cudaEventRecord(e->ev[2], st));
     SVDI_TRY(ensure_corr(e, N, g.G, g.W, e->opt.beta));
     SVDI_CUDA(cudaMemsetAsync(d_out, 0, (size_t)N * N * sizeof(float), st));
@@ -799,7 +869,7 @@ int image_wplanes(svdi_engine* e, SampleSource src, const GridGeom& g, const Sla
         SVDI_CUDA(cudaMemsetAsync(e->planes.p, 0, plane_bytes * (hi - lo), st));
         if (lo == 0 && vis_ready) SVDI_CUDA(cudaStreamWaitEvent(st, vis_ready, 0));
         SVDI_TRY(launch_grid_w(src, g, wp, e->poly, e->wpoly, lo, hi, e->planes.as<float2>(),
-                               lo == 0 ? e->dropped.as<unsigned long long>() : nullptr, st));
+                               lo == 0 ? dropped : nullptr, st));
         SVDI_CUDA(cudaEventRecord(e->ev[4], st));
         SVDI_TRY(exec_fft(plan, e->planes.as<cufftComplex>(), hi - lo));
         SVDI_CUDA(cudaEventRecord(e->ev[5], st));
@@ -815,7 +885,7 @@ int image_wplanes(svdi_engine* e, SampleSource src, const GridGeom& g, const Sla
             ms[k] += t;
         }
     }
-    SVDI_CUDA(cudaMemcpyAsync(e->h_ndrop, e->dropped.p, 8, cudaMemcpyDeviceToHost, st));
+    SVDI_CUDA(cudaMemcpyAsync(e->h_ndrop, dropped, 8, cudaMemcpyDeviceToHost, st));
     record_call(e, src, g, sp, N, cell);
     record_stats(e, src, g, sp, sp.nslab * g.ntile * g.ntile2, false, alpha_max, slab_alpha, r3min, r3max, mt3);
     e->pending = true;
@@ -839,8 +909,11 @@ int image_wplanes(svdi_engine* e, SampleSource src, const GridGeom& g, const Sla
 int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, float cell_f,
                float* d_out, const ExecPlan* fixed = nullptr, ExecPlan* record = nullptr,
                unsigned int* d_status_out = nullptr, cudaEvent_t vis_ready = nullptr, bool allow_spec = true,
-               bool allow_w = true) {
+               bool allow_w = true, const Prep* prep = nullptr) {
     cudaStream_t st = e->stream;
+    // vis_ready: the side stream was forked from the main one for this call
+    const bool forked = vis_ready && !(prep && prep->uploads);
+    cudaStream_t side = forked ? e->side : st;
     const svdi_options& o = e->opt;
     const double cell = (double)cell_f;
     const long long n = src.n;
@@ -849,7 +922,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
     SlabParams sp{};
     double alpha_max = 0, slab_alpha = 0, r3min = 0, r3max = 0, mt3 = 0;
     const DevPlan* dplan = nullptr;  // speculative: slab geometry and 1 / |det| from the device
-    size_t spec_bslabs = 0;
+    size_t spec_bslabs = prep ? prep->bslabs : 0;
     if (fixed) {
         src.inv_det = fixed->inv_det;
         sp = fixed->sp;
@@ -859,59 +932,35 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
         r3max = fixed->r3max;
         mt3 = fixed->mt3;
     } else {
-        // statistics: max |t3|, then one small read
-        SVDI_TRY(launch_t3_stats(e->vin64.as<double>(), N, cell, e->partial.as<double>(), kPartialCap,
-                                 e->stats.as<double>(), st));
-        SVDI_CUDA(cudaMemcpyAsync(e->h_stats, e->stats.p, ST_COUNT * sizeof(double), cudaMemcpyDeviceToHost, st));
-        SVDI_CUDA(cudaMemcpyAsync(e->h_stats + ST_COUNT, e->vin64.p, 9 * sizeof(double), cudaMemcpyDeviceToHost, st));
-        bool spec = allow_spec && !record && e->spec_valid && e->spec_archive == archive && e->spec_N == N &&
-                    e->spec_cell == cell_f && e->spec_n == n && e->spec_R == src.R &&
-                    e->spec_bin == (src.bin != nullptr);
-        if (spec) {  // one batch of all slabs only
-            spec_bslabs = batch_slabs_for(e, e->spec_sp.nslab, e->spec_sp.K, grid_size(N, o.sigma));
-            spec = (int)spec_bslabs >= e->spec_sp.nslab;
-        }
+        // statistics: max |t3|, then one small read, beside the binning of a speculative call
+        if (forked) SVDI_CUDA(cudaStreamWaitEvent(side, e->ev_basis, 0));
+        SVDI_TRY(launch_t3_stats(e->vin64.as<double>(), N, cell, e->partial.as<double>() + 5 * kPartialCap, kPartialCap,
+                                 e->counters.as<unsigned int>() + 2, e->stats.as<double>(), side));
+        if (forked) SVDI_CUDA(cudaStreamWaitEvent(side, e->ev_rows, 0));
+        SVDI_CUDA(cudaMemcpyAsync(e->h_stats, e->stats.p, ST_COUNT * sizeof(double), cudaMemcpyDeviceToHost, side));
+        SVDI_CUDA(cudaMemcpyAsync(e->h_stats + ST_COUNT, e->vin64.p, 9 * sizeof(double), cudaMemcpyDeviceToHost, side));
+        SVDI_CUDA(cudaEventRecord(e->ev_stats, side));
+        const bool spec = prep ? prep->spec
+                               : allow_spec && !record && spec_usable(e, archive, N, cell_f, src, spec_bslabs);
         if (spec) {
-            SVDI_CUDA(cudaEventRecord(e->ev_stats, st));
             sp = e->spec_sp;
-            SVDI_TRY(e->plan_buf.ensure(sizeof(DevPlan)));
-            SVDI_TRY(launch_plan(e->stats.as<double>(), e->vin64.as<double>(), archive, sp.nslab, sp.K,
-                                 e->plan_buf.as<DevPlan>(), st));
+            if (!prep) {
+                SVDI_TRY(e->plan_buf.ensure(sizeof(DevPlan)));
+                SVDI_TRY(launch_plan(e->stats.as<double>(), e->vin64.as<double>(), archive, sp.nslab, sp.K,
+                                     e->plan_buf.as<DevPlan>(), st));
+            }
             dplan = e->plan_buf.as<DevPlan>();
         } else {
-            SVDI_CUDA(cudaStreamSynchronize(st));
+            SVDI_CUDA(cudaEventSynchronize(e->ev_stats));
             SVDI_TRY(host_decision(e, archive, src, sp, alpha_max, slab_alpha, r3min, r3max, mt3));
         }
     }
 
-    GridGeom g{};
-    g.G = grid_size(N, o.sigma);
-    g.gmin = -(g.G / 2);
-    g.gmax = (g.G - 1) / 2;
-    g.W = o.support;
-    // the tensor-core gridders accumulate one moment plane at a time in TMEM: the FP16 / BF16 form
-    // (K == 1) bins into 56 x 8 tiles (64 x 16 accumulator window, gridder_tc.cu), the integer form
-    // (any K, one launch per Chebyshev term) into 24 x 8 tiles (32 x 16 window, gridder_i8.cu);
-    // the integer form scales each key by its own max |value| from the scatter
-    const bool use_tc = is_tc_gridder(o.gridder) && (sp.K == 1 || o.gridder == SVDI_GRIDDER_TC_I8) && g.W <= 8;
-    const bool use_i8 = use_tc && o.gridder == SVDI_GRIDDER_TC_I8;
-    const bool use_mma = !use_tc && use_mma_gridder(o, g.G, sp.nslab);
-    const int chunk = use_mma ? mma_chunk(n) : kGridChunk;  // records per chunk of the scan's table
-    if (use_tc) {
-        tc_tiles(o.gridder, g);
-    } else {
-        fp32_tiles(use_mma ? kMmaTile : (o.tile ? o.tile : (sp.K == 1 ? 64 : 32)), g);
-    }
-    g.edge_mode = o.edge_mode;
-    g.coord_mode = o.coord_mode;
-    g.scale = cell * (double)g.G;
-    g.scale32 = cell_f * (float)g.G;
-    const long long n_keys_ll = (long long)sp.nslab * g.ntile * g.ntile2;
-    if (n_keys_ll > (1LL << 26)) {
-        set_error("too many tile keys");
-        return SVDI_ERR_UNSUPPORTED;
-    }
-    const int n_keys = (int)n_keys_ll;
+    CallGeom cg;
+    SVDI_TRY(call_geom(o, N, cell_f, sp, n, cg));
+    const GridGeom& g = cg.g;
+    const bool use_tc = cg.use_tc, use_i8 = cg.use_i8, use_mma = cg.use_mma;
+    const int chunk = cg.chunk, n_keys = cg.n_keys;
 
     if (e->poly_W != g.W || e->poly_beta != o.beta) {
         build_es_poly(g.W, o.beta, &e->poly);
@@ -924,25 +973,36 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
     if (e->last_w)
         return image_wplanes(e, src, g, sp, wp, N, cell, d_out, vis_ready, alpha_max, slab_alpha, r3min, r3max, mt3);
 
+    // the planes of the first slab batch and the image are cleared on the side stream, beside the binning
+    const size_t bslabs = fixed ? fixed->bslabs : (dplan ? spec_bslabs : batch_slabs_for(e, sp.nslab, sp.K, g.G));
+    const int planes_per_batch = (int)bslabs * sp.K;
+    const size_t plane_bytes = (size_t)g.G * g.G * sizeof(float2);
+    SVDI_TRY(e->planes.ensure(plane_bytes * planes_per_batch));
+    SVDI_CUDA(cudaMemsetAsync(e->planes.p, 0, plane_bytes * planes_per_batch, side));
+    SVDI_CUDA(cudaMemsetAsync(d_out, 0, (size_t)N * N * sizeof(float), side));
+    if (forked) SVDI_CUDA(cudaEventRecord(e->ev_clear, side));
+
     // binning
     if (timed) SVDI_CUDA(cudaEventRecord(e->ev[1], st));
-    SVDI_TRY(e->counts.ensure((size_t)n_keys * 4));
     SVDI_TRY(e->offsets.ensure((size_t)(n_keys + 1) * 4));
     SVDI_TRY(e->cursor.ensure((size_t)n_keys * 4));
-    SVDI_TRY(e->dropped.ensure(16));  // [0] dropped samples, [1] non-finite gridded values
     SVDI_TRY(e->rec.ensure((size_t)std::max<long long>(n, 1) * sizeof(SampleRec)));
     const bool need_s = sp.K > 1;
     if (need_s) SVDI_TRY(e->rec_s.ensure((size_t)std::max<long long>(n, 1) * sizeof(float)));
-    SVDI_CUDA(cudaMemsetAsync(e->counts.p, 0, (size_t)n_keys * 4, st));
-    SVDI_CUDA(cudaMemsetAsync(e->dropped.p, 0, 16, st));
+    if (!(prep && prep->zeroed)) {
+        SVDI_TRY(e->zero.ensure(cg.zero_words() * 4));
+        SVDI_CUDA(cudaMemsetAsync(e->zero.p, 0, cg.zero_words() * 4, st));
+    }
+    unsigned int* const counts = e->zero.as<unsigned int>() + kZeroCounts;
+    unsigned int* const work = e->zero.as<unsigned int>() + kZeroWork;
+    unsigned long long* const dropped = e->zero.as<unsigned long long>();  // dropped, non-finite samples
     // a NaN or Inf among the gridded values makes the image NaN, as the reference's float atomics
     // and FFT do (SVDIntegratedImager.cu:606-612 keeps NaN under a zero weight)
-    src.nonfinite = e->dropped.as<unsigned long long>() + 1;
-    SVDI_TRY(launch_histogram(src, g, sp, e->counts.as<unsigned int>(), n_keys,
-                              e->dropped.as<unsigned long long>(), st, dplan));
+    src.nonfinite = dropped + 1;
+    SVDI_TRY(launch_histogram(src, g, sp, counts, n_keys, dropped, st, dplan));
     if (use_tc) {
         SVDI_TRY(e->kb_offsets.ensure((size_t)(n_keys + 1) * 4));
-    } else {  // the FP32 gridders' chunk table, then the work counter
+    } else {  // the FP32 gridders' chunk table
         SVDI_TRY(e->chunk_key.ensure(((size_t)std::max<long long>(n, 1) / chunk + 2) * 4));
     }
     SVDI_TRY(e->scan_sums.ensure(scan_sums_words(n_keys) * 4));
@@ -951,7 +1011,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
         SVDI_TRY(e->keymax.ensure((size_t)n_keys * 4));
         SVDI_CUDA(cudaMemsetAsync(e->keymax.p, 0, (size_t)n_keys * 4, st));
     }
-    SVDI_TRY(launch_scan(e->counts.as<unsigned int>(), n_keys, e->offsets.as<unsigned int>(),
+    SVDI_TRY(launch_scan(counts, n_keys, e->offsets.as<unsigned int>(),
                          e->cursor.as<unsigned int>(), st,
                          use_tc ? e->kb_offsets.as<unsigned int>() : nullptr, kTcKBlock,
                          use_tc ? nullptr : e->chunk_key.as<unsigned int>(), chunk,
@@ -969,7 +1029,6 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
     if (timed) SVDI_CUDA(cudaEventRecord(e->ev[2], st));
 
     // slab batches: grid -> FFT -> recombine
-    const size_t bslabs = fixed ? fixed->bslabs : (dplan ? spec_bslabs : batch_slabs_for(e, sp.nslab, sp.K, g.G));
     if (record) {
         record->inv_det = src.inv_det;
         record->sp = sp;
@@ -980,13 +1039,9 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
         record->mt3 = mt3;
         record->bslabs = bslabs;
     }
-    const int planes_per_batch = (int)bslabs * sp.K;
-    const size_t plane_bytes = (size_t)g.G * g.G * sizeof(float2);
-    SVDI_TRY(e->planes.ensure(plane_bytes * planes_per_batch));
     FftPlan plan;
     SVDI_TRY(get_plan(e, g.G, N, planes_per_batch, plan));
     SVDI_TRY(ensure_corr(e, N, g.G, g.W, o.beta));
-    SVDI_CUDA(cudaMemsetAsync(d_out, 0, (size_t)N * N * sizeof(float), st));
     // slabs split over several batches: the signed sums of all batches before |.| (the reference
     // takes |.| per batch, SVDIntegratedImager.cu:1445, inside its batch loop at :1681)
     const bool multi_batch = (int)bslabs < sp.nslab;
@@ -998,8 +1053,9 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
     for (int s0 = 0; s0 < sp.nslab; s0 += (int)bslabs) {
         const int s1 = std::min(sp.nslab, s0 + (int)bslabs);
         SlabParams bp = sp;
+        if (s0 == 0 && forked) SVDI_CUDA(cudaStreamWaitEvent(st, e->ev_clear, 0));
         if (timed) SVDI_CUDA(cudaEventRecord(e->ev[3], st));
-        SVDI_CUDA(cudaMemsetAsync(e->planes.p, 0, plane_bytes * planes_per_batch, st));
+        if (s0 > 0) SVDI_CUDA(cudaMemsetAsync(e->planes.p, 0, plane_bytes * planes_per_batch, st));
         const int tiles2 = g.ntile * g.ntile2;
         if (use_i8) {
             SVDI_TRY(launch_grid_i8(e->rec.as<SampleRec>(), need_s ? e->rec_s.as<float>() : nullptr,
@@ -1015,16 +1071,13 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
                                     e->sm_count, st, o.gridder == SVDI_GRIDDER_TC_BF16));
         } else if (use_mma) {
             SVDI_TRY(launch_grid_mma(e->rec.as<SampleRec>(), need_s ? e->rec_s.as<float>() : nullptr,
-                                     e->offsets.as<unsigned int>(), e->chunk_key.as<unsigned int>(), chunk,
-                                     e->chunk_key.as<unsigned int>() + (size_t)std::max<long long>(n, 1) / chunk + 1,
-                                     n_keys, s0 * tiles2, s1 * tiles2, g, sp.K, e->poly, e->planes.as<float2>(),
+                                     e->offsets.as<unsigned int>(), e->chunk_key.as<unsigned int>(), chunk, work,
+                                     s0 == 0, n_keys, s0 * tiles2, s1 * tiles2, g, sp.K, e->poly, e->planes.as<float2>(),
                                      e->sm_count, st));
         } else {
             SVDI_TRY(launch_grid_fp32(e->rec.as<SampleRec>(), need_s ? e->rec_s.as<float>() : nullptr,
                                       e->offsets.as<unsigned int>(), e->chunk_key.as<unsigned int>(),
-                                      e->keymax.as<unsigned int>(),
-                                      e->chunk_key.as<unsigned int>() + (size_t)std::max<long long>(n, 1) / chunk + 1,
-                                      n_keys, s0 * tiles2, s1 * tiles2, s0, g,
+                                      e->keymax.as<unsigned int>(), work, n_keys, s0 * tiles2, s1 * tiles2, s0, g,
                                       sp, e->poly, e->planes.as<float2>(), e->sm_count, st));
         }
         if (o.keep_grid && s0 == 0) {
@@ -1065,7 +1118,8 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
         }
         if (real.nslab != sp.nslab || real.K != sp.K) {  // other counts: image again with them
             e->spec_valid = false;
-            return image_core(e, archive, src, N, cell_f, d_out, nullptr, nullptr, d_status_out, vis_ready, false, allow_w);
+            // on the main stream alone, behind the work of the first attempt (which waited for vis_ready)
+            return image_core(e, archive, src, N, cell_f, d_out, nullptr, nullptr, d_status_out, nullptr, false, allow_w);
         }
         sp = real;  // the same bits as the device plan (slab_params_for, basis_det)
     }
@@ -1090,7 +1144,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
         }
         return SVDI_OK;
     }
-    SVDI_CUDA(cudaMemcpyAsync(e->h_ndrop, e->dropped.p, 8, cudaMemcpyDeviceToHost, st));
+    SVDI_CUDA(cudaMemcpyAsync(e->h_ndrop, dropped, 8, cudaMemcpyDeviceToHost, st));
     if (use_tc) {  // the tensor-core gridder's give-up status is checked before the call returns
         unsigned int tc_status = 0;
         SVDI_CUDA(cudaMemcpyAsync(&tc_status, e->tc_status.p, 4, cudaMemcpyDeviceToHost, st));
@@ -1181,7 +1235,7 @@ int check_options(const svdi_options& o) {
 // Main path on device-resident raw snapshot arrays.
 int main_path_device(svdi_engine* e, const svdi_host_ms* d, size_t N, float cell, float* d_out,
                      const ExecPlan* fixed = nullptr, ExecPlan* record = nullptr,
-                     unsigned int* d_status_out = nullptr) {
+                     unsigned int* d_status_out = nullptr, bool uploads = false) {
     cudaStream_t st = e->stream;
     const long long R = (long long)d->num_rows, C = (long long)d->num_channels;
     const long long n = (long long)d->num_samples;
@@ -1201,9 +1255,6 @@ int main_path_device(svdi_engine* e, const svdi_host_ms* d, size_t N, float cell
     SVDI_TRY(launch_collapse(d->vis0_real, d->vis0_imag, d->vis3_real, d->vis3_imag, d->flag0, d->flag3,
                              d->weight0, d->weight3, e->vr.as<float>(), e->vi.as<float>(), n, e->side));
     SVDI_CUDA(cudaEventRecord(e->ev_vis, e->side));
-    SVDI_TRY(launch_preprocess(d->uvw, d->frequencies_hz, R, C, d->array_center_x, e->partial.as<double>(),
-                               kPartialCap, e->vin64.as<double>(), e->vin32.as<float>(), e->q.as<double>(),
-                               e->s.as<double>(), e->stats.as<double>(), st));
     SampleSource src{};
     src.q = e->q.as<double>();
     src.s = e->s.as<double>();
@@ -1213,7 +1264,26 @@ int main_path_device(svdi_engine* e, const svdi_host_ms* d, size_t N, float cell
     src.n = n;
     e->sz_q = (size_t)R * 24;
     e->sz_s = (size_t)C * 8;
-    SVDI_TRY(image_core(e, false, src, (long long)N, cell, d_out, fixed, record, d_status_out, e->ev_vis));
+    // a speculative call knows its plan's counts: the rotation clears the binning's counters and makes the
+    // device plan
+    Prep prep;
+    prep.uploads = uploads;
+    prep.spec = !fixed && !record && spec_usable(e, false, (long long)N, cell, src, prep.bslabs);
+    CallGeom cg;
+    if (prep.spec) {
+        SVDI_TRY(call_geom(e->opt, (long long)N, cell, e->spec_sp, n, cg));
+        SVDI_TRY(e->zero.ensure(cg.zero_words() * 4));
+        SVDI_TRY(e->plan_buf.ensure(sizeof(DevPlan)));
+        prep.zeroed = true;
+    }
+    SVDI_TRY(launch_preprocess(d->uvw, d->frequencies_hz, R, C, d->array_center_x, e->partial.as<double>(), kPartialCap,
+                               e->counters.as<unsigned int>(), e->vin64.as<double>(), e->vin32.as<float>(),
+                               e->q.as<double>(), e->s.as<double>(), e->stats.as<double>(), st, e->ev_basis,
+                               e->zero.as<unsigned int>(), prep.zeroed ? (long long)cg.zero_words() : 0,
+                               prep.spec ? e->plan_buf.as<DevPlan>() : nullptr, e->spec_sp.nslab, e->spec_sp.K));
+    SVDI_CUDA(cudaEventRecord(e->ev_rows, st));
+    SVDI_TRY(image_core(e, false, src, (long long)N, cell, d_out, fixed, record, d_status_out, e->ev_vis, true, true,
+                        &prep));
     if (fixed) return SVDI_OK;
     SVDI_CUDA(cudaEventRecord(e->ev[7], st));
     e->pending_total = true;  // preprocessing and total times are read with the other statistics
@@ -1441,7 +1511,7 @@ int svdi_engine_image_host(svdi_engine* e, const svdi_host_ms* h, size_t N, floa
     d.weight0 = e->in_w0.as<float>();
     d.weight3 = e->in_w3.as<float>();
     SVDI_TRY(e->image.ensure(N * N * 4));
-    SVDI_TRY(main_path_device(e, &d, N, cell, e->image.as<float>()));
+    SVDI_TRY(main_path_device(e, &d, N, cell, e->image.as<float>(), nullptr, nullptr, nullptr, true));
     SVDI_TRY(e->stager.d2h(dirty_image, e->image.p, N * N * 4, st));
     SVDI_TRY(finish_pending(e));
     return SVDI_OK;
@@ -1621,8 +1691,8 @@ int svdi_preprocess_measurement_set(const svdi_host_ms* h, svdi_device_buffers* 
                              e->in_w0.as<float>(), e->in_w3.as<float>(), e->vr.as<float>(), e->vi.as<float>(),
                              (long long)n, st));
     SVDI_TRY(launch_preprocess(e->in_uvw.as<float>(), e->in_freq.as<float>(), (long long)R, (long long)C,
-                               h->array_center_x, e->partial.as<double>(), kPartialCap, e->vin64.as<double>(),
-                               e->vin32.as<float>(), e->q.as<double>(), e->s.as<double>(), e->stats.as<double>(),
+                               h->array_center_x, e->partial.as<double>(), kPartialCap,
+                               e->counters.as<unsigned int>(), e->vin64.as<double>(), e->vin32.as<float>(), e->q.as<double>(), e->s.as<double>(), e->stats.as<double>(),
                                st));
     if (want_bin) {
         SVDI_TRY(e->bin_out.ensure(n * 12));
@@ -1719,7 +1789,7 @@ struct svdi_batch {
     // per Chebyshev order over the keys of all snapshots, one FFT over all moment planes).
     bool wide = false;
     svdi::DevBuf vr, vi, q, s, vin64, vin32, stats, partial, counts, offsets, cursor, keymax, chunk_key,
-        kb_offsets, rec, rec_s, planes, dropped, work, corr, scan_sums;
+        kb_offsets, rec, rec_s, planes, dropped, work, corr, scan_sums, counters;
     svdi::FftPlan fft;
     std::vector<cudaStream_t> lanes;
     std::vector<cudaEvent_t> lane_ev;
@@ -1864,6 +1934,8 @@ int wide_capture(svdi_batch* b) {
     SVDI_TRY(b->stats.ensure(B * ST_COUNT * 8));
     const int L = (int)std::min<size_t>(8, B);
     SVDI_TRY(b->partial.ensure((size_t)L * kPartialCap * 9 * 8));
+    SVDI_TRY(b->counters.ensure((size_t)L * kCounterWords * sizeof(unsigned int)));
+    SVDI_CUDA(cudaMemsetAsync(b->counters.p, 0, (size_t)L * kCounterWords * sizeof(unsigned int), e->stream));
     SVDI_TRY(b->counts.ensure((size_t)nkeys * 4));
     SVDI_TRY(b->offsets.ensure((size_t)(nkeys + 1) * 4));
     SVDI_TRY(b->cursor.ensure((size_t)nkeys * 4));
@@ -1934,7 +2006,7 @@ int wide_capture(svdi_batch* b) {
         SVDI_CUDA(cudaMemsetAsync(b->keymax.p, 0, (size_t)nkeys * 4, st));
         SVDI_CUDA(cudaMemsetAsync(b->dropped.p, 0, B * 2 * 8, st));
         SVDI_CUDA(cudaMemsetAsync(b->status.p, 0, (size_t)NG * 4 * sizeof(unsigned int), st));
-        SVDI_CUDA(cudaMemsetAsync(vmax, 0, sizeof(unsigned int), st));
+        SVDI_CUDA(cudaMemsetAsync(b->work.p, 0, 4 * sizeof(unsigned int) * (size_t)(NG + 1), st));  // vmax too
         SVDI_CUDA(cudaMemsetAsync(b->d_images, 0, B * NN * 4, st));
         // per snapshot: collapse, rotation, histogram
         SVDI_TRY(fork());
@@ -1947,7 +2019,8 @@ int wide_capture(svdi_batch* b) {
                                      (long long)d.num_samples, ls));
             SVDI_TRY(launch_preprocess(d.uvw, d.frequencies_hz, (long long)d.num_rows, (long long)d.num_channels,
                                        d.array_center_x, b->partial.as<double>() + (size_t)(s % L) * kPartialCap * 9,
-                                       kPartialCap, b->vin64.as<double>() + 9 * s, b->vin32.as<float>() + 9 * s,
+                                       kPartialCap, b->counters.as<unsigned int>() + (s % L) * kCounterWords,
+                                       b->vin64.as<double>() + 9 * s, b->vin32.as<float>() + 9 * s,
                                        b->q.as<double>() + 3 * row_off[s], b->s.as<double>() + chan_off[s],
                                        b->stats.as<double>() + ST_COUNT * s, ls));
             const SlabParams& sp = b->plans[s].sp;
@@ -1997,12 +2070,12 @@ int wide_capture(svdi_batch* b) {
             } else if (G.mma) {
                 SVDI_TRY(launch_grid_mma(b->rec.as<SampleRec>(), need_s ? b->rec_s.as<float>() : nullptr,
                                          b->offsets.as<unsigned int>(), b->chunk_key.as<unsigned int>(), chunk,
-                                         b->work.as<unsigned int>() + gi, (int)nkeys, (int)G.key_lo, (int)G.key_hi,
-                                         G.g, G.K, e->poly, pl, e->sm_count, st));
+                                         b->work.as<unsigned int>() + 4 * gi, true, (int)nkeys, (int)G.key_lo,
+                                         (int)G.key_hi, G.g, G.K, e->poly, pl, e->sm_count, st));
             } else {
                 SVDI_TRY(launch_grid_fp32(b->rec.as<SampleRec>(), need_s ? b->rec_s.as<float>() : nullptr,
                                           b->offsets.as<unsigned int>(), b->chunk_key.as<unsigned int>(),
-                                          b->keymax.as<unsigned int>(), b->work.as<unsigned int>() + gi, (int)nkeys,
+                                          b->keymax.as<unsigned int>(), b->work.as<unsigned int>() + 4 * gi, (int)nkeys,
                                           (int)G.key_lo, (int)G.key_hi, (int)G.slab_lo, G.g, sg, e->poly, pl,
                                           e->sm_count, st));
             }

@@ -573,7 +573,6 @@ int launch_kc(const SampleRec* d_rec, const float* d_rec_s, const unsigned int* 
     auto kern = k_grid_mma<W, KC>;
     const size_t smem = sizeof(WarpStage<KC>) * kWarps;
     SVDI_TRY(ensure_dynamic_smem((const void*)kern, smem, true));
-    SVDI_CUDA(cudaMemsetAsync(d_work, 0, sizeof(unsigned int), st));
     kern<<<sm_count * min_ctas<KC>(), 32 * kWarps, smem, st>>>(d_rec, d_rec_s, d_offsets, d_chunk_key, chunk, d_work,
                                                                key_lo, key_hi, g, fast_div(g.ntile * g.ntile2),
                                                                fast_div(g.ntile2), K, poly, d_planes, term_lo, groups);
@@ -593,12 +592,12 @@ int launch_w(const SampleRec* d_rec, const float* d_rec_s, const unsigned int* d
         t0 += 4 * n;
     }
     if (K - t0 >= 2) {
-        SVDI_TRY((launch_kc<W, 2>(d_rec, d_rec_s, d_offsets, d_chunk_key, chunk, d_work, key_lo, key_hi, g, K,
+        SVDI_TRY((launch_kc<W, 2>(d_rec, d_rec_s, d_offsets, d_chunk_key, chunk, d_work + 1, key_lo, key_hi, g, K,
                                   poly, d_planes, t0, 1, sm_count, st)));
         t0 += 2;
     }
     if (K - t0 >= 1)
-        SVDI_TRY((launch_kc<W, 1>(d_rec, d_rec_s, d_offsets, d_chunk_key, chunk, d_work, key_lo, key_hi, g, K,
+        SVDI_TRY((launch_kc<W, 1>(d_rec, d_rec_s, d_offsets, d_chunk_key, chunk, d_work + 2, key_lo, key_hi, g, K,
                                   poly, d_planes, t0, 1, sm_count, st)));
     return SVDI_OK;
 }
@@ -611,14 +610,15 @@ int launch_w(const SampleRec* d_rec, const float* d_rec_s, const unsigned int* d
 int mma_chunk(long long n) { return n >= 2000000 ? 256 : 64; }
 
 int launch_grid_mma(const SampleRec* d_rec, const float* d_rec_s, const unsigned int* d_offsets,
-                    const unsigned int* d_chunk_key, int chunk, unsigned int* d_work, int n_keys, int key_lo,
-                    int key_hi, const GridGeom& g, int K, const EsPoly& poly, float2* d_planes,
+                    const unsigned int* d_chunk_key, int chunk, unsigned int* d_work, bool work_cleared, int n_keys,
+                    int key_lo, int key_hi, const GridGeom& g, int K, const EsPoly& poly, float2* d_planes,
                     int sm_count, cudaStream_t st) {
     if (key_lo < 0 || key_hi > n_keys || key_lo >= key_hi || key_hi - key_lo > (1 << 26) || g.T != kMmaTile ||
         g.T2 != kMmaTile) {
         set_error("matrix gridder: bad key range or tile size");
         return SVDI_ERR_INTERNAL;
     }
+    if (!work_cleared) SVDI_CUDA(cudaMemsetAsync(d_work, 0, 3 * sizeof(unsigned int), st));
     MmaPoly p{};
     p.beta = poly.beta;
     for (int i = 0; i < g.W / 2; ++i)

@@ -32,10 +32,51 @@ __device__ inline void block_sum(T (&v)[N], T* smem /* [N][kThreads] */) {
     __syncthreads();
 }
 
-// Per-block partial sums of uvw (3) and uvw uvw^T (6) over rows.
-__global__ void __launch_bounds__(kThreads) k_row_moments(const float* __restrict__ uvw, long long R,
-                                                         double* __restrict__ partial) {
+// Block-wide minimum and maximum (all threads receive them); smem: 2 * kThreads doubles.
+__device__ inline void block_min_max(double& lo, double& hi, double* sm) {
+    const int t = threadIdx.x;
+    sm[t] = lo;
+    sm[kThreads + t] = hi;
+    __syncthreads();
+    for (int stride = kThreads / 2; stride > 0; stride >>= 1) {
+        if (t < stride) {
+            sm[t] = fmin(sm[t], sm[t + stride]);
+            sm[kThreads + t] = fmax(sm[kThreads + t], sm[kThreads + t + stride]);
+        }
+        __syncthreads();
+    }
+    lo = sm[0];
+    hi = sm[kThreads];
+    __syncthreads();
+}
+
+// True in every thread of the block that arrives last of the grid's (all blocks' earlier global writes are
+// visible to it). The counter returns to zero by itself.
+__device__ inline bool last_block(unsigned int* counter) {
+    __shared__ unsigned int ticket;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) ticket = atomicInc(counter, gridDim.x - 1);
+    __syncthreads();
+    const bool last = ticket == gridDim.x - 1;
+    if (last) __threadfence();
+    return last;
+}
+
+// Per-block partial sums of uvw (3) and uvw uvw^T (6) over rows; the last block reduces them, forms the
+// channel sums, the covariance, its eigenvectors and the basis. The first n_zero words of `zero` are cleared
+// on the way (the binning's counters). One launch for what used to be two kernels and two memsets: the
+// rotation, w range and plan took 36 of a 217 us call (130 k samples), almost all launch gaps.
+__global__ void __launch_bounds__(kThreads) k_row_basis(const float* __restrict__ uvw, long long R,
+                                                       double* __restrict__ partial, unsigned int* __restrict__ counter,
+                                                       const float* __restrict__ freq, long long C,
+                                                       float array_center_x, double* __restrict__ vin64,
+                                                       float* __restrict__ vin32, double* __restrict__ s_out,
+                                                       double* __restrict__ stats, unsigned int* __restrict__ zero,
+                                                       long long n_zero) {
     __shared__ double sm[9 * kThreads];
+    for (long long i = blockIdx.x * (long long)kThreads + threadIdx.x; i < n_zero; i += (long long)gridDim.x * kThreads)
+        zero[i] = 0u;
     double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     for (long long r = blockIdx.x * (long long)kThreads + threadIdx.x; r < R;
          r += (long long)gridDim.x * kThreads) {
@@ -47,18 +88,12 @@ __global__ void __launch_bounds__(kThreads) k_row_moments(const float* __restric
     block_sum<double, 9>(v, sm);
     if (threadIdx.x == 0)
         for (int k = 0; k < 9; ++k) partial[blockIdx.x * 9 + k] = v[k];
-}
+    if (!last_block(counter)) return;
 
-// One block: final reduction, channel sums, covariance, Jacobi, orientation.
-__global__ void __launch_bounds__(kThreads) k_basis(const double* __restrict__ partial, int nblocks,
-                                                   const float* __restrict__ freq, long long C,
-                                                   long long R, float array_center_x,
-                                                   double* __restrict__ vin64, float* __restrict__ vin32,
-                                                   double* __restrict__ s_out, double* __restrict__ stats) {
-    __shared__ double sm[9 * kThreads];
-    double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    const int nblocks = (int)gridDim.x;
+    for (int k = 0; k < 9; ++k) v[k] = 0.0;
     for (int b = threadIdx.x; b < nblocks; b += kThreads)
-        for (int k = 0; k < 9; ++k) v[k] += partial[b * 9 + k];
+        for (int k = 0; k < 9; ++k) v[k] += __ldcg(&partial[b * 9 + k]);
     block_sum<double, 9>(v, sm);
     double cs[2] = {0, 0};
     double smin = 1e300, smax = -1e300;
@@ -71,17 +106,7 @@ __global__ void __launch_bounds__(kThreads) k_basis(const double* __restrict__ p
         smax = fmax(smax, s);
     }
     block_sum<double, 2>(cs, sm);
-    // min / max of s
-    sm[threadIdx.x] = smin;
-    sm[kThreads + threadIdx.x] = smax;
-    __syncthreads();
-    for (int stride = kThreads / 2; stride > 0; stride >>= 1) {
-        if (threadIdx.x < stride) {
-            sm[threadIdx.x] = fmin(sm[threadIdx.x], sm[threadIdx.x + stride]);
-            sm[kThreads + threadIdx.x] = fmax(sm[kThreads + threadIdx.x], sm[kThreads + threadIdx.x + stride]);
-        }
-        __syncthreads();
-    }
+    block_min_max(smin, smax, sm);
     if (threadIdx.x == 0) {
         const double ns = (double)R * (double)C;
         double m[3], cov[9];
@@ -96,20 +121,29 @@ __global__ void __launch_bounds__(kThreads) k_basis(const double* __restrict__ p
             vin64[k] = vin[k];
             vin32[k] = (float)vin[k];
         }
-        stats[ST_S_MIN] = sm[0];
-        stats[ST_S_MAX] = sm[kThreads];
+        stats[ST_S_MIN] = smin;
+        stats[ST_S_MAX] = smax;
         stats[ST_EIG0] = ev[0];
         stats[ST_EIG1] = ev[1];
         stats[ST_EIG2] = ev[2];
     }
 }
 
-// q[row] = Vin . uvw_row (FP64) and per-block min/max of r3 = s * q3 over the row's channels.
+// The slab geometry and 1 / |det| of nslab slabs and K terms (one thread).
+__device__ inline void make_plan(const double* stats, const double* vin, int archive, int nslab, int K, DevPlan* plan) {
+    slab_params_for(archive != 0, nslab, K, stats[ST_R3_MIN], stats[ST_R3_MAX], plan->sp);
+    plan->inv_det = (float)(1.0 / basis_det(vin));  // inf or NaN for a degenerate basis, which the host rejects
+}
+
+// q[row] = Vin . uvw_row (FP64) and the min/max of r3 = s * q3 over rows and channels: per block, then the
+// last block over the blocks, which also makes the device plan when one is asked for.
 __global__ void __launch_bounds__(kThreads) k_project_rows(const float* __restrict__ uvw, long long R,
                                                           const double* __restrict__ vin,
-                                                          const double* __restrict__ stats,
+                                                          double* __restrict__ stats,
                                                           double* __restrict__ q,
-                                                          double* __restrict__ partial) {
+                                                          double* __restrict__ partial,
+                                                          unsigned int* __restrict__ counter, int nslab, int K,
+                                                          DevPlan* __restrict__ plan) {
     __shared__ double sm[2 * kThreads];
     double v[9];
     for (int k = 0; k < 9; ++k) v[k] = vin[k];
@@ -128,23 +162,27 @@ __global__ void __launch_bounds__(kThreads) k_project_rows(const float* __restri
         lo = fmin(lo, fmin(e0, e1));
         hi = fmax(hi, fmax(e0, e1));
     }
-    sm[threadIdx.x] = lo;
-    sm[kThreads + threadIdx.x] = hi;
-    __syncthreads();
-    for (int stride = kThreads / 2; stride > 0; stride >>= 1) {
-        if (threadIdx.x < stride) {
-            sm[threadIdx.x] = fmin(sm[threadIdx.x], sm[threadIdx.x + stride]);
-            sm[kThreads + threadIdx.x] = fmax(sm[kThreads + threadIdx.x], sm[kThreads + threadIdx.x + stride]);
-        }
-        __syncthreads();
-    }
+    block_min_max(lo, hi, sm);
     if (threadIdx.x == 0) {
-        partial[blockIdx.x * 2 + 0] = sm[0];
-        partial[blockIdx.x * 2 + 1] = sm[kThreads];
+        partial[blockIdx.x * 2 + 0] = lo;
+        partial[blockIdx.x * 2 + 1] = hi;
+    }
+    if (!last_block(counter)) return;
+    lo = 1e300;
+    hi = -1e300;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += kThreads) {
+        lo = fmin(lo, __ldcg(&partial[b * 2 + 0]));
+        hi = fmax(hi, __ldcg(&partial[b * 2 + 1]));
+    }
+    block_min_max(lo, hi, sm);
+    if (threadIdx.x == 0) {
+        stats[ST_R3_MIN] = lo;
+        stats[ST_R3_MAX] = hi;
+        if (plan) make_plan(stats, vin, 0, nslab, K, plan);
     }
 }
 
-// Final min/max of r3 partials -> stats.
+// Final min/max of r3 partials -> stats (archive path).
 __global__ void __launch_bounds__(kThreads) k_minmax_final(const double* __restrict__ partial, int nblocks,
                                                           double* __restrict__ stats) {
     __shared__ double sm[2 * kThreads];
@@ -153,19 +191,10 @@ __global__ void __launch_bounds__(kThreads) k_minmax_final(const double* __restr
         lo = fmin(lo, partial[b * 2 + 0]);
         hi = fmax(hi, partial[b * 2 + 1]);
     }
-    sm[threadIdx.x] = lo;
-    sm[kThreads + threadIdx.x] = hi;
-    __syncthreads();
-    for (int stride = kThreads / 2; stride > 0; stride >>= 1) {
-        if (threadIdx.x < stride) {
-            sm[threadIdx.x] = fmin(sm[threadIdx.x], sm[threadIdx.x + stride]);
-            sm[kThreads + threadIdx.x] = fmax(sm[kThreads + threadIdx.x], sm[kThreads + threadIdx.x + stride]);
-        }
-        __syncthreads();
-    }
+    block_min_max(lo, hi, sm);
     if (threadIdx.x == 0) {
-        stats[ST_R3_MIN] = sm[0];
-        stats[ST_R3_MAX] = sm[kThreads];
+        stats[ST_R3_MIN] = lo;
+        stats[ST_R3_MAX] = hi;
     }
 }
 
@@ -268,19 +297,10 @@ __global__ void __launch_bounds__(kThreads) k_bin_r3(const float* __restrict__ b
         lo = fmin(lo, r3);
         hi = fmax(hi, r3);
     }
-    sm[threadIdx.x] = lo;
-    sm[kThreads + threadIdx.x] = hi;
-    __syncthreads();
-    for (int stride = kThreads / 2; stride > 0; stride >>= 1) {
-        if (threadIdx.x < stride) {
-            sm[threadIdx.x] = fmin(sm[threadIdx.x], sm[threadIdx.x + stride]);
-            sm[kThreads + threadIdx.x] = fmax(sm[kThreads + threadIdx.x], sm[kThreads + threadIdx.x + stride]);
-        }
-        __syncthreads();
-    }
+    block_min_max(lo, hi, sm);
     if (threadIdx.x == 0) {
-        partial[blockIdx.x * 2 + 0] = sm[0];
-        partial[blockIdx.x * 2 + 1] = sm[kThreads];
+        partial[blockIdx.x * 2 + 0] = lo;
+        partial[blockIdx.x * 2 + 1] = hi;
     }
 }
 
@@ -290,17 +310,18 @@ __global__ void k_vin_from_float(const float* __restrict__ v32, double* __restri
 
 // max |t3| and the valid-pixel count over the N x N rotated-frame pixels
 // (SVDIntegratedImager.cu:1029-1077), FP64, pixel offsets from the integer image centre.
-// max |t3| and the valid-pixel count over the image. t3 = -v33 + sgn(v33) sqrt(ra) is monotone in
-// the radicand ra (FP64 square root and subtraction of a constant preserve order), so the largest
-// |t3| sits at the smallest or the largest valid radicand: the pixel loop keeps only those two and
-// the final reduction takes the square roots (the same values the per-pixel form would produce).
-// Rows are spread over blocks and columns over threads (no 64-bit division per pixel).
+// t3 = -v33 + sgn(v33) sqrt(ra) is monotone in the radicand ra (FP64 square root and subtraction of a
+// constant preserve order), so the largest |t3| sits at the smallest or the largest valid radicand: the
+// pixel loop keeps only those two and the last block takes the square roots (the same values the
+// per-pixel form would produce). Rows are spread over blocks and columns over threads (no 64-bit division
+// per pixel).
 __global__ void __launch_bounds__(kThreads) k_t3_stats(const double* __restrict__ vin, long long N, double cell,
-                                                      double* __restrict__ partial) {
-    __shared__ double sm[3 * kThreads];
+                                                      double* __restrict__ partial, unsigned int* __restrict__ counter,
+                                                      double* __restrict__ stats) {
+    __shared__ double sm[2 * kThreads];
     const double v13 = vin[2], v23 = vin[5];
     const long long half = N / 2;
-    double lo = 2.0, hi = -1.0, cnt = 0.0;  // radicands lie in [0, 1]
+    double lo = 2.0, hi = -1.0, cnt[1] = {0.0};  // radicands lie in [0, 1]
     for (long long y = blockIdx.x; y < N; y += gridDim.x) {
         const double t1 = cell * (double)(y - half) + v13;
         const double r1 = 1.0 - t1 * t1;
@@ -310,57 +331,34 @@ __global__ void __launch_bounds__(kThreads) k_t3_stats(const double* __restrict_
             if (ra >= 0.0) {
                 lo = fmin(lo, ra);
                 hi = fmax(hi, ra);
-                cnt += 1.0;
+                cnt[0] += 1.0;
             }
         }
     }
-    sm[threadIdx.x] = lo;
-    sm[kThreads + threadIdx.x] = hi;
-    sm[2 * kThreads + threadIdx.x] = cnt;
-    __syncthreads();
-    for (int stride = kThreads / 2; stride > 0; stride >>= 1) {
-        if (threadIdx.x < stride) {
-            sm[threadIdx.x] = fmin(sm[threadIdx.x], sm[threadIdx.x + stride]);
-            sm[kThreads + threadIdx.x] = fmax(sm[kThreads + threadIdx.x], sm[kThreads + threadIdx.x + stride]);
-            sm[2 * kThreads + threadIdx.x] += sm[2 * kThreads + threadIdx.x + stride];
-        }
-        __syncthreads();
-    }
+    block_min_max(lo, hi, sm);
+    block_sum<double, 1>(cnt, sm);
     if (threadIdx.x == 0) {
-        partial[blockIdx.x * 3 + 0] = sm[0];
-        partial[blockIdx.x * 3 + 1] = sm[kThreads];
-        partial[blockIdx.x * 3 + 2] = sm[2 * kThreads];
+        partial[blockIdx.x * 3 + 0] = lo;
+        partial[blockIdx.x * 3 + 1] = hi;
+        partial[blockIdx.x * 3 + 2] = cnt[0];
     }
-}
-
-__global__ void __launch_bounds__(kThreads) k_t3_final(const double* __restrict__ partial, int nblocks,
-                                                      const double* __restrict__ vin, double* __restrict__ stats) {
-    __shared__ double sm[3 * kThreads];
-    double lo = 2.0, hi = -1.0, cnt = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += kThreads) {
-        lo = fmin(lo, partial[b * 3 + 0]);
-        hi = fmax(hi, partial[b * 3 + 1]);
-        cnt += partial[b * 3 + 2];
+    if (!last_block(counter)) return;
+    lo = 2.0;
+    hi = -1.0;
+    cnt[0] = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += kThreads) {
+        lo = fmin(lo, __ldcg(&partial[b * 3 + 0]));
+        hi = fmax(hi, __ldcg(&partial[b * 3 + 1]));
+        cnt[0] += __ldcg(&partial[b * 3 + 2]);
     }
-    sm[threadIdx.x] = lo;
-    sm[kThreads + threadIdx.x] = hi;
-    sm[2 * kThreads + threadIdx.x] = cnt;
-    __syncthreads();
-    for (int stride = kThreads / 2; stride > 0; stride >>= 1) {
-        if (threadIdx.x < stride) {
-            sm[threadIdx.x] = fmin(sm[threadIdx.x], sm[threadIdx.x + stride]);
-            sm[kThreads + threadIdx.x] = fmax(sm[kThreads + threadIdx.x], sm[kThreads + threadIdx.x + stride]);
-            sm[2 * kThreads + threadIdx.x] += sm[2 * kThreads + threadIdx.x + stride];
-        }
-        __syncthreads();
-    }
+    block_min_max(lo, hi, sm);
+    block_sum<double, 1>(cnt, sm);
     if (threadIdx.x == 0) {
         const double v33 = vin[8], sg = v33 >= 0.0 ? 1.0 : -1.0;
         double mx = 0.0;
-        if (sm[2 * kThreads] > 0.0)
-            mx = fmax(fabs(-v33 + sg * sqrt(sm[0])), fabs(-v33 + sg * sqrt(sm[kThreads])));
+        if (cnt[0] > 0.0) mx = fmax(fabs(-v33 + sg * sqrt(lo)), fabs(-v33 + sg * sqrt(hi)));
         stats[ST_MAX_T3] = mx;
-        stats[ST_VALID_PIX] = sm[2 * kThreads];
+        stats[ST_VALID_PIX] = cnt[0];
     }
 }
 
@@ -432,16 +430,18 @@ int grid_for(long long n, int cap) {
 }  // namespace
 
 int launch_preprocess(const float* d_uvw, const float* d_freq, long long R, long long C,
-                      float array_center_x, double* d_partial, int partial_cap, double* d_vin64,
-                      float* d_vin32, double* d_q, double* d_s, double* d_stats, cudaStream_t st) {
-    const int nb = grid_for(R, partial_cap);
-    k_row_moments<<<nb, kThreads, 0, st>>>(d_uvw, R, d_partial);
+                      float array_center_x, double* d_partial, int partial_cap, unsigned int* d_counters,
+                      double* d_vin64, float* d_vin32, double* d_q, double* d_s, double* d_stats, cudaStream_t st,
+                      cudaEvent_t after_basis, unsigned int* d_zero, long long n_zero, DevPlan* d_plan, int nslab,
+                      int K) {
+    // a block per SM at most: the last block's serial part grows with their number
+    const int nb = grid_for(R, std::min(partial_cap, current_sm_count()));
+    k_row_basis<<<nb, kThreads, 0, st>>>(d_uvw, R, d_partial, d_counters, d_freq, C, array_center_x, d_vin64, d_vin32,
+                                         d_s, d_stats, d_zero, n_zero);
     SVDI_LAUNCHED();
-    k_basis<<<1, kThreads, 0, st>>>(d_partial, nb, d_freq, C, R, array_center_x, d_vin64, d_vin32, d_s, d_stats);
-    SVDI_LAUNCHED();
-    k_project_rows<<<nb, kThreads, 0, st>>>(d_uvw, R, d_vin64, d_stats, d_q, d_partial);
-    SVDI_LAUNCHED();
-    k_minmax_final<<<1, kThreads, 0, st>>>(d_partial, nb, d_stats);
+    if (after_basis) SVDI_CUDA(cudaEventRecord(after_basis, st));
+    k_project_rows<<<grid_for(R, 4 * current_sm_count()), kThreads, 0, st>>>(d_uvw, R, d_vin64, d_stats, d_q, d_partial,
+                                                                            d_counters + 1, nslab, K, d_plan);
     SVDI_LAUNCHED();
     return SVDI_OK;
 }
@@ -493,20 +493,17 @@ int launch_vin_from_float(const float* d_vin32, double* d_vin64, cudaStream_t st
 }
 
 int launch_t3_stats(const double* d_vin64, long long N, double cell, double* d_partial,
-                    int partial_cap, double* d_stats, cudaStream_t st) {
-    const int nb = (int)std::max<long long>(1, std::min<long long>(N, partial_cap));  // one row per block and step
-    k_t3_stats<<<nb, kThreads, 0, st>>>(d_vin64, N, cell, d_partial);
-    SVDI_LAUNCHED();
-    k_t3_final<<<1, kThreads, 0, st>>>(d_partial, nb, d_vin64, d_stats);
+                    int partial_cap, unsigned int* d_counter, double* d_stats, cudaStream_t st) {
+    const long long cap = std::min<long long>(partial_cap, 4LL * current_sm_count());
+    const int nb = (int)std::max<long long>(1, std::min<long long>(N, cap));  // one row per block and step
+    k_t3_stats<<<nb, kThreads, 0, st>>>(d_vin64, N, cell, d_partial, d_counter, d_stats);
     SVDI_LAUNCHED();
     return SVDI_OK;
 }
 
 __global__ void k_plan(const double* __restrict__ stats, const double* __restrict__ vin, int archive,
                        int nslab, int K, DevPlan* __restrict__ plan) {
-    if (threadIdx.x != 0) return;
-    slab_params_for(archive != 0, nslab, K, stats[ST_R3_MIN], stats[ST_R3_MAX], plan->sp);
-    plan->inv_det = (float)(1.0 / basis_det(vin));  // inf or NaN for a degenerate basis, which the host rejects
+    if (threadIdx.x == 0) make_plan(stats, vin, archive, nslab, K, plan);
 }
 
 int launch_plan(const double* d_stats, const double* d_vin64, bool archive, int nslab, int K,

@@ -149,9 +149,15 @@ int current_sm_count();
 
 // ---- kernel launchers (stream-ordered, no synchronisation) ---------------------------------
 // preprocess.cu
+// d_counters: two words, zero before the first launch on the buffer (each launch leaves them zero); launches
+// that may overlap need their own counters and partials. after_basis (optional): recorded once Vin is known.
+// d_zero: n_zero words cleared before the launch's end. d_plan (optional): the device plan of nslab slabs and K
+// terms.
 int launch_preprocess(const float* d_uvw, const float* d_freq, long long R, long long C,
-                      float array_center_x, double* d_partial, int partial_cap, double* d_vin64,
-                      float* d_vin32, double* d_q, double* d_s, double* d_stats, cudaStream_t st);
+                      float array_center_x, double* d_partial, int partial_cap, unsigned int* d_counters,
+                      double* d_vin64, float* d_vin32, double* d_q, double* d_s, double* d_stats, cudaStream_t st,
+                      cudaEvent_t after_basis = nullptr, unsigned int* d_zero = nullptr, long long n_zero = 0,
+                      DevPlan* d_plan = nullptr, int nslab = 0, int K = 0);
 int launch_collapse(const float* v0r, const float* v0i, const float* v3r, const float* v3i,
                     const uint8_t* f0, const uint8_t* f3, const float* w0, const float* w3,
                     float* outr, float* outi, long long n, cudaStream_t st);
@@ -161,7 +167,7 @@ int launch_bin_stats(const float* d_bin, long long n, double* d_partial, int par
                      double* d_stats, cudaStream_t st);
 int launch_vin_from_float(const float* d_vin32, double* d_vin64, cudaStream_t st);
 int launch_t3_stats(const double* d_vin64, long long N, double cell, double* d_partial,
-                    int partial_cap, double* d_stats, cudaStream_t st);
+                    int partial_cap, unsigned int* d_counter, double* d_stats, cudaStream_t st);
 int launch_cheb_errors(double amax, int na, int ns, int kmax, unsigned long long* d_err,
                        cudaStream_t st);
 // The device plan for nslab slabs and K terms from the statistics (ST_R3_MIN, ST_R3_MAX) and Vin.
@@ -298,10 +304,11 @@ constexpr int kMmaTile = 8;
 // records per chunk of the scan's table for n records (a power of two, at least kMmaChunkMin)
 constexpr int kMmaChunkMin = 64;
 int mma_chunk(long long n);
-// key_lo: the first tile of a slab; its planes come first in d_planes
+// key_lo: the first tile of a slab; its planes come first in d_planes. d_work: three counters, cleared here
+// unless work_cleared
 int launch_grid_mma(const SampleRec* d_rec, const float* d_rec_s, const unsigned int* d_offsets,
-                    const unsigned int* d_chunk_key, int chunk, unsigned int* d_work, int n_keys, int key_lo,
-                    int key_hi, const GridGeom& g, int K, const EsPoly& poly, float2* d_planes,
+                    const unsigned int* d_chunk_key, int chunk, unsigned int* d_work, bool work_cleared, int n_keys,
+                    int key_lo, int key_hi, const GridGeom& g, int K, const EsPoly& poly, float2* d_planes,
                     int sm_count, cudaStream_t st);
 
 // wplanes.cu: imaging through P w planes w_p = lo + (p - (W / 2 - 1)) dw (even grid sizes, support 6 or 8)
