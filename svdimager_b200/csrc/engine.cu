@@ -431,9 +431,9 @@ int choose_slabs(svdi_engine* e, bool archive, double r3min, double r3max, doubl
 // every row (length G, contiguous) is transformed, then only the N columns it reads (the checkerboard
 // sign centres the transform, so pixel x reads column G / 2 + x - N / 2: one contiguous run) are
 // transformed along the rows' stride. The second pass does N / G of the full 2-D transform's work
-// there; the other columns keep their first-pass values and are never read. For G = 2^a 3^b
-// (b <= 1, up to 12288) the column pass is this library's shared-memory transform (fft_cols.cu: a
-// CTA per block of adjacent columns, one launch over all planes); other 2,3,5,7-smooth sizes use a
+// there; the other columns keep their first-pass values and are never read. For even 2,3,5,7-smooth G
+// up to 12288 the column pass is this library's shared-memory transform (fft_cols.cu: a
+// CTA per block of adjacent columns, one launch over all planes); other smooth sizes use a
 // strided cuFFT column plan per plane. Grid sizes with a prime factor above 7 (cuFFT's Bluestein
 // path, which gave wrong in-place results for the interleaved column batches on B200) keep one 2-D
 // plan.
@@ -445,7 +445,7 @@ int make_fft_plan(long long G, long long N, int batch, cudaStream_t st, FftPlan&
     if (r == 1) {
         SVDI_CUFFT(cufftPlanMany(&plan.rows, 1, &n, &n, 1, n, &n, 1, n, CUFFT_C2C, (int)(G * batch)));
         if (col_fft_supported(G)) {
-            SVDI_TRY(make_col_fft(G, plan.cp, &plan.d_tw, &plan.d_perm));
+            SVDI_TRY(make_col_fft(G, N * batch, plan.cp, &plan.d_tw, &plan.d_perm));
             plan.mode = FftPlan::kRowsSharedCols;
         } else {
             SVDI_CUFFT(cufftPlanMany(&plan.cols, 1, &n, &n, n, 1, &n, n, 1, CUFFT_C2C, (int)N));

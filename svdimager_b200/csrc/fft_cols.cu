@@ -1,18 +1,18 @@
 // Second pass of the pruned inverse 2-D FFT: the column transforms of the N columns the
-// recombination reads, in shared memory, for grid sizes G = 2^a 3^b (b <= 1, 16 <= G <= 12288).
+// recombination reads, in shared memory, for grid sizes G = 2^a 3^b 5^c 7^d, 16 <= G <= 12288.
 //
 // cuFFT transforms a strided column batch of a large plane at a fraction of the bandwidth of its
 // contiguous row transforms (6144-row columns: ~1.1 TB/s). Here a CTA takes CB adjacent columns
-// whole (G x CB complex values, CB * 8-byte row segments, up to 192 KB of shared memory), runs an
-// in-place mixed-radix decimation-in-frequency FFT over the rows -- one radix-3 pass first (when
-// 3 | G), then radix-16 passes, then one radix-2/4/8 pass -- and writes each output row back from
-// its digit-reversed position. Pass p with radix R and stride S (the product of the later radices,
-// a power of two) takes the R elements b R S + j + S m (m < R) of a column, forms their inverse DFT
+// whole (G x CB complex values, CB * 8-byte row segments, up to 192 KB of shared memory) and runs a
+// mixed-radix decimation-in-frequency FFT over the rows. Pass p with radix R and stride S (the product of
+// the later radices) takes the R elements b R S + j + S m (m < R) of a column, forms their inverse DFT
 // (e^{+2 pi i m k / R}), multiplies element k by e^{+2 pi i j k / (R S)} and writes it back to
-// b R S + j + S k. The twiddles come from a table of e^{+2 pi i t / G} (FP64-rounded), element k of
-// pass p reading entry j k G / (R S) (< G); the output permutation is a table too (the output row
-// of each block row, so the block is read back in order). The transform is the inverse,
-// unnormalised one, as cuFFT's CUFFT_INVERSE.
+// b R S + j + S k. The block comes in by asynchronous copies, all of them in flight at once (a first pass
+// straight from the plane, a radix of loads per thread at a time, was slower: 6144 rows 0.33 -> 0.42 ms per
+// plane); the last pass writes the output rows (a table gives the output row of each block row) straight to the
+// plane. The twiddles come from a table of e^{+2 pi i t / G} (FP64-rounded), element k of
+// pass p reading entry j k G / (R S) (< G). The transform is the inverse, unnormalised one, as cuFFT's
+// CUFFT_INVERSE.
 //
 // Shared-memory rows are swizzled: block row r sits at row r ^ (f(r >> 3) & mask), f(x) = x ^
 // (x >> 2) ^ (x >> 4), mask = 16 / CB - 1 (the rows that share a 128-byte bank line). The last
@@ -50,6 +50,47 @@ __device__ __forceinline__ void dft3(float2& a, float2& b, float2& c) {
     a = c_add(a, t1);
     b = c_add(m, r);
     c = c_sub(m, r);
+}
+
+__device__ __forceinline__ void dft5(float2& a, float2& b, float2& c, float2& d, float2& e) {
+    constexpr float kC1 = 0.309016994374947424f, kC2 = -0.809016994374947424f;  // cos(2 pi / 5), cos(4 pi / 5)
+    constexpr float kS1 = 0.951056516295153572f, kS2 = 0.587785252292473129f;   // sines
+    const float2 p1 = c_add(b, e), q1 = c_sub(b, e), p2 = c_add(c, d), q2 = c_sub(c, d);
+    const float2 x = make_float2(a.x + kC1 * p1.x + kC2 * p2.x, a.y + kC1 * p1.y + kC2 * p2.y);
+    const float2 y = make_float2(a.x + kC2 * p1.x + kC1 * p2.x, a.y + kC2 * p1.y + kC1 * p2.y);
+    const float2 u = make_float2(-(kS1 * q1.y + kS2 * q2.y), kS1 * q1.x + kS2 * q2.x);  // i (S1 q1 + S2 q2)
+    const float2 v = make_float2(-(kS2 * q1.y - kS1 * q2.y), kS2 * q1.x - kS1 * q2.x);  // i (S2 q1 - S1 q2)
+    a = c_add(a, c_add(p1, p2));
+    b = c_add(x, u);
+    e = c_sub(x, u);
+    c = c_add(y, v);
+    d = c_sub(y, v);
+}
+
+__device__ __forceinline__ void dft7(float2 (&v)[16]) {
+    constexpr float kC[3] = {0.623489801858733531f, -0.222520933956314404f, -0.900968867902419126f};
+    constexpr float kS[3] = {0.781831482468029809f, 0.974927912181823607f, 0.433883739117558120f};
+    float2 p[3], q[3];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+        p[m] = c_add(v[m + 1], v[6 - m]);
+        q[m] = c_sub(v[m + 1], v[6 - m]);
+    }
+    const float2 a = v[0];
+    v[0] = c_add(a, c_add(p[0], c_add(p[1], p[2])));
+#pragma unroll
+    for (int k = 1; k <= 3; ++k) {
+        float2 x = a, u = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int m = 1; m <= 3; ++m) {
+            const int t = (k * m) % 7, i = t <= 3 ? t : 7 - t;  // cos and |sin| of 2 pi t / 7
+            const float c = kC[i - 1], sn = t <= 3 ? kS[i - 1] : -kS[i - 1];
+            x = make_float2(fmaf(c, p[m - 1].x, x.x), fmaf(c, p[m - 1].y, x.y));
+            u = make_float2(fmaf(-sn, q[m - 1].y, u.x), fmaf(sn, q[m - 1].x, u.y));
+        }
+        v[k] = c_add(x, u);
+        v[7 - k] = c_sub(x, u);
+    }
 }
 
 __device__ __forceinline__ void dft4(float2& a, float2& b, float2& c, float2& d) {
@@ -107,12 +148,35 @@ __device__ __forceinline__ void dft16(float2 (&v)[16]) {
     t = v[11]; v[11] = v[14]; v[14] = t;
 }
 
+__device__ __forceinline__ void dft9(float2 (&v)[16]) {
+    // x[b + 3 a]: radix-3 DFTs over a, twiddles e^{+2 pi i b k1 / 9}, radix-3 over b: y[k1 + 3 k2]
+#pragma unroll
+    for (int b = 0; b < 3; ++b) dft3(v[b], v[b + 3], v[b + 6]);
+    constexpr float kC1 = 0.766044443118978035f, kS1 = 0.642787609686539326f;  // 2 pi / 9
+    constexpr float kC2 = 0.173648177666930349f, kS2 = 0.984807753012208059f;  // 4 pi / 9
+    constexpr float kC4 = -0.939692620785908384f, kS4 = 0.342020143325668733f; // 8 pi / 9
+    v[4] = c_mul(v[4], make_float2(kC1, kS1));  // b 1, k1 1
+    v[7] = c_mul(v[7], make_float2(kC2, kS2));  // b 1, k1 2
+    v[5] = c_mul(v[5], make_float2(kC2, kS2));  // b 2, k1 1
+    v[8] = c_mul(v[8], make_float2(kC4, kS4));  // b 2, k1 2
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) dft3(v[3 * k1], v[3 * k1 + 1], v[3 * k1 + 2]);
+    // y[k1 + 3 k2] now sits in v[3 k1 + k2]: transpose the 3 x 3 index
+    float2 t;
+    t = v[1]; v[1] = v[3]; v[3] = t;
+    t = v[2]; v[2] = v[6]; v[6] = t;
+    t = v[5]; v[5] = v[7]; v[7] = t;
+}
+
 template <int R>
 __device__ __forceinline__ void dft_r(float2 (&v)[16]) {
     if constexpr (R == 2) dft2(v[0], v[1]);
     else if constexpr (R == 3) dft3(v[0], v[1], v[2]);
     else if constexpr (R == 4) dft4(v[0], v[1], v[2], v[3]);
+    else if constexpr (R == 5) dft5(v[0], v[1], v[2], v[3], v[4]);
+    else if constexpr (R == 7) dft7(v);
     else if constexpr (R == 8) dft8(v);
+    else if constexpr (R == 9) dft9(v);
     else dft16(v);
 }
 
@@ -132,18 +196,49 @@ __device__ __forceinline__ int srow(int r, int mask) {
     return r ^ ((x ^ (x >> 2) ^ (x >> 4)) & mask);
 }
 
-// one pass of radix R over the CTA's G x CB block (see the file comment)
-template <int R, int NT>
-__device__ __forceinline__ void col_pass(float2* __restrict__ sh, int G, int lcb, int s_log, int tw_step,
-                                         const float2* __restrict__ tw) {
-    // a thread takes one butterfly of two adjacent columns: 16-byte shared-memory accesses and
-    // the twiddles loaded once for both
-    const int S = 1 << s_log, CP = 1 << (lcb - 1);
+// The CTA's columns in the plane: `pl` the first of them, ncb of them inside the run; pairs of columns are
+// read and written as 16 bytes where both lie in it and are aligned (al16).
+struct Columns {
+    float2* pl;
+    long long G;
+    int ncb;
+    bool al16;
+    // columns past the block's end are zero
+    __device__ __forceinline__ void load(float2* dst, long long row, int c) const {
+        const float2* p = pl + row * G + c;
+        if (al16 && c + 1 < ncb) {
+            cp_async16(dst, p);
+        } else {
+            if (c < ncb) cp_async8(dst, p);
+            else dst[0] = make_float2(0.0f, 0.0f);
+            if (c + 1 < ncb) cp_async8(dst + 1, p + 1);
+            else dst[1] = make_float2(0.0f, 0.0f);
+        }
+    }
+    __device__ __forceinline__ void store(long long row, int c, float2 a, float2 b) const {
+        float2* p = pl + row * G + c;
+        if (al16 && c + 1 < ncb) {
+            *reinterpret_cast<float4*>(p) = make_float4(a.x, a.y, b.x, b.y);
+        } else {
+            if (c < ncb) p[0] = a;
+            if (c + 1 < ncb) p[1] = b;
+        }
+    }
+};
+
+// one pass of radix R over the CTA's G x CB block (see the file comment); LAST: to the plane
+template <int R, int NT, bool LAST>
+__device__ __forceinline__ void col_pass(float2* __restrict__ sh, const Columns& cols, int G, int lcb,
+                                         const ColFftPass& P, const float2* __restrict__ tw,
+                                         const int* __restrict__ out_row) {
+    // a thread takes one butterfly of two adjacent columns: 16-byte accesses and the twiddles loaded once
+    // for both
+    const int S = P.stride, CP = 1 << (lcb - 1);
     const int nbf = (G / R) << (lcb - 1);
-    const int mask = (16 >> lcb) - 1;
+    const int mask = (16 >> lcb) - 1;  // lcb <= 4
     for (int t = threadIdx.x; t < nbf; t += NT) {
         const int c = (t & (CP - 1)) * 2, q = t >> (lcb - 1);
-        const int b = q >> s_log, j = q & (S - 1);
+        const int b = (int)(((unsigned int)q * P.div_mul) >> P.div_shift), j = q - b * S;
         const int base = b * R * S + j;
         float2 v[16], u[16];
 #pragma unroll
@@ -154,8 +249,8 @@ __device__ __forceinline__ void col_pass(float2* __restrict__ sh, int G, int lcb
         }
         dft_r<R>(v);
         dft_r<R>(u);
-        if (j) {
-            const int st = j * tw_step;
+        if (!LAST && j) {  // the last pass has S = 1
+            const int st = j * P.tw_step;
             int ix = st;
 #pragma unroll
             for (int k = 1; k < R; ++k, ix += st) {
@@ -165,13 +260,33 @@ __device__ __forceinline__ void col_pass(float2* __restrict__ sh, int G, int lcb
             }
         }
 #pragma unroll
-        for (int m = 0; m < R; ++m)
-            *reinterpret_cast<float4*>(sh + (srow(base + S * m, mask) << lcb) + c) =
-                make_float4(v[m].x, v[m].y, u[m].x, u[m].y);
+        for (int m = 0; m < R; ++m) {
+            if (LAST)
+                cols.store(__ldg(&out_row[base + S * m]), c, v[m], u[m]);
+            else
+                *reinterpret_cast<float4*>(sh + (srow(base + S * m, mask) << lcb) + c) =
+                    make_float4(v[m].x, v[m].y, u[m].x, u[m].y);
+        }
     }
 }
 
-// NT threads; NT = 256: two CTAs per SM (blocks of up to 96 KB), NT = 512: one (up to 192 KB)
+template <int NT, bool LAST>
+__device__ __forceinline__ void any_pass(float2* __restrict__ sh, const Columns& cols, int G, int lcb,
+                                         const ColFftPass& P, const float2* __restrict__ tw,
+                                         const int* __restrict__ out_row) {
+    switch (P.radix) {
+        case 2: col_pass<2, NT, LAST>(sh, cols, G, lcb, P, tw, out_row); break;
+        case 3: col_pass<3, NT, LAST>(sh, cols, G, lcb, P, tw, out_row); break;
+        case 4: col_pass<4, NT, LAST>(sh, cols, G, lcb, P, tw, out_row); break;
+        case 5: col_pass<5, NT, LAST>(sh, cols, G, lcb, P, tw, out_row); break;
+        case 7: col_pass<7, NT, LAST>(sh, cols, G, lcb, P, tw, out_row); break;
+        case 8: col_pass<8, NT, LAST>(sh, cols, G, lcb, P, tw, out_row); break;
+        case 9: col_pass<9, NT, LAST>(sh, cols, G, lcb, P, tw, out_row); break;
+        default: col_pass<16, NT, LAST>(sh, cols, G, lcb, P, tw, out_row); break;
+    }
+}
+
+// NT threads; NT = 256: two CTAs per SM and more (blocks of up to 96 KB), NT = 512: one (up to 192 KB)
 template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) k_fft_cols(float2* __restrict__ planes, int G, long long c0,
                                                              int ncols, ColFftPlan P,
@@ -179,105 +294,107 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_fft_cols(float2* __restrict__ 
                                                              const int* __restrict__ out_row) {
     extern __shared__ __align__(16) float2 sh[];
     const int lcb = P.lcb, CB = 1 << lcb;
-    const int mask = (16 >> lcb) - 1;
     const int cb0 = blockIdx.x * CB;
-    const int ncb = min(CB, ncols - cb0);
-    float2* const pl = planes + (long long)blockIdx.y * G * G + c0 + cb0;
-    const int n = G << lcb;
-    // pairs of columns: 16-byte copies where the pair is whole and 16-byte aligned (c0 + cb0 even;
-    // G even keeps every row aligned alike), else 8-byte copies; columns past the block's end are 0
-    const bool al16 = ((c0 + cb0) & 1) == 0;
-    for (int i = threadIdx.x; i < (n >> 1); i += NT) {
+    Columns cols;
+    cols.pl = planes + (long long)blockIdx.y * G * G + c0 + cb0;
+    cols.G = G;
+    cols.ncb = min(CB, ncols - cb0);
+    cols.al16 = ((c0 + cb0) & 1) == 0;  // G even keeps every row aligned alike
+    for (int i = threadIdx.x; i < (G << (lcb - 1)); i += NT) {
         const int r = i >> (lcb - 1), c = (i & ((CB >> 1) - 1)) * 2;
-        const float2* src = pl + (long long)r * G + c;
-        float2* dst = sh + (srow(r, mask) << lcb) + c;
-        if (al16 && c + 1 < ncb) {
-            cp_async16(dst, src);
-        } else {
-            if (c < ncb) cp_async8(dst, src);
-            else dst[0] = make_float2(0.0f, 0.0f);
-            if (c + 1 < ncb) cp_async8(dst + 1, src + 1);
-            else dst[1] = make_float2(0.0f, 0.0f);
-        }
+        cols.load(sh + (srow(r, (16 >> lcb) - 1) << lcb) + c, r, c);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    for (int p = 0; p < P.npass; ++p) {
-        switch (P.rad[p]) {
-            case 2: col_pass<2, NT>(sh, G, lcb, P.s_log[p], P.tw_step[p], tw); break;
-            case 3: col_pass<3, NT>(sh, G, lcb, P.s_log[p], P.tw_step[p], tw); break;
-            case 4: col_pass<4, NT>(sh, G, lcb, P.s_log[p], P.tw_step[p], tw); break;
-            case 8: col_pass<8, NT>(sh, G, lcb, P.s_log[p], P.tw_step[p], tw); break;
-            default: col_pass<16, NT>(sh, G, lcb, P.s_log[p], P.tw_step[p], tw); break;
-        }
+    for (int p = 0; p + 1 < P.npass; ++p) {
+        any_pass<NT, false>(sh, cols, G, lcb, P.pass[p], tw, out_row);
         __syncthreads();
     }
-    // block row r to its output row (digit reversal), pairs of columns as on the way in
-    for (int i = threadIdx.x; i < (n >> 1); i += NT) {
-        const int r = i >> (lcb - 1), c = (i & ((CB >> 1) - 1)) * 2;
-        const float2* src = sh + (srow(r, mask) << lcb) + c;
-        float2* dst = pl + (long long)__ldg(&out_row[r]) * G + c;
-        if (al16 && c + 1 < ncb) {
-            *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>(src);
-        } else {
-            if (c < ncb) dst[0] = src[0];
-            if (c + 1 < ncb) dst[1] = src[1];
-        }
-    }
+    any_pass<NT, true>(sh, cols, G, lcb, P.pass[P.npass - 1], tw, out_row);
 }
 
 }  // namespace
 
-// Where it is used: grid sizes at which it measured faster than cuFFT's strided column plan on
-// B200 -- up to 1536 rows (two CTAs per SM; 1536: configuration B 49.5 -> 46.6 ms per 256
-// snapshots) and from 4096 (6144: 0.38 -> 0.17 ms per plane). At 3072 rows cuFFT's column kernel
-// stays ahead (0.091 against 0.093 ms for the precision snapshot's whole FFT).
-bool col_fft_supported(long long G) {
-    if (G < 16 || G > 12288 || (G > 1536 && G < 4096)) return false;
-    long long r = G;
-    while (r % 2 == 0) r /= 2;
-    return r == 1 || r == 3;
+// Radices of G: the largest power of two first, then the odd ones, then the remaining powers of two; empty
+// when G has a prime factor above 7 or fewer than two radices.
+static std::vector<int> col_radices(long long G) {
+    int k2 = 0, k3 = 0;
+    std::vector<int> odd, two;
+    long long g = G;
+    while (g % 2 == 0) g /= 2, ++k2;
+    while (g % 3 == 0) g /= 3, ++k3;
+    while (g % 5 == 0) g /= 5, odd.push_back(5);
+    while (g % 7 == 0) g /= 7, odd.push_back(7);
+    if (g != 1 || k2 == 0) return {};
+    for (; k3 >= 2; k3 -= 2) odd.push_back(9);
+    if (k3) odd.push_back(3);
+    // 16s with a tail of 8s and 4s (no radix-2 pass beside a larger one: 2^5 = 8 4, 2^9 = 8 8 8)
+    switch (k2 % 4) {
+        case 1:
+            if (k2 == 1) two = {2};
+            else if (k2 == 5) two = {8, 4}, k2 = 0;
+            else two = {8, 8, 8}, k2 -= 9;
+            break;
+        case 2:
+            if (k2 == 2) two = {4};
+            else two = {8, 8}, k2 -= 6;
+            break;
+        case 3: two = {8}; k2 -= 3; break;
+    }
+    if (two.empty() || two[0] > 4 || k2 > 2)
+        for (; k2 >= 4; k2 -= 4) two.insert(two.begin(), 16);
+    std::vector<int> rad = {two[0]};
+    rad.insert(rad.end(), odd.begin(), odd.end());
+    rad.insert(rad.end(), two.begin() + 1, two.end());
+    if (rad.size() < 2 || rad.size() > kColFftPasses) return {};
+    return rad;
 }
 
-int make_col_fft(long long G, ColFftPlan& P, float2** d_tw, int** d_perm) {
+// log2 of the columns per CTA: the largest power of two up to 16 with G * CB * 8 bytes <= 96 KB up to 1536
+// rows (two CTAs per SM), <= 192 KB beyond (one CTA per SM; 6144 rows x 4 columns: 32-byte row
+// segments, where pairs of columns at 96 KB measured slower). At least 1: the passes take pairs of columns.
+static int col_fft_lcb(long long G, long long columns) {
+    const long long cap = G <= 1536 ? 96 * 1024 : 192 * 1024;
+    int lcb = 1;
+    while (lcb < 4 && G * (2LL << lcb) * 8 <= cap) ++lcb;
+    // few columns: narrower blocks until there is a CTA per SM (8 planes of 288 / 384 rows: 19.5 / 25.6 us with
+    // two CTAs per SM asked for, 17.4 / 21.5 us with one)
+    while (lcb > 2 && (columns >> lcb) < 148) --lcb;
+    return lcb;
+}
+
+// Where it is used: every grid size it supports measured at or below cuFFT's strided column plan (whole FFT,
+// rows by cuFFT in both; us): 288 rows, 8 planes 58 -> 17; 720, 8 planes 91 -> 44; 1500, 4 planes 126 -> 83; 1536,
+// 2 planes 52 -> 42; 2304, 8 planes 407 -> 325; 3072, 2 planes 185 -> 165; 3584, 2 planes 341 -> 235; 4500, 2
+// planes 1037 -> 413; 6144, 2 planes 1025 -> 699 (730 before the last pass wrote the plane itself).
+bool col_fft_supported(long long G) {
+    if (G < 16 || G > 12288) return false;
+    return !col_radices(G).empty();
+}
+
+int make_col_fft(long long G, long long columns, ColFftPlan& P, float2** d_tw, int** d_perm) {
+    const std::vector<int> rad = col_radices(G);
     if (!col_fft_supported(G)) {
         set_error("column FFT: unsupported grid size");
         return SVDI_ERR_UNSUPPORTED;
     }
-    // radices: 3 first (when 3 | G), then 16s, then the remaining power of two
-    std::vector<int> rad;
-    long long g = G;
-    int k2 = 0;
-    while (g % 2 == 0) {
-        g /= 2;
-        ++k2;
-    }
-    if (g == 3) rad.push_back(3);
-    while (k2 >= 4) {
-        rad.push_back(16);
-        k2 -= 4;
-    }
-    if (k2) rad.push_back(1 << k2);
     P = ColFftPlan{};
     P.npass = (int)rad.size();
     long long before = 1;  // product of the earlier radices = G / (R S)
     for (int p = 0; p < P.npass; ++p) {
         long long S = 1;
         for (int q = p + 1; q < P.npass; ++q) S *= rad[q];
-        int sl = 0;
-        while ((1LL << sl) < S) ++sl;
-        P.rad[p] = rad[p];
-        P.s_log[p] = sl;
-        P.tw_step[p] = (int)before;
+        P.pass[p].radix = rad[p];
+        P.pass[p].stride = (int)S;
+        P.pass[p].tw_step = (int)before;
+        // mul = ceil(2^shift / S), shift = 14 + ceil(log2 S): the quotient is off by less than q / 2^14 / S < 1 / S
+        unsigned int shift = 14;
+        while ((1LL << (shift - 14)) < S) ++shift;
+        P.pass[p].div_mul = (unsigned int)(((1LL << shift) + S - 1) / S);
+        P.pass[p].div_shift = shift;
         before *= rad[p];
     }
-    // columns per CTA: the largest power of two up to 16 with G * CB * 8 bytes <= 96 KB up to 1536
-    // rows (two CTAs per SM), <= 192 KB beyond (one CTA per SM; 6144 rows x 4 columns: 32-byte row
-    // segments, where pairs of columns at 96 KB measured slower)
-    const long long cap = G <= 1536 ? 96 * 1024 : 192 * 1024;
-    int lcb = 1;
-    while (lcb < 4 && G * (2LL << lcb) * 8 <= cap) ++lcb;
-    P.lcb = lcb;  // >= 1 for every supported G (the copies take pairs of columns)
+    P.lcb = col_fft_lcb(G, columns);
     // tables: e^{+2 pi i t / G} and the digit-reversed position of each output row
     std::vector<float2> tw((size_t)G);
     for (long long t = 0; t < G; ++t) {
@@ -290,7 +407,7 @@ int make_col_fft(long long G, ColFftPlan& P, float2** d_tw, int** d_perm) {
         for (int p = 0; p < P.npass; ++p) {
             const long long k = t % rad[p];
             t /= rad[p];
-            pos += k << P.s_log[p];
+            pos += k * P.pass[p].stride;
         }
         perm[(size_t)pos] = (int)nrow;  // block row pos holds output row nrow
     }
@@ -303,7 +420,8 @@ int make_col_fft(long long G, ColFftPlan& P, float2** d_tw, int** d_perm) {
 
 int launch_col_fft(float2* d_planes, int nplanes, long long G, long long c0, long long ncols, const ColFftPlan& P,
                    const float2* d_tw, const int* d_perm, cudaStream_t st) {
-    const size_t smem = (size_t)G * ((size_t)1 << P.lcb) * sizeof(float2);
+    const size_t bank_rows = (size_t)16 >> P.lcb;  // the swizzle permutes rows within runs of this length
+    const size_t smem = ((size_t)G + bank_rows - 1) / bank_rows * bank_rows * ((size_t)1 << P.lcb) * sizeof(float2);
     const dim3 grid((unsigned)((ncols + (1LL << P.lcb) - 1) >> P.lcb), (unsigned)nplanes);
     if (smem <= 96 * 1024) {
         SVDI_TRY(ensure_dynamic_smem((const void*)k_fft_cols<256>, smem, true));

@@ -221,19 +221,22 @@ int launch_dft_probe(const SampleSource& src, const GridGeom& g, const SlabParam
                      long long N, double cell, const long long* d_px, const long long* d_py, int npix,
                      double* d_acc, int sm_count, cudaStream_t st);
 
-// fft_cols.cu: the pruned inverse FFT's column transforms in shared memory (G = 2^a 3^b, b <= 1,
-// 16 <= G <= 12288): pass radices, log2 of each pass's stride, twiddle-table steps, log2 of the
-// columns per CTA
+// fft_cols.cu: the pruned inverse FFT's column transforms in shared memory (G = 2^a 3^b 5^c 7^d,
+// 16 <= G <= 12288): per pass the radix, its stride, the twiddle-table step and the multiplier that
+// divides by the stride; log2 of the columns per CTA
+constexpr int kColFftPasses = 8;
+struct ColFftPass {
+    int radix = 0, stride = 1, tw_step = 1;
+    unsigned int div_mul = 1, div_shift = 0;  // q / stride = (q div_mul) >> div_shift for q < 2^14
+};
 struct ColFftPlan {
     int npass = 0;
     int lcb = 0;
-    int rad[6] = {};
-    int s_log[6] = {};
-    int tw_step[6] = {};
+    ColFftPass pass[kColFftPasses];
 };
 bool col_fft_supported(long long G);
-// allocates the twiddle and output-permutation tables (cudaFree both)
-int make_col_fft(long long G, ColFftPlan& P, float2** d_tw, int** d_perm);
+// columns: of all planes of a launch; allocates the twiddle and output-permutation tables (cudaFree both)
+int make_col_fft(long long G, long long columns, ColFftPlan& P, float2** d_tw, int** d_perm);
 // columns [c0, c0 + ncols) of each of nplanes G x G planes, in place
 int launch_col_fft(float2* d_planes, int nplanes, long long G, long long c0, long long ncols, const ColFftPlan& P,
                    const float2* d_tw, const int* d_perm, cudaStream_t st);
