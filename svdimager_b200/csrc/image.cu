@@ -109,6 +109,44 @@ __device__ inline SplatTarget reproject_fipk(long long idx, long long idy, long 
     return {oi0 - (double)half, oi1 - (double)half, true};
 }
 
+// A warp takes an 8 x 4 patch of pixels: the splat's targets are the patch turned by the snapshot's rotation,
+// and its reductions cost the L2 one operation per 32-byte sector: about 14 sectors per warp instruction for
+// a patch, up to 32 for a run of 32 pixels. (tx, ty): the thread's place in its block's 32 x 8 tile.
+__device__ __forceinline__ void patch_pixel(int& tx, int& ty) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    tx = (warp & 3) * 8 + (lane & 7);
+    ty = (warp >> 2) * 4 + (lane >> 3);
+}
+
+// floor of x, |x| < 2^31, as a double and an integer: one addition rounds x to the nearest integer, which
+// the low word of the sum holds (the conversion unit, at a sixteenth of the FP64 rate, stays free).
+__device__ __forceinline__ double floor_int(double x, int& i) {
+    const double r = x + 6755399441055744.0;  // 1.5 * 2^52
+    double f = r - 6755399441055744.0;
+    i = __double2loint(r);
+    if (f > x) {
+        f -= 1.0;
+        --i;
+    }
+    return f;
+}
+
+// Bilinear splat of one value at (LL, MM), pixels from the image centre (archive/FIPkernels.cu:627-677).
+__device__ __forceinline__ void splat(float* __restrict__ out, int N, int half, double LL, double MM, double value) {
+    if (!(fabs(LL) < (double)(half - 1) && fabs(MM) < (double)(half - 1))) return;
+    int l, m;
+    const double fl = LL - floor_int(LL, l), fm = MM - floor_int(MM, m);
+    float* d = out + (long long)(m + half) * N + (l + half);
+    // an exactly integer target adds its zero weights to its own cell
+    const int dx = fl > 0.0 ? 1 : 0;
+    const long long dy = fm > 0.0 ? N : 0;
+    const double v0 = (1.0 - fl) * value, v1 = fl * value, gm = 1.0 - fm;
+    atomicAdd(d, (float)(v0 * gm));
+    atomicAdd(d + dy, (float)(v0 * fm));
+    atomicAdd(d + dx, (float)(v1 * gm));
+    atomicAdd(d + dy + dx, (float)(v1 * fm));
+}
+
 // From the sum over planes at pixel (x, y) to the image: checkerboard, grid correction, slab batches,
 // |.| / N_s, reprojection and bilinear splat.
 __device__ __forceinline__ void finish_pixel(long long x, long long y, double sum, long long N, double cell,
@@ -140,14 +178,7 @@ __device__ __forceinline__ void finish_pixel(long long x, long long y, double su
     const SplatTarget tg = reprojection == SVDI_REPROJ_FIPK ? reproject_fipk(x, y, N, cell, V)
                                                             : reproject_sii(x, y, N, kc, V);
     if (!tg.ok) return;
-    const double LL = tg.LL, MM = tg.MM;
-    if (!(fabs(LL) < (double)(half - 1) && fabs(MM) < (double)(half - 1))) return;
-    const double Lf = floor(LL), Mf = floor(MM), Lc = ceil(LL), Mc = ceil(MM);
-    float* d = out + half * N + half;
-    atomicAdd(&d[(long long)Mf * N + (long long)Lf], (float)((1 - LL + Lf) * (1 - MM + Mf) * value));
-    atomicAdd(&d[(long long)Mc * N + (long long)Lf], (float)((1 - LL + Lf) * (0 + MM - Mf) * value));
-    atomicAdd(&d[(long long)Mf * N + (long long)Lc], (float)((0 + LL - Lf) * (1 - MM + Mf) * value));
-    atomicAdd(&d[(long long)Mc * N + (long long)Lc], (float)((0 + LL - Lf) * (0 + MM - Mf) * value));
+    splat(out, (int)N, (int)half, tg.LL, tg.MM, value);
 }
 
 // One pixel (x, y) of the rotated frame: moments -> |Re sum| -> grid correction -> reprojection.
@@ -243,17 +274,175 @@ __global__ void __launch_bounds__(256, 4) k_recombine(const float2* __restrict__
         sp.inv_half = plan->sp.inv_half;
     }
     __shared__ ReprojConst kc;
-    if (threadIdx.x == 0 && threadIdx.y == 0) kc = reproj_const(vin, cell);
+    if (threadIdx.x == 0) kc = reproj_const(vin, cell);
     __syncthreads();
     const bool bad = nonfinite && *nonfinite;
     const long long ntx = (N + 31) / 32, nty = (N + 7) / 8;
+    int px, py;
+    patch_pixel(px, py);
     for (long long t = blockIdx.x; t < ntx * nty; t += gridDim.x) {
         const long long ty = t / ntx, tx = t - ty * ntx;
-        const long long x = tx * 32 + threadIdx.x, y = ty * 8 + threadIdx.y;
+        const long long x = tx * 32 + px, y = ty * 8 + py;
         if (x < N && y < N)
             recombine_pixel<KMAX>(x, y, moments, g, N, cell, vin, sp, corr, inv_n, reprojection, presplat, out, acc,
                                   final_batch, bad, kc);
     }
+}
+
+// J_0 .. J_{KT-1}: bessel_jn_fast with the ascending series (|x| < 1e-3) unrolled in registers.
+template <int KT>
+__device__ __forceinline__ void bessel_few(double x, double (&j)[KT]) {
+    if (fabs(x) < 1e-3) {
+        const double h = 0.5 * x, q = -h * h;
+        double lead = 1.0;  // (x/2)^n / n!
+#pragma unroll
+        for (int n = 0; n < KT; ++n) {
+            if (n > 0) lead *= h * (1.0 / n);
+            const double t1 = q * (1.0 / (n + 1));
+            j[n] = fma(lead * t1, fma(q, 0.5 / (n + 2), 1.0), lead);
+        }
+        return;
+    }
+    double t[KT];
+    bessel_jn_fast(x, KT - 1, t);
+#pragma unroll
+    for (int n = 0; n < KT; ++n) j[n] = t[n];
+}
+
+// Few Chebyshev terms, K = KT (the coplanar snapshots' orders 1 .. 4 and the bucket rule's 8): everything
+// unrolled, what depends on the launch computed once: 330 warp instructions per 32 pixels at two terms, where
+// the general kernel above takes 550 (term loops over a local array, 64-bit indices, conversions). With the
+// patches, two terms: 1024^2 35 -> 24 us, 2048^2 115 -> 74 us (12 us of it the splat's reductions, 55 us before
+// the patches). Four pixels of a row per thread, to share the row's part, was slower (80 us: fewer warps wait for
+// more loads each).
+template <int KT>
+__global__ void __launch_bounds__(256, 3) k_recombine_few(const float2* __restrict__ moments, GridGeom g, int N,
+                                                      double cell, const double* __restrict__ vin, SlabParams sp,
+                                                      const float* __restrict__ corr, double inv_n, int reprojection,
+                                                      int presplat, float* __restrict__ out, double* __restrict__ acc,
+                                                      int final_batch, const DevPlan* __restrict__ plan,
+                                                      const unsigned long long* __restrict__ nonfinite) {
+    if (plan) {  // one batch of all slabs: the device plan's slab geometry
+        sp.r3_min = plan->sp.r3_min;
+        sp.slab_width = plan->sp.slab_width;
+        sp.slab_half = plan->sp.slab_half;
+    }
+    __shared__ ReprojConst kc_s;
+    if (threadIdx.x == 0) kc_s = reproj_const(vin, cell);
+    __syncthreads();
+    const ReprojConst kc = kc_s;
+    const bool bad = nonfinite && *nonfinite;
+    const int half = N / 2, G = (int)g.G;
+    const long long GG = (long long)G * G;
+    const double di2 = (double)N * 0.5;
+    const double v13 = vin[2], v23 = vin[5], v33 = vin[8], sgn = v33 >= 0.0 ? 1.0 : -1.0;
+    const double a0 = -vin[0] * kc.inv_v8, a3 = vin[3] * kc.inv_v8, b1 = -vin[1] * kc.inv_v8, b4 = vin[4] * kc.inv_v8;
+    const double c_alpha = 2.0 * kPi * sp.slab_half;
+    const int ntx = (N + 31) / 32, nty = (N + 7) / 8;
+    int px, py;
+    patch_pixel(px, py);
+    for (int t = blockIdx.x; t < ntx * nty; t += gridDim.x) {
+        const int ty = t / ntx, tx = t - ty * ntx;
+        const int y = ty * 8 + py, yr = y - half;
+        if (y >= N) continue;
+        const double t1 = fma(cell, (double)yr, v13), r1 = 1.0 - t1 * t1;
+        const double idyf = (double)y - di2;
+        const double p1y = fma(a3, idyf, di2), p2y = fma(b4, idyf, di2);
+        const double cy = (double)corr[yr < 0 ? -yr : yr];
+        const float2* mrow = moments + (GG / 2 + G / 2 + (long long)yr * G) - half;
+        const int x = tx * 32 + px, xr = x - half;
+        if (x >= N) continue;
+        const double xd = (double)xr;
+        const double t2 = fma(cell, xd, v23), ra = r1 - t2 * t2;
+        if (ra < 0.0) {
+            if (presplat && final_batch) out[(long long)y * N + x] = __int_as_float(0x7fc00000);  // NaN
+            continue;
+        }
+        const double t3 = fma(sgn, sqrt(ra), -v33);
+        double jv[KT];
+        bessel_few<KT>(t3 * c_alpha, jv);
+        double sum = 0.0;
+        for (int s = 0; s < sp.nslab; ++s) {
+            const float2* mp = mrow + (long long)s * KT * GG + x;
+            float2 m[KT];
+#pragma unroll
+            for (int n = 0; n < KT; ++n) m[n] = mp[n * GG];
+            const double ph = 2.0 * t3 * (sp.r3_min + ((double)s + 0.5) * sp.slab_width);  // e^{i pi ph}
+            double sb, cb;
+            if (fabs(ph) < 0x1p-8) {  // the next terms of the series are below 1e-17
+                const double z = kPi * ph, z2 = z * z;
+                cb = fma(z2, fma(z2, fma(z2, -1.0 / 720.0, 1.0 / 24.0), -0.5), 1.0);
+                sb = z * fma(z2, fma(z2, fma(z2, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), 1.0);
+            } else {
+                sincospi(ph, &sb, &cb);
+            }
+            double part = 0.0;
+#pragma unroll
+            for (int n = 0; n < KT; ++n) {
+                const double amp = n == 0 ? jv[0] : 2.0 * jv[n];
+                const double mx = (double)m[n].x, my = (double)m[n].y;
+                double v;  // Re(i^n e^{i beta} M_n)
+                switch (n & 3) {
+                    case 0: v = cb * mx - sb * my; break;
+                    case 1: v = -sb * mx - cb * my; break;
+                    case 2: v = sb * my - cb * mx; break;
+                    default: v = sb * mx + cb * my; break;
+                }
+                part = fma(amp, v, part);
+            }
+            sum += part;
+        }
+        if ((xr + yr) & 1) sum = -sum;
+        double signed_sum = sum * (double)corr[xr < 0 ? -xr : xr] * cy;
+        if (acc) {  // slab batches: the signed sums add up, |.| is taken once, in the last batch
+            double* a = acc + (long long)y * N + x;
+            signed_sum += *a;
+            if (!final_batch) {
+                *a = signed_sum;
+                continue;
+            }
+        }
+        double value = fabs(signed_sum) * inv_n;
+        if (bad) value = __longlong_as_double(0x7ff8000000000000LL);  // as in finish_pixel
+        if (presplat) {
+            out[(long long)y * N + x] = (float)value;
+            continue;
+        }
+        double LL, MM;
+        if (reprojection == SVDI_REPROJ_FIPK) {
+            const SplatTarget tg = reproject_fipk(x, y, N, cell, vin);
+            if (!tg.ok) continue;
+            LL = tg.LL;
+            MM = tg.MM;
+        } else {  // reproject_sii with the row's part of the rotation at hand
+            const double idxf = (double)x - di2;
+            const double p1 = fma(a0, idxf, p1y), p2 = fma(b1, idxf, p2y);
+            const double xo = p1 - (di2 + 1.0), yo = p2 - (di2 + 1.0);
+            const double s = fma(xo, xo, yo * yo) * kc.dc_r0_sq;
+            LL = p1;
+            MM = p2;
+            if (s <= 1.0) {
+                const float sf = (float)s;
+                const float mv = sf / (1.0f + sqrtf(1.0f - sf)) * kc.r0_dc;
+                LL -= (double)(mv * kc.xi_f);
+                MM += (double)(mv * kc.eta_f);
+            }
+            LL -= (double)half;
+            MM -= (double)half;
+        }
+        splat(out, N, half, LL, MM, value);
+    }
+}
+
+template <int KT>
+void launch_few(const float2* d_moments, const GridGeom& g, int N, double cell, const double* d_vin64,
+                const SlabParams& sp, const float* d_corr, double inv_n, int reprojection, int presplat, float* d_out,
+                cudaStream_t st, double* d_acc, int final_batch, const DevPlan* d_plan,
+                const unsigned long long* d_nonfinite) {
+    const long long tiles = ((N + 31LL) / 32) * ((N + 7) / 8);
+    k_recombine_few<KT><<<(unsigned)std::min<long long>(tiles, 6LL * current_sm_count()), 256, 0, st>>>(
+        d_moments, g, N, cell, d_vin64, sp, d_corr, inv_n, reprojection, presplat, d_out, d_acc, final_batch, d_plan,
+        d_nonfinite);
 }
 
 // One pixel from w planes: Re sum_p e^{2 pi i w_p t3} M_p / psi^(dw t3). The phases advance by one
@@ -265,7 +454,7 @@ __global__ void __launch_bounds__(256, 4) k_recombine_w(const float2* __restrict
                                                     float* __restrict__ out, double* __restrict__ acc,
                                                     int final_batch, const unsigned long long* __restrict__ nonfinite) {
     __shared__ ReprojConst kc;
-    if (threadIdx.x == 0 && threadIdx.y == 0) kc = reproj_const(vin, cell);
+    if (threadIdx.x == 0) kc = reproj_const(vin, cell);
     __syncthreads();
     const bool bad = nonfinite && *nonfinite;
     double V[9];
@@ -273,9 +462,11 @@ __global__ void __launch_bounds__(256, 4) k_recombine_w(const float2* __restrict
     for (int k = 0; k < 9; ++k) V[k] = vin[k];
     const long long half = N / 2, G = g.G, GG = G * G;
     const long long ntx = (N + 31) / 32, nty = (N + 7) / 8;
+    int px, py;
+    patch_pixel(px, py);
     for (long long t = blockIdx.x; t < ntx * nty; t += gridDim.x) {
         const long long ty = t / ntx, tx = t - ty * ntx;
-        const long long x = tx * 32 + threadIdx.x, y = ty * 8 + threadIdx.y;
+        const long long x = tx * 32 + px, y = ty * 8 + py;
         if (x >= N || y >= N) continue;
         const long long xr = x - half, yr = y - half;
         const double t1 = cell * (double)yr, t2 = cell * (double)xr;
@@ -324,11 +515,19 @@ int launch_recombine(const float2* d_moments, const GridGeom& g, long long N, do
                      double inv_n_total, int reprojection, int presplat, float* d_out,
                      cudaStream_t st, double* d_acc, bool final_batch, const DevPlan* d_plan,
                      const unsigned long long* d_nonfinite) {
-    const dim3 block(32, 8);
+    const dim3 block(256);
     const long long tiles = ((N + 31) / 32) * ((N + 7) / 8);
     const dim3 grid((unsigned)std::min<long long>(tiles, 8LL * current_sm_count()));
-    if (sp.K <= 1) k_recombine<1><<<grid, block, 0, st>>>(d_moments, g, N, cell, d_vin64, sp, d_corr, inv_n_total, reprojection, presplat, d_out, d_acc, final_batch ? 1 : 0, d_plan, d_nonfinite);
-    else if (sp.K <= 8) k_recombine<8><<<grid, block, 0, st>>>(d_moments, g, N, cell, d_vin64, sp, d_corr, inv_n_total, reprojection, presplat, d_out, d_acc, final_batch ? 1 : 0, d_plan, d_nonfinite);
+#define SVDI_FEW(KT)                                                                                          \
+    launch_few<KT>(d_moments, g, (int)N, cell, d_vin64, sp, d_corr, inv_n_total, reprojection, presplat, d_out, st, \
+                   d_acc, final_batch ? 1 : 0, d_plan, d_nonfinite)
+    if (sp.K == 1) SVDI_FEW(1);
+    else if (sp.K == 2) SVDI_FEW(2);
+    else if (sp.K == 3) SVDI_FEW(3);
+    else if (sp.K == 4) SVDI_FEW(4);
+    else if (sp.K == 8) SVDI_FEW(8);
+#undef SVDI_FEW
+    else if (sp.K < 8) k_recombine<8><<<grid, block, 0, st>>>(d_moments, g, N, cell, d_vin64, sp, d_corr, inv_n_total, reprojection, presplat, d_out, d_acc, final_batch ? 1 : 0, d_plan, d_nonfinite);
     else if (sp.K <= 16) k_recombine<16><<<grid, block, 0, st>>>(d_moments, g, N, cell, d_vin64, sp, d_corr, inv_n_total, reprojection, presplat, d_out, d_acc, final_batch ? 1 : 0, d_plan, d_nonfinite);
     else if (sp.K <= 32) k_recombine<32><<<grid, block, 0, st>>>(d_moments, g, N, cell, d_vin64, sp, d_corr, inv_n_total, reprojection, presplat, d_out, d_acc, final_batch ? 1 : 0, d_plan, d_nonfinite);
     else if (sp.K <= kMaxTerms) k_recombine<kMaxTerms><<<grid, block, 0, st>>>(d_moments, g, N, cell, d_vin64, sp, d_corr, inv_n_total, reprojection, presplat, d_out, d_acc, final_batch ? 1 : 0, d_plan, d_nonfinite);
@@ -344,7 +543,7 @@ int launch_recombine_w(const float2* d_planes, const GridGeom& g, long long N, d
                        const WPlanes& wp, int plane_lo, int plane_hi, const float* d_corr, double inv_n_total,
                        int reprojection, int presplat, float* d_out, cudaStream_t st, double* d_acc, bool final_batch,
                        const unsigned long long* d_nonfinite) {
-    const dim3 block(32, 8);
+    const dim3 block(256);
     const long long tiles = ((N + 31) / 32) * ((N + 7) / 8);
     const dim3 grid((unsigned)std::min<long long>(tiles, 8LL * current_sm_count()));
     k_recombine_w<<<grid, block, 0, st>>>(d_planes, g, N, cell, d_vin64, wp, plane_lo, plane_hi, d_corr, inv_n_total,
