@@ -318,11 +318,13 @@ __global__ void __launch_bounds__(kThreads) k_scatter(SampleSource src, GridGeom
 // Separable sources (r = s[chan] q[row], idx = row + chan R). A warp takes units of UR
 // rows x one chunk of `lpr` channels (lpr a power of two <= 32): lane -> (row subset
 // lane / lpr, channel lane % lpr), so consecutive lanes hold consecutive channels of one row. The
-// channels of a baseline mostly share a tile, so match groups are large: one shared-memory or
-// global atomic per group, and a group's records land in consecutive slots. No 64-bit division.
+// channels of a baseline mostly share a tile, so runs of equal keys are long: one shared-memory or
+// global atomic per run, and a run's records land in consecutive slots. No 64-bit division.
 // UR = 16, or 4 where 16 would leave most of the chip idle: a unit is a serial chain of row steps (FP64 key
-// rule, match, a returning cursor atomic in the scatter). 130 k samples: histogram 11 -> 6 us, scatter 18 ->
-// 9 us; 8.4 M samples keep 16, whose staging loads are whole 64-byte pieces.
+// rule, a run search, a returning cursor atomic in the scatter). 130 k samples: both and the scan 41 -> 27 us;
+// 8.4 M samples keep 16, whose staging loads are whole 64-byte pieces. What bounds them is latency: 130
+// (histogram) and 240 warp instructions per 32 samples at 50-70 % of the issue slots; four CTAs per SM for the
+// scatter took it from 127 to 110 us at 8.4 M samples.
 constexpr int kUnitRows = 16, kUnitRowsSmall = 4;
 
 struct SepMap {
@@ -335,6 +337,17 @@ struct SepMap {
 __device__ inline void unit_of(long long u, const SepMap& m, int& rt, int& ch) {
     rt = (int)(u / m.nch);
     ch = (int)(u - (long long)rt * m.nch);
+}
+
+// Runs of equal keys on consecutive lanes (consecutive channels of one baseline mostly stay in a tile, and a key
+// that comes again later is another run): the first lane of this lane's run and the run's length. One shuffle
+// and one vote; a match over the warp costs several times that on the unit the atomics share.
+__device__ __forceinline__ void lane_run(int key, int lane, int& first, int& length) {
+    const int before = __shfl_up_sync(0xffffffffu, key, 1);
+    const unsigned int starts = __ballot_sync(0xffffffffu, lane == 0 || key != before);
+    first = 31 - __clz(starts & (0xffffffffu >> (31 - lane)));
+    const unsigned int after = starts & ~(0xffffffffu >> (31 - lane));
+    length = (after ? __ffs(after) - 1 : 32) - first;
 }
 
 template <int UR>
@@ -370,10 +383,11 @@ __global__ void __launch_bounds__(kThreads) k_histogram_sep(SampleSource src, Se
                 key = row_chan_key(sc, q[0], q[1], q[2], g, sp).key;
                 if (key < 0) ++ndrop;
             }
-            const unsigned int peers = __match_any_sync(0xffffffffu, key);
-            if (key >= 0 && lane == __ffs(peers) - 1) {
-                if (use_smem) atomicAdd(&sh[key], __popc(peers));
-                else atomicAdd(&counts[key], __popc(peers));
+            int first, length;
+            lane_run(key, lane, first, length);
+            if (key >= 0 && lane == first) {
+                if (use_smem) atomicAdd(&sh[key], (unsigned int)length);
+                else atomicAdd(&counts[key], (unsigned int)length);
             }
         }
     }
@@ -390,7 +404,7 @@ __global__ void __launch_bounds__(kThreads) k_histogram_sep(SampleSource src, Se
 // shared memory with row-contiguous loads, then writes each group's records to the slots one
 // global atomic on the key's cursor reserved.
 template <int UR>
-__global__ void __launch_bounds__(kThreads) k_scatter_sep(SampleSource src, SepMap m, GridGeom g, SlabParams sp,
+__global__ void __launch_bounds__(kThreads, 4) k_scatter_sep(SampleSource src, SepMap m, GridGeom g, SlabParams sp,
                                                          unsigned int* __restrict__ cursor,
                                                          SampleRec* __restrict__ rec, float* __restrict__ rec_s,
                                                          unsigned int* __restrict__ vmax,
@@ -431,39 +445,54 @@ __global__ void __launch_bounds__(kThreads) k_scatter_sep(SampleSource src, SepM
         const int c = c0 + coff;
         const bool cvalid = c < m.C;
         const double sc = cvalid ? src.s[c] : 0.0;
-        for (int i0 = 0; i0 < UR; i0 += rps) {  // every lane takes every step
-            const int i = i0 + sub;
-            const long long row = row0 + i;
+        // every lane takes every step; a step's records are written after the next step's keys, so that the
+        // latency of its cursor atomic is covered
+        KeyRec last;
+        last.key = -1;
+        int last_i = 0, last_first = 0, last_len = 0;
+        unsigned int last_base = 0;
+        for (int i0 = 0; i0 < UR + rps; i0 += rps) {
             KeyRec kr;
             kr.key = -2;
-            if (cvalid && i < UR && row < R) {
-                const double* q = src.q + row * 3;
-                kr = row_chan_key(sc, q[0], q[1], q[2], g, sp);
+            const int i = i0 + sub;
+            int first = 0, length = 0;
+            unsigned int base = 0;
+            if (i0 < UR) {
+                const long long row = row0 + i;
+                if (cvalid && i < UR && row < R) {
+                    const double* q = src.q + row * 3;
+                    kr = row_chan_key(sc, q[0], q[1], q[2], g, sp);
+                }
+                lane_run(kr.key, lane, first, length);
+                if (kr.key >= 0 && lane == first) base = atomicAdd(&cursor[kr.key], (unsigned int)length);
             }
-            const int key = kr.key;
-            const unsigned int peers = __match_any_sync(0xffffffffu, key);
-            const int leader = __ffs(peers) - 1;
-            unsigned int b0 = 0;
-            if (key >= 0 && lane == leader) b0 = atomicAdd(&cursor[key], __popc(peers));
-            b0 = __shfl_sync(0xffffffffu, b0, leader);
-            if (key >= 0) {
-                const unsigned int pos = b0 + __popc(peers & ((1u << lane) - 1u));
-                const float2 v = my[coff * kVisPitch + i];
-                SampleRec r;
-                r.xq = kr.xq;
-                r.yq = kr.yq;
-                r.vre = __fmul_rn(v.x, src.inv_det);
-                r.vim = __fmul_rn(v.y, src.inv_det);
-                rec[pos] = r;
-                if (rec_s) rec_s[pos] = kr.s;
-                nbad += nonfinite2(r.vre, r.vim);
-                const float m = fmaxf(fabsf(r.vre), fabsf(r.vim));
-                vm = fmaxf(vm, m);
-                if (keymax) {  // the group's maximum, one atomic per group
-                    const unsigned int gm = __reduce_max_sync(peers, __float_as_uint(m));
-                    if (lane == leader && gm) atomicMax(&keymax[key], gm);
+            if (i0 > 0) {
+                const unsigned int b0 = __shfl_sync(0xffffffffu, last_base, last_first);
+                if (last.key >= 0) {
+                    const unsigned int pos = b0 + (unsigned int)(lane - last_first);
+                    const float2 v = my[coff * kVisPitch + last_i];
+                    SampleRec r;
+                    r.xq = last.xq;
+                    r.yq = last.yq;
+                    r.vre = __fmul_rn(v.x, src.inv_det);
+                    r.vim = __fmul_rn(v.y, src.inv_det);
+                    rec[pos] = r;
+                    if (rec_s) rec_s[pos] = last.s;
+                    nbad += nonfinite2(r.vre, r.vim);
+                    const float m = fmaxf(fabsf(r.vre), fabsf(r.vim));
+                    vm = fmaxf(vm, m);
+                    if (keymax) {  // the run's maximum, one atomic per run
+                        const unsigned int run = (0xffffffffu >> (32 - last_len)) << last_first;
+                        const unsigned int gm = __reduce_max_sync(run, __float_as_uint(m));
+                        if (lane == last_first && gm) atomicMax(&keymax[last.key], gm);
+                    }
                 }
             }
+            last = kr;
+            last_i = i;
+            last_first = first;
+            last_len = length;
+            last_base = base;
         }
     }
     flush_nonfinite(src.nonfinite, nbad);

@@ -14,23 +14,34 @@ struct KeyRec {
     float s;
 };
 
-// floor(x / T) for 0 <= x < 2^24 and 1 <= T < 2^24, exact: a float estimate (off by at most one
-// for these ranges) and one integer correction.
+// floor(x / T) for 0 <= x < 2^24 and 1 <= T < 2^24, exact: a shift for the power-of-two tiles (a test every
+// thread of a launch takes alike), else a float estimate (off by at most one for these ranges) and one
+// integer correction.
 __device__ inline int tile_div(int x, int T) {
+    if ((T & (T - 1)) == 0) return x >> (31 - __clz(T));
     int t = __float2int_rz(__fmul_rn(__int2float_rn(x), __frcp_rn(__int2float_rn(T))));
     if (t * T > x) --t;
     else if ((t + 1) * T <= x) ++t;
     return t;
 }
 
+// floor(x) of |x| < 2^51 as a 64-bit integer, exact: adding 1.5 2^52 rounds x to the nearest integer, held by the
+// low bits of the sum, and one comparison turns nearest into floor. Three FP64 additions at the FP64 rate; the
+// conversion instruction runs on the unit that bounded the binning (40 % busy in the histogram).
+__device__ inline long long floor_to_int(double x) {
+    constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52
+    const double r = __dadd_rn(x, kMagic);
+    const long long q = __double_as_longlong(r) - __double_as_longlong(kMagic);
+    return __dsub_rn(r, kMagic) > x ? q - 1 : q;
+}
+
 // Q = floor(p 2^24) split into cell = floor(p) = Q >> 24 and frac = Q & (2^24 - 1): p 2^24 is exact
-// (power-of-two scaling) and one round-down conversion to a 64-bit integer gives Q exactly
-// (|Q| < 1e9 2^24 < 2^54), so the split is integer arithmetic. |p| >= 1e9 lies beyond every grid
-// (G < 2^24) and is dropped under both edge rules, like the contract's 1e15 bound; within it every
+// (power-of-two scaling) and its floor too, so the split is integer arithmetic. |p| >= 2^26 lies beyond every
+// grid (G < 2^24) and is dropped under both edge rules, like the contract's 1e15 bound; within it every
 // cell fits 32 bits (tiles T <= 64).
 __device__ inline bool quantise_axis(double p, const GridGeom& g, int T, int& tile, int& qrel) {
-    if (!(fabs(p) < 1e9)) return false;
-    const long long Q = __double2ll_rd(p * 16777216.0);
+    if (!(fabs(p) < 67108864.0)) return false;
+    const long long Q = floor_to_int(p * 16777216.0);
     const int cell = (int)(Q >> 24);
     const int frac = (int)(Q & 0xFFFFFF);
     const int hw = g.W / 2;
@@ -80,10 +91,12 @@ __device__ inline KeyRec coord_key(double r1, double r2, double r3, const GridGe
     int j = 0;
     double sv = 0.0;
     if (sp.nslab > 1 || sp.K > 1) {
-        double jf = floor(__ddiv_rn(__dsub_rn(r3, sp.r3_min), sp.slab_width));
-        if (!(jf >= 0.0)) jf = 0.0;  // also NaN
-        if (jf > (double)(sp.nslab - 1)) jf = (double)(sp.nslab - 1);
-        j = (int)jf;
+        if (sp.nslab > 1) {  // one slab: the clamp leaves 0 whatever the quotient
+            double jf = floor(__ddiv_rn(__dsub_rn(r3, sp.r3_min), sp.slab_width));
+            if (!(jf >= 0.0)) jf = 0.0;  // also NaN
+            if (jf > (double)(sp.nslab - 1)) jf = (double)(sp.nslab - 1);
+            j = (int)jf;
+        }
         const double centre = __dadd_rn(sp.r3_min, __dmul_rn((double)j + 0.5, sp.slab_width));
         sv = __dmul_rn(__dsub_rn(r3, centre), sp.inv_half);
         sv = fmin(1.0, fmax(-1.0, sv));
