@@ -602,7 +602,7 @@ size_t batch_slabs_for(svdi_engine* e, int nslab, int K, long long G) {
 }
 
 // Moment planes from which the error-target rule images through w planes instead (wplanes.cu).
-constexpr int kWPlanesMin = 48;
+constexpr int kWPlanesMin = 24;
 
 // ES transform psi^(k) = integral of psi(x / (W / 2)) cos(2 pi k x) over the support, composite
 // Gauss-Legendre quadrature.
@@ -626,10 +626,11 @@ double es_transform(int W, double beta, double k) {
 // images through Chebyshev moments: other rules than the error target (their truncation is part of the
 // result), other gridders, odd grid sizes (the reference's indexing of those does not commute with the
 // mirrored samples), few moment planes, or when the moments are estimated to be faster. The estimate, fitted
-// to B200 times: a sample and w plane 0.17 ns (its reductions in the L2), a sample and Chebyshev term 0.018
-// ns, a plane's clearing, FFT and recombination 10 ps a cell (12 ps for moments). Measured (w planes against
-// moments): 2.9 M samples, 1536^2 grid, 53 moments 5.5 / 4.1 ms; 0.64 M, 1536^2, 144 moments 2.4 / 4.5 ms;
-// 0.32 M, 3072^2, 43 moments 3.2 / 6.5 ms; 89 k, 384^2, 92 moments 0.40 / 0.55 ms.
+// to B200 times: a sample and w plane 0.11 ns, a sample and Chebyshev term 0.02 ns, a plane's FFT and
+// recombination 8.5 ps a cell (9.2 ps for moments). Measured (w planes / moments, device time of the call):
+// 0.64 M samples, 1536^2 grid, 144 moments 2.1 / 4.2 ms; 768^2, 78 moments 1.14 / 1.33; 0.32 M, 3072^2, 43
+// moments 2.7 / 5.7 and 30 moments 2.3 / 4.0; 89 k, 384^2, 92 moments 0.34 / 0.49; 2.9 M, 1536^2, 53 moments
+// 4.1 / 4.0 and 36 moments 3.9 / 2.7.
 bool plan_wplanes(svdi_engine* e, const SampleSource& src, long long G, const SlabParams& sp, double r3min,
                   double r3max, double mt3, WPlanes& wp) {
     const svdi_options& o = e->opt;
@@ -647,7 +648,7 @@ bool plan_wplanes(svdi_engine* e, const SampleSource& src, long long G, const Sl
     wp.inv_dw = 1.0 / wp.dw;
     const double span = std::floor((hi - wp.lo) * wp.inv_dw * (1.0 + 1e-12)) + wp.W;
     const double n = (double)src.n, cells = (double)G * (double)G;
-    if (!(n * wp.W * 1.7e-7 + span * cells * 1.0e-8 < n * sp.K * 1.8e-8 + (double)sp.nslab * sp.K * cells * 1.2e-8))
+    if (!(n * wp.W * 1.1e-7 + span * cells * 8.5e-9 < n * sp.K * 2.0e-8 + (double)sp.nslab * sp.K * cells * 9.2e-9))
         return false;
     wp.P = (int)span;
     wp.kmax = mt3 * wp.dw;
@@ -847,11 +848,20 @@ int image_wplanes(svdi_engine* e, SampleSource src, const GridGeom& g, const Sla
     const size_t bslabs = batch_slabs_for(e, sp.nslab, sp.K, g.G);
     const int per = (int)std::min<size_t>((size_t)wp.P, bslabs * (size_t)sp.K);
     SVDI_TRY(e->planes.ensure(plane_bytes * per));
-    SVDI_TRY(e->zero.ensure(kZeroCounts * 4));
+    const long long wkeys = (long long)w_tiles(g.G) * w_tiles(g.G);
+    SVDI_TRY(e->zero.ensure((kZeroCounts + (size_t)wkeys) * 4));
+    SVDI_TRY(e->offsets.ensure((size_t)(wkeys + 1) * 4));
+    SVDI_TRY(e->cursor.ensure((size_t)wkeys * 4));
+    SVDI_TRY(e->scan_sums.ensure(scan_sums_words(wkeys) * 4));
+    SVDI_TRY(e->rec.ensure((size_t)src.n * w_record_bytes()));
+    SVDI_TRY(e->chunk_key.ensure(w_list_words(src.n) * 4));
     unsigned long long* const dropped = e->zero.as<unsigned long long>();
     SVDI_CUDA(cudaEventRecord(e->ev[1], st));
-    SVDI_CUDA(cudaMemsetAsync(dropped, 0, 16, st));
+    SVDI_CUDA(cudaMemsetAsync(e->zero.p, 0, (kZeroCounts + (size_t)wkeys) * 4, st));
     src.nonfinite = dropped + 1;
+    if (vis_ready) SVDI_CUDA(cudaStreamWaitEvent(st, vis_ready, 0));
+    SVDI_TRY(launch_bin_w(src, g, wp, e->zero.as<unsigned int>() + kZeroCounts, e->offsets.as<unsigned int>(),
+                          e->cursor.as<unsigned int>(), e->scan_sums.as<unsigned int>(), e->rec.p, st));
     SVDI_CUDA(cudaEventRecord(e->ev[2], st));
     SVDI_TRY(ensure_corr(e, N, g.G, g.W, e->opt.beta));
     SVDI_CUDA(cudaMemsetAsync(d_out, 0, (size_t)N * N * sizeof(float), st));
@@ -866,9 +876,8 @@ int image_wplanes(svdi_engine* e, SampleSource src, const GridGeom& g, const Sla
         FftPlan plan;
         SVDI_TRY(get_plan(e, g.G, N, hi - lo, plan));
         SVDI_CUDA(cudaEventRecord(e->ev[3], st));
-        SVDI_CUDA(cudaMemsetAsync(e->planes.p, 0, plane_bytes * (hi - lo), st));
-        if (lo == 0 && vis_ready) SVDI_CUDA(cudaStreamWaitEvent(st, vis_ready, 0));
-        SVDI_TRY(launch_grid_w(src, g, wp, e->poly, e->wpoly, lo, hi, e->planes.as<float2>(),
+        SVDI_TRY(launch_grid_w(src, g, wp, e->poly, e->wpoly, e->rec.p, e->offsets.as<unsigned int>(),
+                               e->chunk_key.as<unsigned int>(), lo, hi, e->planes.as<float2>(),
                                lo == 0 ? dropped : nullptr, st));
         SVDI_CUDA(cudaEventRecord(e->ev[4], st));
         SVDI_TRY(exec_fft(plan, e->planes.as<cufftComplex>(), hi - lo));

@@ -323,10 +323,19 @@ struct WPlanes {
     double corr[kWCorrTerms];  // 1 / psi^(k) = sum_i corr[i] T_i(2 (k / kmax)^2 - 1)
     float beta_xy;
 };
-// Grids the samples of a separable source into planes [plane_lo, plane_hi); pxy and pz: the kernels of
-// the image axes and of the w axis. Dropped and non-finite samples are counted as the binning does.
+// Bins the samples of a separable source by 8 x 8 tiles of their footprints: w_tiles(G)^2 keys (counts cleared by
+// the caller, offsets one more, d_sums as for launch_scan), w_record_bytes() per sample in d_rec.
+int w_tiles(long long G);
+size_t w_record_bytes();
+size_t w_list_words(long long n);  // of the gridder's work list (d_list)
+int launch_bin_w(const SampleSource& src, const GridGeom& g, const WPlanes& wp, unsigned int* d_counts,
+                 unsigned int* d_offsets, unsigned int* d_cursor, unsigned int* d_sums, void* d_rec, cudaStream_t st);
+// Grids the binned samples into planes [plane_lo, plane_hi), every cell of which is written; pxy and pz: the
+// kernels of the image axes and of the w axis. With d_dropped, dropped and non-finite samples are counted as the
+// binning of the moments does.
 int launch_grid_w(const SampleSource& src, const GridGeom& g, const WPlanes& wp, const EsPoly& pxy, const EsPoly& pz,
-                  int plane_lo, int plane_hi, float2* d_planes, unsigned long long* d_dropped, cudaStream_t st);
+                  const void* d_rec, const unsigned int* d_offsets, unsigned int* d_list, int plane_lo, int plane_hi,
+                  float2* d_planes, unsigned long long* d_dropped, cudaStream_t st);
 
 // image.cu
 // The planes [plane_lo, plane_hi) of a w-plane call; d_acc and final_batch as below.
