@@ -121,6 +121,13 @@ struct DevBuf {
         cap = want;
         return SVDI_OK;
     }
+    // a buffer whose users leave it as zeros: cleared when it is allocated
+    int ensure_zeros(size_t bytes, cudaStream_t st) {
+        const size_t had = cap;
+        SVDI_TRY(ensure(bytes));
+        if (cap != had) SVDI_CUDA(cudaMemsetAsync(p, 0, cap, st));
+        return SVDI_OK;
+    }
     template <typename T>
     T* as() const { return reinterpret_cast<T*>(p); }
 };
@@ -179,7 +186,7 @@ struct svdi_engine {
     // intermediates
     svdi::DevBuf vr, vi, q, s, vin64, vin32, stats, partial, zero, offsets, cursor, counters, rec,
         rec_s, planes, corr, image, cheb_err, bin_out, grid_keep, tc_status, kb_offsets, acc, chunk_key, keymax,
-        plan_buf, scan_sums;
+        plan_buf, scan_sums, mma_slots;
     size_t sz_vr = 0, sz_q = 0, sz_s = 0, sz_off = 0, sz_rec = 0, sz_rec_s = 0, sz_grid = 0, sz_mom = 0;
     const float* cur_vr = nullptr;
     const float* cur_vi = nullptr;
@@ -236,7 +243,7 @@ struct svdi_engine {
              {&in_uvw, &in_freq, &in_v0r, &in_v0i, &in_v3r, &in_v3i, &in_f0, &in_f3, &in_w0, &in_w3, &in_bin, &in_vin, &vr,
               &vi, &q, &s, &vin64, &vin32, &stats, &partial, &zero, &offsets, &cursor, &counters, &rec, &rec_s, &planes,
               &corr, &image, &cheb_err, &bin_out, &grid_keep, &tc_status, &kb_offsets, &acc, &chunk_key, &keymax,
-              &plan_buf, &scan_sums, &probe, &remade})
+              &plan_buf, &scan_sums, &mma_slots, &probe, &remade})
             n += b->cap;
         return n;
     }
@@ -1013,6 +1020,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
         SVDI_TRY(e->kb_offsets.ensure((size_t)(n_keys + 1) * 4));
     } else {  // the FP32 gridders' chunk table
         SVDI_TRY(e->chunk_key.ensure(((size_t)std::max<long long>(n, 1) / chunk + 2) * 4));
+        if (use_mma) SVDI_TRY(e->mma_slots.ensure_zeros(mma_slot_bytes(n, sp.K), st));
     }
     SVDI_TRY(e->scan_sums.ensure(scan_sums_words(n_keys) * 4));
     const bool need_keymax = use_i8 || (!use_tc && !use_mma);  // per-key max |value| (fixed-point gridders)
@@ -1080,7 +1088,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
                                     e->sm_count, st, o.gridder == SVDI_GRIDDER_TC_BF16));
         } else if (use_mma) {
             SVDI_TRY(launch_grid_mma(e->rec.as<SampleRec>(), need_s ? e->rec_s.as<float>() : nullptr,
-                                     e->offsets.as<unsigned int>(), e->chunk_key.as<unsigned int>(), chunk, work,
+                                     e->offsets.as<unsigned int>(), e->chunk_key.as<unsigned int>(), n, e->mma_slots.p, work,
                                      s0 == 0, n_keys, s0 * tiles2, s1 * tiles2, g, sp.K, e->poly, e->planes.as<float2>(),
                                      e->sm_count, st));
         } else {
@@ -1798,7 +1806,7 @@ struct svdi_batch {
     // per Chebyshev order over the keys of all snapshots, one FFT over all moment planes).
     bool wide = false;
     svdi::DevBuf vr, vi, q, s, vin64, vin32, stats, partial, counts, offsets, cursor, keymax, chunk_key,
-        kb_offsets, rec, rec_s, planes, dropped, work, corr, scan_sums, counters;
+        kb_offsets, rec, rec_s, planes, dropped, work, corr, scan_sums, counters, mma_slots;
     svdi::FftPlan fft;
     std::vector<cudaStream_t> lanes;
     std::vector<cudaEvent_t> lane_ev;
@@ -1951,6 +1959,11 @@ int wide_capture(svdi_batch* b) {
     SVDI_TRY(b->keymax.ensure((size_t)nkeys * 4));
     SVDI_TRY(b->chunk_key.ensure(((size_t)std::max<long long>(ntot, 1) / chunk + 2) * 4));
     SVDI_TRY(b->scan_sums.ensure(scan_sums_words(nkeys) * 4));
+    if (mma_batch) {
+        size_t bytes = 0;
+        for (const Group& G : groups) bytes = std::max(bytes, mma_slot_bytes(ntot, G.K));
+        SVDI_TRY(b->mma_slots.ensure_zeros(bytes, e->stream));
+    }
     if (any_tc) SVDI_TRY(b->kb_offsets.ensure((size_t)(nkeys + 1) * 4));
     SVDI_TRY(b->rec.ensure((size_t)std::max<long long>(ntot, 1) * sizeof(SampleRec)));
     if (need_s) SVDI_TRY(b->rec_s.ensure((size_t)std::max<long long>(ntot, 1) * 4));
@@ -2078,7 +2091,7 @@ int wide_capture(svdi_batch* b) {
                                         o.gridder == SVDI_GRIDDER_TC_BF16));
             } else if (G.mma) {
                 SVDI_TRY(launch_grid_mma(b->rec.as<SampleRec>(), need_s ? b->rec_s.as<float>() : nullptr,
-                                         b->offsets.as<unsigned int>(), b->chunk_key.as<unsigned int>(), chunk,
+                                         b->offsets.as<unsigned int>(), b->chunk_key.as<unsigned int>(), ntot, b->mma_slots.p,
                                          b->work.as<unsigned int>() + 4 * gi, true, (int)nkeys, (int)G.key_lo,
                                          (int)G.key_hi, G.g, G.K, e->poly, pl, e->sm_count, st));
             } else {

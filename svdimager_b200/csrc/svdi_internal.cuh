@@ -307,11 +307,14 @@ constexpr int kMmaTile = 8;
 // records per chunk of the scan's table for n records (a power of two, at least kMmaChunkMin)
 constexpr int kMmaChunkMin = 64;
 int mma_chunk(long long n);
-// key_lo: the first tile of a slab; its planes come first in d_planes. d_work: three counters, cleared here
-// unless work_cleared
+// bytes of the sums of dense tiles for n records and K terms; zeros before the first launch, and zeros again
+// after each one
+size_t mma_slot_bytes(long long n, int K);
+// key_lo: the first tile of a slab; its planes come first in d_planes. n: the sample count that the chunk table
+// and d_slots are laid out for (at least the records). d_work: three counters, cleared here unless work_cleared
 int launch_grid_mma(const SampleRec* d_rec, const float* d_rec_s, const unsigned int* d_offsets,
-                    const unsigned int* d_chunk_key, int chunk, unsigned int* d_work, bool work_cleared, int n_keys,
-                    int key_lo, int key_hi, const GridGeom& g, int K, const EsPoly& poly, float2* d_planes,
+                    const unsigned int* d_chunk_key, long long n, void* d_slots, unsigned int* d_work, bool work_cleared,
+                    int n_keys, int key_lo, int key_hi, const GridGeom& g, int K, const EsPoly& poly, float2* d_planes,
                     int sm_count, cudaStream_t st);
 
 // wplanes.cu: imaging through P w planes w_p = lo + (p - (W / 2 - 1)) dw (even grid sizes, support 6 or 8)

@@ -73,3 +73,38 @@ def test_long_runs_match_oracle(cuda_device, n):
     """Both chunk sizes (64 and 256 records), most tiles split over many chunks."""
     grid, ref = _run(n, 48, 8, 1, spread=12.0)
     assert np.linalg.norm(grid[0] - ref[0]) <= GRID_TOL * np.linalg.norm(ref[0])
+
+
+@pytest.mark.parametrize("calls", [((200_000, 1),), ((200_000, 3), (130_003, 6), (200_000, 3))])
+def test_dense_tile_rounding(cuda_device, calls):
+    """Coherent samples of one tile (the sums of 32 chunks are formed apart), several shapes in turn on one
+    engine. Tolerance: n / 2048 sums and at most 62 single chunks are added to a cell, 160 FP32 additions of rms
+    error 0.29 * 2^-23 at up to the whole sum, 2.5e-7; the two polynomials 1.2e-7 each, the splits 2e-7, in
+    squares 3.7e-7, of which 6e-7 leaves room for their all having one sign. (Added chunk by chunk: 1.1e-6.)"""
+    N, cell, G = 64, 2e-3, 96
+    scale = float(np.float32(cell)) * G
+    v = np.eye(3, dtype=np.float32)
+    v[0], v[1] = [0.8, 0.6, 0.0], [-0.6, 0.8, 0.0]
+    engines = {}
+    try:
+        for call, (n, K) in enumerate(calls):
+            rng = np.random.default_rng(call)
+            p = np.clip(rng.normal(3.6, 0.7, (n, 2)), 1.0, 6.0)
+            b = np.concatenate([p / scale, rng.uniform(-40.0, 40.0, (n, 1))], axis=1).astype(np.float32)
+            vr, vi = ((c + 0.1 * rng.normal(size=n)).astype(np.float32) for c in (1.0, 0.3))
+            if K not in engines:
+                engines[K] = api.Engine(api.archive_options(coord_mode=api.COORD_REF32, keep_grid=1, fixed_k=K,
+                                                            k_rule=api.KRULE_FIXED))
+            e = engines[K]
+            e.fipipe(vr, vi, b, v, N, cell)
+            st = e.stats()
+            grid = e.buffer(api.BUF_GRID).reshape(K, G, G)
+            sc = O.SlabConfig(st["slab_r3_min"], st["r3_max"], st["max_abs_t3"], st["alpha_max"], 1, st["slab_width"],
+                              st["slab_half"], 1.0 / st["slab_half"], st["slab_alpha_max"], K)
+            ref = O.grid(b.astype(np.float64), vr, vi, scale, G, sc, 1.0, W=8, coord_mode=1)
+            assert np.linalg.norm(grid[0] - ref[0]) <= 6e-7 * np.linalg.norm(ref[0])
+            for k in range(1, K):  # odd terms nearly cancel over the symmetric w range
+                assert np.linalg.norm(grid[k] - ref[k]) <= 6e-7 * np.linalg.norm(ref[0])
+    finally:
+        for e in engines.values():
+            e.close()
