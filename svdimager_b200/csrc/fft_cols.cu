@@ -9,10 +9,15 @@
 // (e^{+2 pi i m k / R}), multiplies element k by e^{+2 pi i j k / (R S)} and writes it back to
 // b R S + j + S k. The block comes in by asynchronous copies, all of them in flight at once (a first pass
 // straight from the plane, a radix of loads per thread at a time, was slower: 6144 rows 0.33 -> 0.42 ms per
-// plane); the last pass writes the output rows (a table gives the output row of each block row) straight to the
-// plane. The twiddles come from a table of e^{+2 pi i t / G} (FP64-rounded), element k of
-// pass p reading entry j k G / (R S) (< G). The transform is the inverse, unnormalised one, as cuFFT's
-// CUFFT_INVERSE.
+// plane); the last pass writes the output rows (a table gives the output row of each butterfly's first
+// element, the others follow G / R apart) straight to the plane. The transform is the inverse, unnormalised one,
+// as cuFFT's CUFFT_INVERSE.
+//
+// What bounds it: latency of one tile's passes (one or two CTAs per SM, 43 % of the issue slots at 3072 rows),
+// so fewer and shorter accesses count. The twiddles (FP64-rounded) lie in one table per pass, pairs of them
+// 16 bytes, j running fastest: neighbouring threads read one line. Against entries j k G / (R S) of a single
+// table e^{+2 pi i t / G} and a table look-up per output row (columns alone): 2 planes of 1536 rows 24 -> 20 us, of
+// 3072 rows 98 -> 88 us, 116 planes of 6144 rows 22 -> 18 ms.
 //
 // Shared-memory rows are swizzled: block row r sits at row r ^ (f(r >> 3) & mask), f(x) = x ^
 // (x >> 2) ^ (x >> 4), mask = 16 / CB - 1 (the rows that share a 128-byte bank line). The last
@@ -249,20 +254,23 @@ __device__ __forceinline__ void col_pass(float2* __restrict__ sh, const Columns&
         }
         dft_r<R>(v);
         dft_r<R>(u);
-        if (!LAST && j) {  // the last pass has S = 1
-            const int st = j * P.tw_step;
-            int ix = st;
+        if (!LAST) {  // the last pass has S = 1
 #pragma unroll
-            for (int k = 1; k < R; ++k, ix += st) {
-                const float2 w = __ldg(&tw[ix]);
-                v[k] = c_mul(v[k], w);
-                u[k] = c_mul(u[k], w);
+            for (int k = 1; k < R; k += 2) {
+                const float4 w = __ldg(reinterpret_cast<const float4*>(tw) + P.tw_at + (k / 2) * S + j);
+                v[k] = c_mul(v[k], make_float2(w.x, w.y));
+                u[k] = c_mul(u[k], make_float2(w.x, w.y));
+                if (k + 1 < R) {
+                    v[k + 1] = c_mul(v[k + 1], make_float2(w.z, w.w));
+                    u[k + 1] = c_mul(u[k + 1], make_float2(w.z, w.w));
+                }
             }
         }
+        const int row0 = LAST ? __ldg(&out_row[base]) : 0;
 #pragma unroll
         for (int m = 0; m < R; ++m) {
             if (LAST)
-                cols.store(__ldg(&out_row[base + S * m]), c, v[m], u[m]);
+                cols.store(row0 + m * (G / R), c, v[m], u[m]);  // the last digit of the output row
             else
                 *reinterpret_cast<float4*>(sh + (srow(base + S * m, mask) << lcb) + c) =
                     make_float4(v[m].x, v[m].y, u[m].x, u[m].y);
@@ -364,9 +372,9 @@ static int col_fft_lcb(long long G, long long columns) {
 }
 
 // Where it is used: every grid size it supports measured at or below cuFFT's strided column plan (whole FFT,
-// rows by cuFFT in both; us): 288 rows, 8 planes 58 -> 17; 720, 8 planes 91 -> 44; 1500, 4 planes 126 -> 83; 1536,
-// 2 planes 52 -> 42; 2304, 8 planes 407 -> 325; 3072, 2 planes 185 -> 165; 3584, 2 planes 341 -> 235; 4500, 2
-// planes 1037 -> 413; 6144, 2 planes 1025 -> 699 (730 before the last pass wrote the plane itself).
+// rows by cuFFT in both; us): 288 rows, 8 planes 58 -> 17; 720, 8 planes 91 -> 42; 1500, 4 planes 126 -> 79; 1536,
+// 2 planes 52 -> 38; 2304, 8 planes 407 -> 304; 3072, 2 planes 185 -> 155; 3584, 2 planes 341 -> 214; 4500, 2
+// planes 1037 -> 370; 6144, 2 planes 1025 -> 626.
 bool col_fft_supported(long long G) {
     if (G < 16 || G > 12288) return false;
     return !col_radices(G).empty();
@@ -380,13 +388,22 @@ int make_col_fft(long long G, long long columns, ColFftPlan& P, float2** d_tw, i
     }
     P = ColFftPlan{};
     P.npass = (int)rad.size();
+    std::vector<float2> tw;
     long long before = 1;  // product of the earlier radices = G / (R S)
     for (int p = 0; p < P.npass; ++p) {
         long long S = 1;
         for (int q = p + 1; q < P.npass; ++q) S *= rad[q];
         P.pass[p].radix = rad[p];
         P.pass[p].stride = (int)S;
-        P.pass[p].tw_step = (int)before;
+        P.pass[p].tw_at = (int)(tw.size() / 2);
+        if (p + 1 < P.npass)  // pairs k, k + 1 of twiddles e^{2 pi i j k / (R S)}, runs over j
+            for (int k = 1; k < rad[p]; k += 2)
+                for (long long j = 0; j < S; ++j)
+                    for (int i = k; i < k + 2; ++i) {
+                        const long long t = j * i * before % G;
+                        const double a = 2.0 * 3.14159265358979323846 * (double)t / (double)G;
+                        tw.push_back(make_float2((float)std::cos(a), (float)std::sin(a)));
+                    }
         // mul = ceil(2^shift / S), shift = 14 + ceil(log2 S): the quotient is off by less than q / 2^14 / S < 1 / S
         unsigned int shift = 14;
         while ((1LL << (shift - 14)) < S) ++shift;
@@ -395,12 +412,7 @@ int make_col_fft(long long G, long long columns, ColFftPlan& P, float2** d_tw, i
         before *= rad[p];
     }
     P.lcb = col_fft_lcb(G, columns);
-    // tables: e^{+2 pi i t / G} and the digit-reversed position of each output row
-    std::vector<float2> tw((size_t)G);
-    for (long long t = 0; t < G; ++t) {
-        const double a = 2.0 * 3.14159265358979323846 * (double)t / (double)G;
-        tw[(size_t)t] = make_float2((float)std::cos(a), (float)std::sin(a));
-    }
+    // the digit-reversed position of each output row
     std::vector<int> perm((size_t)G);
     for (long long nrow = 0; nrow < G; ++nrow) {
         long long t = nrow, pos = 0;
@@ -411,9 +423,9 @@ int make_col_fft(long long G, long long columns, ColFftPlan& P, float2** d_tw, i
         }
         perm[(size_t)pos] = (int)nrow;  // block row pos holds output row nrow
     }
-    SVDI_CUDA(cudaMalloc(d_tw, (size_t)G * sizeof(float2)));
+    SVDI_CUDA(cudaMalloc(d_tw, tw.size() * sizeof(float2)));
     SVDI_CUDA(cudaMalloc(d_perm, (size_t)G * sizeof(int)));
-    SVDI_CUDA(cudaMemcpy(*d_tw, tw.data(), (size_t)G * sizeof(float2), cudaMemcpyHostToDevice));
+    SVDI_CUDA(cudaMemcpy(*d_tw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice));
     SVDI_CUDA(cudaMemcpy(*d_perm, perm.data(), (size_t)G * sizeof(int), cudaMemcpyHostToDevice));
     return SVDI_OK;
 }

@@ -226,7 +226,7 @@ int launch_dft_probe(const SampleSource& src, const GridGeom& g, const SlabParam
 // divides by the stride; log2 of the columns per CTA
 constexpr int kColFftPasses = 8;
 struct ColFftPass {
-    int radix = 0, stride = 1, tw_step = 1;
+    int radix = 0, stride = 1, tw_at = 0;  // tw_at: the pass' first pair of twiddles
     unsigned int div_mul = 1, div_shift = 0;  // q / stride = (q div_mul) >> div_shift for q < 2^14
 };
 struct ColFftPlan {
