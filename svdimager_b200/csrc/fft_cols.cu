@@ -173,6 +173,37 @@ __device__ __forceinline__ void dft9(float2 (&v)[16]) {
     t = v[5]; v[5] = v[7]; v[7] = t;
 }
 
+// Prime-factor forms (no twiddles): R = 3 Q, input (Q a + 3 b) mod R -> radix-3 DFTs over a, radix-Q DFTs over b;
+// bin (Q Q' k1 + 3 T k2) mod R, Q Q' = 1 mod 3, 3 T = 1 mod Q, ends where input (Q k1 + 3 k2) mod R was.
+__device__ __forceinline__ void dft12(float2 (&v)[16]) {
+#pragma unroll
+    for (int b = 0; b < 4; ++b) dft3(v[3 * b % 12], v[(4 + 3 * b) % 12], v[(8 + 3 * b) % 12]);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) dft4(v[4 * a], v[(4 * a + 3) % 12], v[(4 * a + 6) % 12], v[(4 * a + 9) % 12]);
+    float2 y[12];
+#pragma unroll
+    for (int i = 0; i < 12; ++i) y[(4 * (i / 4) + 9 * (i % 4)) % 12] = v[(4 * (i / 4) + 3 * (i % 4)) % 12];
+#pragma unroll
+    for (int i = 0; i < 12; ++i) v[i] = y[i];
+}
+
+__device__ __forceinline__ void dft24(float2 (&v)[24]) {
+#pragma unroll
+    for (int b = 0; b < 8; ++b) dft3(v[3 * b % 24], v[(8 + 3 * b) % 24], v[(16 + 3 * b) % 24]);
+    float2 y[24];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        float2 t[16];
+#pragma unroll
+        for (int b = 0; b < 8; ++b) t[b] = v[(8 * a + 3 * b) % 24];
+        dft8(t);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) y[(16 * a + 9 * k) % 24] = t[k];
+    }
+#pragma unroll
+    for (int i = 0; i < 24; ++i) v[i] = y[i];
+}
+
 template <int R>
 __device__ __forceinline__ void dft_r(float2 (&v)[16]) {
     if constexpr (R == 2) dft2(v[0], v[1]);
@@ -182,6 +213,7 @@ __device__ __forceinline__ void dft_r(float2 (&v)[16]) {
     else if constexpr (R == 7) dft7(v);
     else if constexpr (R == 8) dft8(v);
     else if constexpr (R == 9) dft9(v);
+    else if constexpr (R == 12) dft12(v);
     else dft16(v);
 }
 
@@ -278,6 +310,28 @@ __device__ __forceinline__ void col_pass(float2* __restrict__ sh, const Columns&
     }
 }
 
+// a first pass of radix 24, a thread one column: two would not fit the registers
+template <int NT>
+__device__ __forceinline__ void pass24(float2* __restrict__ sh, int G, int lcb, const ColFftPass& P,
+                                       const float2* __restrict__ tw) {
+    const int S = P.stride, mask = (16 >> lcb) - 1;
+    for (int t = threadIdx.x; t < S << lcb; t += NT) {
+        const int c = t & ((1 << lcb) - 1), j = t >> lcb;
+        float2 v[24];
+#pragma unroll
+        for (int m = 0; m < 24; ++m) v[m] = sh[(srow(j + S * m, mask) << lcb) + c];
+        dft24(v);
+#pragma unroll
+        for (int k = 1; k < 24; k += 2) {
+            const float4 w = __ldg(reinterpret_cast<const float4*>(tw) + P.tw_at + (k / 2) * S + j);
+            v[k] = c_mul(v[k], make_float2(w.x, w.y));
+            if (k + 1 < 24) v[k + 1] = c_mul(v[k + 1], make_float2(w.z, w.w));
+        }
+#pragma unroll
+        for (int m = 0; m < 24; ++m) sh[(srow(j + S * m, mask) << lcb) + c] = v[m];
+    }
+}
+
 template <int NT, bool LAST>
 __device__ __forceinline__ void any_pass(float2* __restrict__ sh, const Columns& cols, int G, int lcb,
                                          const ColFftPass& P, const float2* __restrict__ tw,
@@ -290,6 +344,10 @@ __device__ __forceinline__ void any_pass(float2* __restrict__ sh, const Columns&
         case 7: col_pass<7, NT, LAST>(sh, cols, G, lcb, P, tw, out_row); break;
         case 8: col_pass<8, NT, LAST>(sh, cols, G, lcb, P, tw, out_row); break;
         case 9: col_pass<9, NT, LAST>(sh, cols, G, lcb, P, tw, out_row); break;
+        case 12: col_pass<12, NT, LAST>(sh, cols, G, lcb, P, tw, out_row); break;
+        case 24:
+            if constexpr (!LAST) pass24<NT>(sh, G, lcb, P, tw);
+            break;
         default: col_pass<16, NT, LAST>(sh, cols, G, lcb, P, tw, out_row); break;
     }
 }
@@ -335,7 +393,13 @@ static std::vector<int> col_radices(long long G) {
     while (g % 7 == 0) g /= 7, odd.push_back(7);
     if (g != 1 || k2 == 0) return {};
     for (; k3 >= 2; k3 -= 2) odd.push_back(9);
-    if (k3) odd.push_back(3);
+    // a lone 3 joins a 4 or an 8 where that saves a pass (24 first: see pass24). Whole FFT, us: 1536 rows = 8 3 8 8
+    // -> 16 12 8, 2 planes 38 -> 36; 3072 = 16 3 8 8 -> 16 12 16, 8 planes 542 -> 523; 6144 = 16 3 16 8 -> 24 16 16,
+    // 2 planes 626 -> 605; 1500 = 4 5 5 5 3 -> 5 5 5 12, 4 planes 79 -> 75
+    int first = 0;
+    if (k3 && (k2 % 4 == 1 || k2 % 4 == 2) && k2 >= 2) odd.push_back(12), k2 -= 2;
+    else if (k3 && k2 % 4 == 3 && k2 > 3) first = 24, k2 -= 3;
+    else if (k3) odd.push_back(3);
     // 16s with a tail of 8s and 4s (no radix-2 pass beside a larger one: 2^5 = 8 4, 2^9 = 8 8 8)
     switch (k2 % 4) {
         case 1:
@@ -351,18 +415,22 @@ static std::vector<int> col_radices(long long G) {
     }
     if (two.empty() || two[0] > 4 || k2 > 2)
         for (; k2 >= 4; k2 -= 4) two.insert(two.begin(), 16);
-    std::vector<int> rad = {two[0]};
+    std::vector<int> rad;
+    if (first) rad.push_back(first);
+    if (!two.empty()) rad.push_back(two[0]);
     rad.insert(rad.end(), odd.begin(), odd.end());
-    rad.insert(rad.end(), two.begin() + 1, two.end());
+    if (!two.empty()) rad.insert(rad.end(), two.begin() + 1, two.end());
     if (rad.size() < 2 || rad.size() > kColFftPasses) return {};
     return rad;
 }
 
-// log2 of the columns per CTA: the largest power of two up to 16 with G * CB * 8 bytes <= 96 KB up to 1536
-// rows (two CTAs per SM), <= 192 KB beyond (one CTA per SM; 6144 rows x 4 columns: 32-byte row
-// segments, where pairs of columns at 96 KB measured slower). At least 1: the passes take pairs of columns.
+// log2 of the columns per CTA: the largest power of two up to 16 with G * CB * 8 bytes <= 96 KB where that gives
+// blocks above 64 KB or 8 columns (two CTAs per SM overlap their copies and passes), else <= 192 KB (one CTA per
+// SM); at least 1: the passes take pairs of columns. Whole FFT, us, at 96 / 192 KB: 1536 rows, 8 planes 126 /
+// 138; 2304, 8 planes 290 / 300; 3072, 2 planes 146 / 152; but 1792, 2 planes 50 / 48; 2048, 2 planes 56 / 54;
+// 3584, 2 planes 220 / 214; 6144, 2 planes 648 / 626.
 static int col_fft_lcb(long long G, long long columns) {
-    const long long cap = G <= 1536 ? 96 * 1024 : 192 * 1024;
+    const long long cap = G <= 1536 || (G > 2048 && G <= 3072) ? 96 * 1024 : 192 * 1024;
     int lcb = 1;
     while (lcb < 4 && G * (2LL << lcb) * 8 <= cap) ++lcb;
     // few columns: narrower blocks until there is a CTA per SM (8 planes of 288 / 384 rows: 19.5 / 25.6 us with
@@ -372,9 +440,9 @@ static int col_fft_lcb(long long G, long long columns) {
 }
 
 // Where it is used: every grid size it supports measured at or below cuFFT's strided column plan (whole FFT,
-// rows by cuFFT in both; us): 288 rows, 8 planes 58 -> 17; 720, 8 planes 91 -> 42; 1500, 4 planes 126 -> 79; 1536,
-// 2 planes 52 -> 38; 2304, 8 planes 407 -> 304; 3072, 2 planes 185 -> 155; 3584, 2 planes 341 -> 214; 4500, 2
-// planes 1037 -> 370; 6144, 2 planes 1025 -> 626.
+// rows by cuFFT in both; us): 288 rows, 8 planes 58 -> 17; 720, 8 planes 91 -> 42; 1500, 4 planes 126 -> 75; 1536,
+// 2 planes 52 -> 36; 2304, 8 planes 407 -> 290; 3072, 2 planes 185 -> 146; 3584, 2 planes 341 -> 214; 4500, 2
+// planes 1037 -> 370; 6144, 2 planes 1025 -> 605.
 bool col_fft_supported(long long G) {
     if (G < 16 || G > 12288) return false;
     return !col_radices(G).empty();
