@@ -33,6 +33,11 @@ __global__ void __launch_bounds__(kThreads) k_histogram(SampleSource src, GridGe
                                                        unsigned int* __restrict__ counts, int n_keys,
                                                        unsigned long long* __restrict__ dropped,
                                                        const DevPlan* __restrict__ plan) {
+    if (plan && first_thread()) {
+        unsigned long long* const stamps = plan_stamps(plan);
+        stamps[STAMP_BIN] = stamp_now();
+        stamps[STAMP_FFT] = stamps[STAMP_END] = 0;  // maxima over the blocks of later kernels
+    }
     if (plan) sp = plan->sp;
     extern __shared__ unsigned int sh[];
     const bool use_smem = n_keys <= kSmemKeyLimit;
@@ -355,6 +360,11 @@ __global__ void __launch_bounds__(kThreads) k_histogram_sep(SampleSource src, Se
                                                            unsigned int* __restrict__ counts, int n_keys,
                                                            unsigned long long* __restrict__ dropped,
                                                            const DevPlan* __restrict__ plan) {
+    if (plan && first_thread()) {
+        unsigned long long* const stamps = plan_stamps(plan);
+        stamps[STAMP_BIN] = stamp_now();
+        stamps[STAMP_FFT] = stamps[STAMP_END] = 0;  // maxima over the blocks of later kernels
+    }
     if (plan) sp = plan->sp;
     extern __shared__ unsigned int sh[];
     const bool use_smem = n_keys <= kSmemKeyLimit;

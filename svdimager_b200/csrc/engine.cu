@@ -212,6 +212,7 @@ struct svdi_engine {
     bool pending_times = false;             // its stage events are valid (single slab batch)
     bool pending_total = false;             // ev[0] -> ev[7] spans the whole call
     bool pending_need_s = false;
+    bool pending_stamps = false;            // stage times: the plan's stamps instead of the events
     long long pending_n = 0;
     std::map<std::tuple<long long, long long, int>, svdi::FftPlan> plans;
     std::map<std::tuple<long long, long long, int, double>, std::vector<float>> corr_cache;
@@ -760,7 +761,18 @@ int finish_pending(svdi_engine* e) {
     L.num_gridded = (size_t)(e->pending_n - (long long)ndrop);
     e->sz_rec = (size_t)(e->pending_n - (long long)ndrop) * sizeof(SampleRec);
     e->sz_rec_s = e->pending_need_s ? (size_t)(e->pending_n - (long long)ndrop) * 4 : 0;
-    if (e->pending_times) {
+    unsigned long long t[STAMP_COUNT] = {};
+    if (e->pending_stamps) {
+        SVDI_CUDA(cudaMemcpyAsync(t, plan_stamps(e->plan_buf.as<DevPlan>()), sizeof(t), cudaMemcpyDeviceToHost, e->stream));
+        SVDI_CUDA(cudaStreamSynchronize(e->stream));
+        if (!t[STAMP_FFT]) t[STAMP_FFT] = t[STAMP_GRID];  // no sample gridded
+        auto ms = [&](int from, int to) { return t[to] > t[from] ? (float)((double)(t[to] - t[from]) * 1e-6) : 0.0f; };
+        L.ms_preprocess = ms(STAMP_PRE, STAMP_BIN);
+        L.ms_bin = ms(STAMP_BIN, STAMP_GRID);
+        L.ms_grid = ms(STAMP_GRID, STAMP_FFT);
+        L.ms_fft = ms(STAMP_FFT, STAMP_IMAGE);
+        L.ms_image = ms(STAMP_IMAGE, STAMP_END);
+    } else if (e->pending_times) {
         float a = 0, b = 0, c = 0, d = 0;
         cudaEventElapsedTime(&d, e->ev[1], e->ev[2]);
         cudaEventElapsedTime(&a, e->ev[3], e->ev[4]);
@@ -773,9 +785,11 @@ int finish_pending(svdi_engine* e) {
     }
     if (e->pending_total) {
         float mp = 0, mt = 0;
-        cudaEventElapsedTime(&mp, e->ev[0], e->ev[1]);
+        if (!e->pending_stamps) {
+            cudaEventElapsedTime(&mp, e->ev[0], e->ev[1]);
+            L.ms_preprocess = mp;
+        }
         cudaEventElapsedTime(&mt, e->ev[0], e->ev[7]);
-        L.ms_preprocess = mp;
         L.ms_total = mt;
     }
     e->pending = false;
@@ -906,6 +920,7 @@ int image_wplanes(svdi_engine* e, SampleSource src, const GridGeom& g, const Sla
     record_stats(e, src, g, sp, sp.nslab * g.ntile * g.ntile2, false, alpha_max, slab_alpha, r3min, r3max, mt3);
     e->pending = true;
     e->pending_times = !multi;
+    e->pending_stamps = false;
     if (multi) {
         e->last.ms_bin = 0;
         e->last.ms_grid = ms[0];
@@ -961,7 +976,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
         if (spec) {
             sp = e->spec_sp;
             if (!prep) {
-                SVDI_TRY(e->plan_buf.ensure(sizeof(DevPlan)));
+                SVDI_TRY(e->plan_buf.ensure(kPlanBytes));
                 SVDI_TRY(launch_plan(e->stats.as<double>(), e->vin64.as<double>(), archive, sp.nslab, sp.K,
                                      e->plan_buf.as<DevPlan>(), st));
             }
@@ -977,6 +992,9 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
     const GridGeom& g = cg.g;
     const bool use_tc = cg.use_tc, use_i8 = cg.use_i8, use_mma = cg.use_mma;
     const int chunk = cg.chunk, n_keys = cg.n_keys;
+    // stage times: stamps of the kernels that see the device plan, else events between the stages
+    const bool stamped = dplan && prep && !prep->uploads && use_mma;
+    const bool evented = timed && !stamped;
 
     if (e->poly_W != g.W || e->poly_beta != o.beta) {
         build_es_poly(g.W, o.beta, &e->poly);
@@ -999,7 +1017,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
     if (forked) SVDI_CUDA(cudaEventRecord(e->ev_clear, side));
 
     // binning
-    if (timed) SVDI_CUDA(cudaEventRecord(e->ev[1], st));
+    if (evented) SVDI_CUDA(cudaEventRecord(e->ev[1], st));
     SVDI_TRY(e->offsets.ensure((size_t)(n_keys + 1) * 4));
     SVDI_TRY(e->cursor.ensure((size_t)n_keys * 4));
     SVDI_TRY(e->rec.ensure((size_t)std::max<long long>(n, 1) * sizeof(SampleRec)));
@@ -1043,7 +1061,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
                             need_s ? e->rec_s.as<float>() : nullptr,
                             use_tc ? e->tc_status.as<unsigned int>() + 1 : nullptr, st,
                             need_keymax ? e->keymax.as<unsigned int>() : nullptr, dplan));
-    if (timed) SVDI_CUDA(cudaEventRecord(e->ev[2], st));
+    if (evented) SVDI_CUDA(cudaEventRecord(e->ev[2], st));
 
     // slab batches: grid -> FFT -> recombine
     if (record) {
@@ -1071,7 +1089,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
         const int s1 = std::min(sp.nslab, s0 + (int)bslabs);
         SlabParams bp = sp;
         if (s0 == 0 && forked) SVDI_CUDA(cudaStreamWaitEvent(st, e->ev_clear, 0));
-        if (timed) SVDI_CUDA(cudaEventRecord(e->ev[3], st));
+        if (evented) SVDI_CUDA(cudaEventRecord(e->ev[3], st));
         if (s0 > 0) SVDI_CUDA(cudaMemsetAsync(e->planes.p, 0, plane_bytes * planes_per_batch, st));
         const int tiles2 = g.ntile * g.ntile2;
         if (use_i8) {
@@ -1090,7 +1108,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
             SVDI_TRY(launch_grid_mma(e->rec.as<SampleRec>(), need_s ? e->rec_s.as<float>() : nullptr,
                                      e->offsets.as<unsigned int>(), e->chunk_key.as<unsigned int>(), n, e->mma_slots.p, work,
                                      s0 == 0, n_keys, s0 * tiles2, s1 * tiles2, g, sp.K, e->poly, e->planes.as<float2>(),
-                                     e->sm_count, st));
+                                     e->sm_count, st, stamped ? plan_stamps(dplan) : nullptr));
         } else {
             SVDI_TRY(launch_grid_fp32(e->rec.as<SampleRec>(), need_s ? e->rec_s.as<float>() : nullptr,
                                       e->offsets.as<unsigned int>(), e->chunk_key.as<unsigned int>(),
@@ -1103,9 +1121,9 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
                                       cudaMemcpyDeviceToDevice, st));
             e->sz_grid = plane_bytes * (size_t)(std::min(sp.nslab, (int)bslabs) * sp.K);
         }
-        if (timed) SVDI_CUDA(cudaEventRecord(e->ev[4], st));
+        if (evented) SVDI_CUDA(cudaEventRecord(e->ev[4], st));
         SVDI_TRY(exec_fft(plan, e->planes.as<cufftComplex>(), planes_per_batch));
-        if (timed) SVDI_CUDA(cudaEventRecord(e->ev[5], st));
+        if (evented) SVDI_CUDA(cudaEventRecord(e->ev[5], st));
         // recombine the slabs of this batch (moment plane index relative to the batch)
         bp.nslab = s1 - s0;
         bp.r3_min = sp.r3_min + (double)s0 * sp.slab_width;
@@ -1113,7 +1131,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
                                   e->corr.as<float>(), 1.0 / (double)n, o.reprojection, o.presplat, d_out,
                                   st, multi_batch ? e->acc.as<double>() : nullptr, s1 == sp.nslab, dplan,
                                   src.nonfinite));
-        if (!timed) continue;
+        if (!evented) continue;
         SVDI_CUDA(cudaEventRecord(e->ev[6], st));
         if (!multi_batch) continue;  // one batch: its stage times are read when the call completes
         SVDI_CUDA(cudaEventSynchronize(e->ev[6]));
@@ -1174,6 +1192,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
     }
     e->pending = true;
     e->pending_times = !multi_batch;
+    e->pending_stamps = stamped;
     e->pending_total = false;
     e->pending_need_s = need_s;
     e->pending_n = n;
@@ -1290,7 +1309,7 @@ int main_path_device(svdi_engine* e, const svdi_host_ms* d, size_t N, float cell
     if (prep.spec) {
         SVDI_TRY(call_geom(e->opt, (long long)N, cell, e->spec_sp, n, cg));
         SVDI_TRY(e->zero.ensure(cg.zero_words() * 4));
-        SVDI_TRY(e->plan_buf.ensure(sizeof(DevPlan)));
+        SVDI_TRY(e->plan_buf.ensure(kPlanBytes));
         prep.zeroed = true;
     }
     SVDI_TRY(launch_preprocess(d->uvw, d->frequencies_hz, R, C, d->array_center_x, e->partial.as<double>(), kPartialCap,

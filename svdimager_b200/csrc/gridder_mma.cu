@@ -310,7 +310,8 @@ __global__ void __launch_bounds__(32 * kWarps, min_ctas<KC>()) k_grid_mma(
     const SampleRec* __restrict__ rec, const float* __restrict__ rec_s, const unsigned int* __restrict__ offsets,
     const unsigned int* __restrict__ chunk_key, int chunk, unsigned int* __restrict__ work, int key_lo, int key_hi,
     GridGeom g, FastDiv by_slab, FastDiv by_row, int K, MmaPoly poly,
-    float2* __restrict__ planes, int term_lo, int groups, DenseSlots dense) {
+    float2* __restrict__ planes, int term_lo, int groups, DenseSlots dense, unsigned long long* __restrict__ stamps) {
+    if (stamps && term_lo == 0 && first_thread()) stamps[STAMP_GRID] = stamp_now();
     constexpr int HW = W / 2;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -618,19 +619,20 @@ __global__ void __launch_bounds__(32 * kWarps, min_ctas<KC>()) k_grid_mma(
         ch = nch;
         kb = nkb;
     }
+    if (stamps && threadIdx.x == 0) atomicMax(stamps + STAMP_FFT, stamp_now());
 }
 
 template <int W, int KC>
 int launch_kc(const SampleRec* d_rec, const float* d_rec_s, const unsigned int* d_offsets,
               const unsigned int* d_chunk_key, int chunk, unsigned int* d_work, int key_lo, int key_hi,
               const GridGeom& g, int K, const MmaPoly& poly, float2* d_planes, int term_lo, int groups,
-              const DenseSlots& dense, int sm_count, cudaStream_t st) {
+              const DenseSlots& dense, int sm_count, cudaStream_t st, unsigned long long* d_stamps) {
     auto kern = k_grid_mma<W, KC>;
     const size_t smem = sizeof(WarpStage<KC>) * kWarps;
     SVDI_TRY(ensure_dynamic_smem((const void*)kern, smem, true));
     kern<<<sm_count * min_ctas<KC>(), 32 * kWarps, smem, st>>>(d_rec, d_rec_s, d_offsets, d_chunk_key, chunk, d_work,
                                                                key_lo, key_hi, g, fast_div(g.ntile * g.ntile2),
-                                                               fast_div(g.ntile2), K, poly, d_planes, term_lo, groups, dense);
+                                                               fast_div(g.ntile2), K, poly, d_planes, term_lo, groups, dense, d_stamps);
     SVDI_LAUNCHED();
     return SVDI_OK;
 }
@@ -639,22 +641,22 @@ template <int W>
 int launch_w(const SampleRec* d_rec, const float* d_rec_s, const unsigned int* d_offsets,
              const unsigned int* d_chunk_key, int chunk, unsigned int* d_work, int key_lo, int key_hi,
              const GridGeom& g, int K, const MmaPoly& poly, float2* d_planes, const DenseSlots& dense, int sm_count,
-             cudaStream_t st) {
+             cudaStream_t st, unsigned long long* d_stamps) {
     int t0 = 0;
     if (K >= 4) {
         const int n = K / 4;
         SVDI_TRY((launch_kc<W, 4>(d_rec, d_rec_s, d_offsets, d_chunk_key, chunk, d_work, key_lo, key_hi, g, K,
-                                  poly, d_planes, t0, n, dense, sm_count, st)));
+                                  poly, d_planes, t0, n, dense, sm_count, st, d_stamps)));
         t0 += 4 * n;
     }
     if (K - t0 >= 2) {
         SVDI_TRY((launch_kc<W, 2>(d_rec, d_rec_s, d_offsets, d_chunk_key, chunk, d_work + 1, key_lo, key_hi, g, K,
-                                  poly, d_planes, t0, 1, dense, sm_count, st)));
+                                  poly, d_planes, t0, 1, dense, sm_count, st, d_stamps)));
         t0 += 2;
     }
     if (K - t0 >= 1)
         SVDI_TRY((launch_kc<W, 1>(d_rec, d_rec_s, d_offsets, d_chunk_key, chunk, d_work + 2, key_lo, key_hi, g, K,
-                                  poly, d_planes, t0, 1, dense, sm_count, st)));
+                                  poly, d_planes, t0, 1, dense, sm_count, st, d_stamps)));
     return SVDI_OK;
 }
 
@@ -681,7 +683,7 @@ size_t mma_slot_bytes(long long n, int K) { return slot_count(n, K) * (kSlotWord
 int launch_grid_mma(const SampleRec* d_rec, const float* d_rec_s, const unsigned int* d_offsets,
                     const unsigned int* d_chunk_key, long long n, void* d_slots, unsigned int* d_work, bool work_cleared,
                     int n_keys, int key_lo, int key_hi, const GridGeom& g, int K, const EsPoly& poly, float2* d_planes,
-                    int sm_count, cudaStream_t st) {
+                    int sm_count, cudaStream_t st, unsigned long long* d_stamps) {
     if (key_lo < 0 || key_hi > n_keys || key_lo >= key_hi || key_hi - key_lo > (1 << 26) || g.T != kMmaTile ||
         g.T2 != kMmaTile) {
         set_error("matrix gridder: bad key range or tile size");
@@ -700,8 +702,8 @@ int launch_grid_mma(const SampleRec* d_rec, const float* d_rec_s, const unsigned
             (d & 1 ? p.ox[i][d / 2] : p.ex[i][d / 2]) = poly.c[i][d] * kWeightScale;
         }
     switch (g.W) {
-        case 6: return launch_w<6>(d_rec, d_rec_s, d_offsets, d_chunk_key, chunk, d_work, key_lo, key_hi, g, K, p, d_planes, dense, sm_count, st);
-        case 8: return launch_w<8>(d_rec, d_rec_s, d_offsets, d_chunk_key, chunk, d_work, key_lo, key_hi, g, K, p, d_planes, dense, sm_count, st);
+        case 6: return launch_w<6>(d_rec, d_rec_s, d_offsets, d_chunk_key, chunk, d_work, key_lo, key_hi, g, K, p, d_planes, dense, sm_count, st, d_stamps);
+        case 8: return launch_w<8>(d_rec, d_rec_s, d_offsets, d_chunk_key, chunk, d_work, key_lo, key_hi, g, K, p, d_planes, dense, sm_count, st, d_stamps);
         default:
             set_error("matrix gridder: ES support must be 6 or 8");
             return SVDI_ERR_UNSUPPORTED;

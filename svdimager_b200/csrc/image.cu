@@ -267,6 +267,7 @@ __global__ void __launch_bounds__(256, 4) k_recombine(const float2* __restrict__
                                                   float* __restrict__ out, double* __restrict__ acc,
                                                   int final_batch, const DevPlan* __restrict__ plan,
                                                   const unsigned long long* __restrict__ nonfinite) {
+    if (plan && first_thread()) plan_stamps(plan)[STAMP_IMAGE] = stamp_now();
     if (plan) {  // one batch of all slabs: the device plan's slab geometry
         sp.r3_min = plan->sp.r3_min;
         sp.slab_width = plan->sp.slab_width;
@@ -287,6 +288,7 @@ __global__ void __launch_bounds__(256, 4) k_recombine(const float2* __restrict__
             recombine_pixel<KMAX>(x, y, moments, g, N, cell, vin, sp, corr, inv_n, reprojection, presplat, out, acc,
                                   final_batch, bad, kc);
     }
+    if (plan && threadIdx.x == 0) atomicMax(plan_stamps(plan) + STAMP_END, stamp_now());
 }
 
 // J_0 .. J_{KT-1}: bessel_jn_fast with the ascending series (|x| < 1e-3) unrolled in registers.
@@ -322,6 +324,7 @@ __global__ void __launch_bounds__(256, 3) k_recombine_few(const float2* __restri
                                                       int presplat, float* __restrict__ out, double* __restrict__ acc,
                                                       int final_batch, const DevPlan* __restrict__ plan,
                                                       const unsigned long long* __restrict__ nonfinite) {
+    if (plan && first_thread()) plan_stamps(plan)[STAMP_IMAGE] = stamp_now();
     if (plan) {  // one batch of all slabs: the device plan's slab geometry
         sp.r3_min = plan->sp.r3_min;
         sp.slab_width = plan->sp.slab_width;
@@ -432,6 +435,7 @@ __global__ void __launch_bounds__(256, 3) k_recombine_few(const float2* __restri
         }
         splat(out, N, half, LL, MM, value);
     }
+    if (plan && threadIdx.x == 0) atomicMax(plan_stamps(plan) + STAMP_END, stamp_now());
 }
 
 template <int KT>

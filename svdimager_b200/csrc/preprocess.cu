@@ -73,7 +73,8 @@ __global__ void __launch_bounds__(kThreads) k_row_basis(const float* __restrict_
                                                        float array_center_x, double* __restrict__ vin64,
                                                        float* __restrict__ vin32, double* __restrict__ s_out,
                                                        double* __restrict__ stats, unsigned int* __restrict__ zero,
-                                                       long long n_zero) {
+                                                       long long n_zero, DevPlan* __restrict__ plan) {
+    if (plan && first_thread()) plan_stamps(plan)[STAMP_PRE] = stamp_now();
     __shared__ double sm[9 * kThreads];
     for (long long i = blockIdx.x * (long long)kThreads + threadIdx.x; i < n_zero; i += (long long)gridDim.x * kThreads)
         zero[i] = 0u;
@@ -437,7 +438,7 @@ int launch_preprocess(const float* d_uvw, const float* d_freq, long long R, long
     // a block per SM at most: the last block's serial part grows with their number
     const int nb = grid_for(R, std::min(partial_cap, current_sm_count()));
     k_row_basis<<<nb, kThreads, 0, st>>>(d_uvw, R, d_partial, d_counters, d_freq, C, array_center_x, d_vin64, d_vin32,
-                                         d_s, d_stats, d_zero, n_zero);
+                                         d_s, d_stats, d_zero, n_zero, d_plan);
     SVDI_LAUNCHED();
     if (after_basis) SVDI_CUDA(cudaEventRecord(after_basis, st));
     k_project_rows<<<grid_for(R, 4 * current_sm_count()), kThreads, 0, st>>>(d_uvw, R, d_vin64, d_stats, d_q, d_partial,
