@@ -962,15 +962,24 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
         r3min = fixed->r3min;
         r3max = fixed->r3max;
         mt3 = fixed->mt3;
-    } else {
-        // statistics: max |t3|, then one small read, beside the binning of a speculative call
-        if (forked) SVDI_CUDA(cudaStreamWaitEvent(side, e->ev_basis, 0));
+    }
+    // statistics: max |t3|, then one small read
+    auto read_stats = [&](cudaEvent_t basis) -> int {
+        if (forked) SVDI_CUDA(cudaStreamWaitEvent(side, basis, 0));
         SVDI_TRY(launch_t3_stats(e->vin64.as<double>(), N, cell, e->partial.as<double>() + 5 * kPartialCap, kPartialCap,
                                  e->counters.as<unsigned int>() + 2, e->stats.as<double>(), side));
         if (forked) SVDI_CUDA(cudaStreamWaitEvent(side, e->ev_rows, 0));
         SVDI_CUDA(cudaMemcpyAsync(e->h_stats, e->stats.p, ST_COUNT * sizeof(double), cudaMemcpyDeviceToHost, side));
         SVDI_CUDA(cudaMemcpyAsync(e->h_stats + ST_COUNT, e->vin64.p, 9 * sizeof(double), cudaMemcpyDeviceToHost, side));
         SVDI_CUDA(cudaEventRecord(e->ev_stats, side));
+        return SVDI_OK;
+    };
+    // a speculative call needs them for the check at its end only, and an event between two kernels costs an
+    // idle device some 3 us: they are read beside its gridding, after the event that follows the binning (192^2
+    // image 115 -> 108 us, 256^2 149 -> 142; after an event that follows the scan 112 and 144)
+    const bool late_stats = prep && prep->spec && forked;
+    if (!fixed) {
+        if (!late_stats) SVDI_TRY(read_stats(e->ev_basis));
         const bool spec = prep ? prep->spec
                                : allow_spec && !record && spec_usable(e, archive, N, cell_f, src, spec_bslabs);
         if (spec) {
@@ -1062,6 +1071,10 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
                             use_tc ? e->tc_status.as<unsigned int>() + 1 : nullptr, st,
                             need_keymax ? e->keymax.as<unsigned int>() : nullptr, dplan));
     if (evented) SVDI_CUDA(cudaEventRecord(e->ev[2], st));
+    if (late_stats) {
+        SVDI_CUDA(cudaEventRecord(e->ev_rows, st));
+        SVDI_TRY(read_stats(e->ev_rows));
+    }
 
     // slab batches: grid -> FFT -> recombine
     if (record) {
@@ -1314,10 +1327,11 @@ int main_path_device(svdi_engine* e, const svdi_host_ms* d, size_t N, float cell
     }
     SVDI_TRY(launch_preprocess(d->uvw, d->frequencies_hz, R, C, d->array_center_x, e->partial.as<double>(), kPartialCap,
                                e->counters.as<unsigned int>(), e->vin64.as<double>(), e->vin32.as<float>(),
-                               e->q.as<double>(), e->s.as<double>(), e->stats.as<double>(), st, e->ev_basis,
+                               e->q.as<double>(), e->s.as<double>(), e->stats.as<double>(), st,
+                               prep.spec && !uploads ? nullptr : e->ev_basis,  // (image_core: late_stats)
                                e->zero.as<unsigned int>(), prep.zeroed ? (long long)cg.zero_words() : 0,
                                prep.spec ? e->plan_buf.as<DevPlan>() : nullptr, e->spec_sp.nslab, e->spec_sp.K));
-    SVDI_CUDA(cudaEventRecord(e->ev_rows, st));
+    if (!(prep.spec && !uploads)) SVDI_CUDA(cudaEventRecord(e->ev_rows, st));
     SVDI_TRY(image_core(e, false, src, (long long)N, cell, d_out, fixed, record, d_status_out, e->ev_vis, true, true,
                         &prep));
     if (fixed) return SVDI_OK;
