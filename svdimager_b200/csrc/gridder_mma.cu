@@ -664,8 +664,10 @@ int launch_w(const SampleRec* d_rec, const float* d_rec_s, const unsigned int* d
 
 // Records per chunk: small inputs need many chunks to fill 148 SMs x 12-20 warps, large ones lose more to
 // the extra reductions of tiles split between chunks (6.5 M samples: 64 / 128 / 256 / 512 records 0.52 /
-// 0.41 / 0.40 / 0.42 ms; 1.04 M samples: 64 / 128 records 0.107 / 0.14 ms, 32 no faster).
-int mma_chunk(long long n) { return n >= 2000000 ? 256 : 64; }
+// 0.41 / 0.40 / 0.42 ms; 1.04 M samples: 64 / 128 records 0.107 / 0.14 ms, 32 no faster). Below 64 records for
+// each of 148 x 12 warps a chunk's own time counts: 24 k samples, 8 terms, whole call 110 us with 64, 106 with 32
+// (130 k samples: 141.6 / 141.7).
+int mma_chunk(long long n) { return n >= 2000000 ? 256 : n >= 64 * 148 * 12 ? 64 : 32; }
 
 namespace {
 // Chunks per slot, as a power of two: 32 (136 additions per cell instead of 4360 where 0.28 M samples share one

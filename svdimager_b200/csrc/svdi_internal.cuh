@@ -323,8 +323,7 @@ void build_es_poly(int W, double beta, EsPoly* out);
 
 // gridder_mma.cu: the FP32 gridder on warp-level matrix instructions (support <= 8, 8 x 8 tiles)
 constexpr int kMmaTile = 8;
-// records per chunk of the scan's table for n records (a power of two, at least kMmaChunkMin)
-constexpr int kMmaChunkMin = 64;
+// records per chunk of the scan's table for n records (a power of two)
 int mma_chunk(long long n);
 // bytes of the sums of dense tiles for n records and K terms; zeros before the first launch, and zeros again
 // after each one

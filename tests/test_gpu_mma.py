@@ -68,9 +68,9 @@ def test_planes_match_oracle(cuda_device, n, N, W, K):
         assert err <= GRID_TOL * den, (k, err, den)
 
 
-@pytest.mark.parametrize("n", [600_000, 2_100_000])
+@pytest.mark.parametrize("n", [113_663, 600_000, 2_100_000])
 def test_long_runs_match_oracle(cuda_device, n):
-    """Both chunk sizes (64 and 256 records), most tiles split over many chunks."""
+    """The chunk sizes (32, 64 and 256 records), most tiles split over many chunks."""
     grid, ref = _run(n, 48, 8, 1, spread=12.0)
     assert np.linalg.norm(grid[0] - ref[0]) <= GRID_TOL * np.linalg.norm(ref[0])
 
