@@ -522,7 +522,8 @@ def run_ours(args):
     dom = max(ours, key=ours.get)
     if dom == "ms_grid":
         alg = grid_kernel_bytes(st["num_gridded"], planes, G)
-        name = (("k_grid_i8" if args.gridder == "tc_i8" else "k_grid_tc") if st["used_tc"] else "k_grid_fp32") \
+        fp32 = "k_grid_mma" if st["tile"] == 8 else "k_grid_fp32"
+        name = (("k_grid_i8" if args.gridder == "tc_i8" else "k_grid_tc") if st["used_tc"] else fp32) \
             + " (+ plane zeroing)"
     elif dom == "ms_bin":
         alg = (26 + 8) * snap.num_samples + 16 * st["num_gridded"]
@@ -558,7 +559,8 @@ def run_ours(args):
         "config": {
             "workload": f"{args.config}: {snap.num_rows} baselines x {snap.num_channels} channels = "
                         f"{snap.num_samples} vis, one snapshot, {N}^2 image, cell {cell} rad",
-            "gridder": GRIDDER_LABEL[args.gridder] if st["used_tc"] else "fp32 fixed-point",
+            "gridder": GRIDDER_LABEL[args.gridder] if st["used_tc"] else (
+                "fp32 matrix-instruction (FP16 hi+lo products, FP32 sums)" if st["tile"] == 8 else "fp32 fixed-point"),
             "grid": G, "planes": planes, "num_slabs": st["num_slabs"], "chebyshev_terms": st["num_terms"],
             "support": 8, "beta": 15.3704324328, "oversampling": 1.5, "tile": st["tile"],
             "k_rule": "target 1e-6", "edges": "strict (samples whose footprint leaves the grid are dropped)",
@@ -583,8 +585,8 @@ def run_ours(args):
         "roofline": {"bound": "hbm", "kernel": name, "achieved": round(achieved, 1), "peak": peak,
                      "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": traffic,
                      "peak_kind": peak_kind,
-                     "limiter": ("warp-instruction issue: the gridder is a shared-memory reduction of 64 "
-                                 "cells per sample, its DRAM traffic is small" if dom == "ms_grid" else None),
+                     "limiter": ("warp-instruction issue: weights, FP16 splits and operand loads of 64 cells "
+                                 "per sample, its DRAM traffic is small" if dom == "ms_grid" else None),
                      "snapshot_alg_bytes": algorithmic_bytes(snap.num_samples, snap.num_rows,
                                                              snap.num_channels, planes, G, N),
                      "snapshot_frac": round(algorithmic_bytes(snap.num_samples, snap.num_rows,
@@ -846,7 +848,7 @@ def main():
     ap.add_argument("--gridder", default="fp32", choices=["tc", "tc_bf16", "tc_i8", "fp32"],
                     help="tc: split-precision tcgen05 gridder (FP16 hi+lo); tc_bf16: the same with BF16 hi+lo; "
                          "tc_i8: exact integer tcgen05 gridder (three byte digits, int32 sums); "
-                         "fp32: CUDA-core fixed-point gridder")
+                         "fp32: FP32 gridder (matrix-instruction form at the automatic tile size)")
     args = ap.parse_args()
     if args.warmup < 3:
         args.warmup = 3

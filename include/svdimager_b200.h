@@ -129,7 +129,8 @@ typedef struct svdi_engine svdi_engine;
 #define SVDI_REPROJ_SII 0        /* simplified SIN deprojection (SVDIntegratedImager.cu)        */
 #define SVDI_REPROJ_FIPK 1       /* trigonometric SIN deprojection (archive/FIPkernels.cu)      */
 
-#define SVDI_GRIDDER_FP32 0      /* tile-local FP32 gridder (CUDA cores, shared memory)         */
+#define SVDI_GRIDDER_FP32 0      /* tile-local FP32 gridder: matrix-instruction form on 8 x 8 tiles
+                                  * (automatic tile, support <= 8), else CUDA cores              */
 #define SVDI_GRIDDER_TC 1        /* split-precision tcgen05 tensor-core gridder, FP16 hi + lo   */
 #define SVDI_GRIDDER_TC_BF16 2   /* the same with BF16 hi + lo operands (16-bit significand)    */
 #define SVDI_GRIDDER_TC_I8 3     /* exact integer tcgen05 gridder: 3-byte digits, int32 sums    */
@@ -185,19 +186,22 @@ typedef struct svdi_stats {
     size_t grid_size;            /* G                                                          */
     int num_slabs;               /* w-slabs                                                    */
     int num_terms;               /* Chebyshev terms K                                          */
-    int num_planes;              /* num_slabs * K moment planes                                */
+    int num_planes;              /* num_slabs * K moment planes (also of calls that image through
+                                  * fewer w planes: SVDI_KRULE_TARGET, wide fields)             */
     double r3_min, r3_max;       /* range of the third rotated coordinate (wavelengths)        */
     double max_abs_t3;           /* max |t3| over valid pixels                                 */
     size_t valid_pixels;
     double alpha_max;            /* 2 pi max|t3| (r3 range / 2)                                */
     double slab_alpha_max;
     double vin[9];               /* FP64 basis used                                            */
-    int tile;                    /* gridder tile rows                                          */
+    int tile;                    /* gridder tile rows (8: matrix-instruction form)             */
     int tile_cols;               /* gridder tile columns                                       */
     int used_tc;                 /* 1 when the tensor-core gridder ran                         */
     int num_keys;                /* tile keys: num_slabs * ceil(G/T)^2                         */
     double slab_r3_min, slab_width, slab_half;  /* slab geometry used by the gridder           */
     float ms_total;              /* device time of the call (CUDA events)                      */
+    /* stage times: events, or the kernels' own time stamps (repeated device calls of one shape,
+     * where each stage then lasts until the next one starts)                                    */
     float ms_preprocess, ms_bin, ms_grid, ms_fft, ms_image;
 } svdi_stats;
 
