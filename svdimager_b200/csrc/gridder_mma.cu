@@ -31,10 +31,10 @@
 // the rest per tile), then the L2's reductions (16-byte reductions of 64-byte row pieces add 4.7 TB/s,
 // 8-byte ones of 32-byte pieces 3.3 TB/s: hence the column order of b_row). Gridding stage, B200, against the
 // fixed-point shared-memory gridder (gridder.cu, which keeps supports above 8 and the explicit tile
-// sizes 32 and 64): 6.5 M samples, 2 terms, 3072^2 grid 0.541 -> 0.365 ms; 1.04 M, 2 terms, 1536^2
-// 0.324 -> 0.100 ms; support 6 at 2048^2 0.590 -> 0.115 ms; 130 k samples, 8 terms, 384^2 0.119 ->
-// 0.061 ms; 0.64 M samples, 59 terms, 2304^2 7.7 -> 3.1 ms. Error against 64 bits is lower on every
-// configuration measured (device images 0.85-0.95 of before).
+// sizes 32 and 64): 6.5 M samples, 2 terms, 3072^2 grid 0.541 -> 0.315 ms; 1.04 M, 2 terms, 1536^2
+// 0.324 -> 0.080 ms; support 6 at 2048^2 0.590 -> 0.098 ms; 130 k samples, 8 terms, 384^2 0.119 ->
+// 0.043 ms; 0.64 M samples, 59 terms, 2304^2 7.7 -> 3.1 ms. Error against 64 bits over 143 random images:
+// median 0.86, at most 1.03 of that gridder's.
 #include "svdi_internal.cuh"
 
 #include <cuda_fp16.h>
