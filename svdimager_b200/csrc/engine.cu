@@ -92,17 +92,19 @@ constexpr int kZeroWork = 4, kZeroCounts = 8;
 // Frees the idle engines of the two-step entry's pool; true when there were any.
 bool drop_idle_engines();
 
-// Grow-only device buffer.
+// Grow-only device buffer. `keep` (optional): outgrown allocations go there instead of being freed.
 struct DevBuf {
     void* p = nullptr;
     size_t cap = 0;
+    std::vector<void*>* keep = nullptr;
     ~DevBuf() {
         if (p) cudaFree(p);
     }
     int ensure(size_t bytes) {
         if (bytes <= cap) return SVDI_OK;
         if (p) {
-            cudaFree(p);
+            if (keep) keep->push_back(p);
+            else cudaFree(p);
             p = nullptr;
             cap = 0;
         }
@@ -236,17 +238,29 @@ struct svdi_engine {
     svdi::DevBuf probe, remade;
     // pageable host uploads and image downloads of the archive entry and the host-input call
     svdi::HostStager stager;
-    bool batch_bound = false;  // a batch's captured graph refers to this engine's buffers
+    bool batch_bound = false;  // it holds a batch
+    // A chained batch's graph runs on this engine's buffers: until the batch is destroyed, other calls of the
+    // engine leave the allocations it refers to where they are (those they outgrow wait in `kept`).
+    bool graph_bound = false;
+    std::vector<void*> kept;
 
-    size_t device_bytes() const {
+    std::vector<svdi::DevBuf*> buffers() {
+        return {&in_uvw, &in_freq, &in_v0r, &in_v0i, &in_v3r, &in_v3i, &in_f0, &in_f3, &in_w0, &in_w3, &in_bin, &in_vin,
+                &vr, &vi, &q, &s, &vin64, &vin32, &stats, &partial, &zero, &offsets, &cursor, &counters, &rec, &rec_s,
+                &planes, &corr, &image, &cheb_err, &bin_out, &grid_keep, &tc_status, &kb_offsets, &acc, &chunk_key,
+                &keymax, &plan_buf, &scan_sums, &mma_slots, &probe, &remade};
+    }
+    size_t device_bytes() {
         size_t n = 0;
-        for (const svdi::DevBuf* b :
-             {&in_uvw, &in_freq, &in_v0r, &in_v0i, &in_v3r, &in_v3i, &in_f0, &in_f3, &in_w0, &in_w3, &in_bin, &in_vin, &vr,
-              &vi, &q, &s, &vin64, &vin32, &stats, &partial, &zero, &offsets, &cursor, &counters, &rec, &rec_s, &planes,
-              &corr, &image, &cheb_err, &bin_out, &grid_keep, &tc_status, &kb_offsets, &acc, &chunk_key, &keymax,
-              &plan_buf, &scan_sums, &mma_slots, &probe, &remade})
-            n += b->cap;
+        for (const svdi::DevBuf* b : buffers()) n += b->cap;
         return n;
+    }
+    void bind_graph(bool on) {
+        graph_bound = on;
+        for (svdi::DevBuf* b : buffers()) b->keep = on ? &kept : nullptr;
+        if (on) return;
+        for (void* p : kept) cudaFree(p);
+        kept.clear();
     }
 
     ~svdi_engine() {
@@ -642,7 +656,9 @@ double es_transform(int W, double beta, double k) {
 bool plan_wplanes(svdi_engine* e, const SampleSource& src, long long G, const SlabParams& sp, double r3min,
                   double r3max, double mt3, WPlanes& wp) {
     const svdi_options& o = e->opt;
-    if (o.k_rule != SVDI_KRULE_TARGET || o.target_error < 1e-8 || o.gridder != SVDI_GRIDDER_FP32 || o.tile != 0 ||
+    // not while a chained batch holds the moments' buffers: its graph was recorded through the moments, and the
+    // planes and records of this form would come on top
+    if (e->graph_bound || o.k_rule != SVDI_KRULE_TARGET || o.target_error < 1e-8 || o.gridder != SVDI_GRIDDER_FP32 || o.tile != 0 ||
         (o.support != 6 && o.support != 8) || o.keep_grid || src.bin || (G & 1) || sp.nslab * sp.K < kWPlanesMin ||
         !(mt3 > 0.0) || src.R <= 0 || src.n % src.R || G < 32)
         return false;
@@ -1853,6 +1869,7 @@ struct svdi_batch {
     cudaStream_t split_stream = nullptr;
     cudaEvent_t ev_split_fork = nullptr, ev_split_join = nullptr;
     ~svdi_batch() {
+        // e is not set before the batch is complete, so no caller holds its mutex
         if (second) delete second;  // releases own_engine's binding
         if (own_engine) svdi_engine_destroy(own_engine);
         if (e) cudaSetDevice(e->device);
@@ -1865,7 +1882,11 @@ struct svdi_batch {
         for (auto ev : lane_ev) cudaEventDestroy(ev);
         for (auto st : lanes) cudaStreamDestroy(st);
         if (ev_fork) cudaEventDestroy(ev_fork);
-        if (e) e->batch_bound = false;
+        if (e) {
+            std::lock_guard<std::mutex> lk(e->mu);
+            e->bind_graph(false);
+            e->batch_bound = false;
+        }
     }
 };
 
@@ -2245,6 +2266,11 @@ int batch_create_one(svdi_engine* e, const svdi_host_ms* snapshots, size_t num_s
     SVDI_CUDA(cudaGraphInstantiate(&b->exec, b->graph, 0));
     b->e = e;
     e->batch_bound = true;
+    e->bind_graph(true);
+    // the correction table is uploaded on the host's side, so the graph's own one goes with the batch
+    std::swap(b->corr, e->corr);
+    b->corr.keep = nullptr;
+    e->corr_key = {-1, -1, -1, 0.0};
     *out = b.release();
     return SVDI_OK;
 }
