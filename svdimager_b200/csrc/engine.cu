@@ -1636,8 +1636,10 @@ static int materialise_moments(svdi_engine* e, int which) {
     const svdi_stats kept = e->last;
     const size_t N = (size_t)e->last_N;
     SVDI_TRY(e->remade.ensure(N * N * sizeof(float)));
-    SVDI_TRY(image_core(e, false, e->last_src, (long long)N, (float)e->last_cell, e->remade.as<float>(), nullptr, nullptr,
-                        nullptr, nullptr, false, false));
+    const int rc = image_core(e, false, e->last_src, (long long)N, (float)e->last_cell, e->remade.as<float>(), nullptr,
+                              nullptr, nullptr, nullptr, false, false);
+    e->spec_valid = false;  // the next call of this shape goes through w planes like the one before
+    SVDI_TRY(rc);
     SVDI_TRY(finish_pending(e));
     e->last = kept;
     return SVDI_OK;

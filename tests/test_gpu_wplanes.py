@@ -123,6 +123,26 @@ def test_buffers_and_next_calls(cuda_device):
         assert O.rel_rms(e.image(flat), c.image(flat)) < 1e-6  # a Chebyshev call after it
 
 
+def test_reading_buffers_keeps_the_route(cuda_device):
+    """The calls that follow a buffer read launch the kernels of the calls before it (the moments take others)."""
+    s = _snap(256, 4, 3000)
+    with api.Engine(k_rule=api.KRULE_TARGET, target_error=1e-6, edge_mode=api.EDGE_STRICT) as e:
+        def launches():
+            n0 = api.kernel_launch_count()
+            e.image(s)
+            return api.kernel_launch_count() - n0
+
+        e.image(s)
+        before = launches()
+        e.buffer(api.BUF_RECORDS)
+        assert [launches() for _ in range(3)] == [before] * 3
+        with api.Engine(k_rule=api.KRULE_TARGET, target_error=1e-6, edge_mode=api.EDGE_STRICT, keep_grid=1) as c:
+            c.image(s)
+            n0 = api.kernel_launch_count()
+            c.image(s)
+            assert api.kernel_launch_count() - n0 != before
+
+
 def test_non_finite_visibility(cuda_device):
     s = _snap(256, 4, 3000)
     v = s.vis0_real.copy()
