@@ -214,6 +214,7 @@ struct svdi_engine {
     bool pending_times = false;             // its stage events are valid (single slab batch)
     bool pending_total = false;             // ev[0] -> ev[7] spans the whole call
     bool pending_need_s = false;
+    bool pending_records = false;           // its records are held or can be made
     bool pending_stamps = false;            // stage times: the plan's stamps instead of the events
     long long pending_n = 0;
     std::map<std::tuple<long long, long long, int>, svdi::FftPlan> plans;
@@ -775,8 +776,9 @@ int finish_pending(svdi_engine* e) {
     svdi_stats& L = e->last;
     const unsigned long long ndrop = *e->h_ndrop;
     L.num_gridded = (size_t)(e->pending_n - (long long)ndrop);
-    e->sz_rec = (size_t)(e->pending_n - (long long)ndrop) * sizeof(SampleRec);
-    e->sz_rec_s = e->pending_need_s ? (size_t)(e->pending_n - (long long)ndrop) * 4 : 0;
+    const size_t records = e->pending_records ? L.num_gridded : 0;
+    e->sz_rec = records * sizeof(SampleRec);
+    e->sz_rec_s = e->pending_need_s ? records * 4 : 0;
     unsigned long long t[STAMP_COUNT] = {};
     if (e->pending_stamps) {
         SVDI_CUDA(cudaMemcpyAsync(t, plan_stamps(e->plan_buf.as<DevPlan>()), sizeof(t), cudaMemcpyDeviceToHost, e->stream));
@@ -867,6 +869,14 @@ void record_stats(svdi_engine* e, const SampleSource& src, const GridGeom& g, co
     L.slab_alpha_max = slab_alpha;
 }
 
+// A new call is about to overwrite the inputs that the records and moments of a last call through w planes would
+// be made from: it has none from here on, also if the new call fails.
+void forget_w_call(svdi_engine* e) {
+    if (!e->last_w) return;
+    e->last_w = e->pending_records = false;
+    e->sz_off = e->sz_rec = e->sz_rec_s = e->sz_mom = 0;
+}
+
 // The imaging of one call through w planes (plan_wplanes), as many planes at a time as the memory rule of
 // the Chebyshev batches allows. The statistics report the Chebyshev configuration that the error target
 // asks for (sp); the records, the grid and the moments of it are made when they are asked for
@@ -946,8 +956,10 @@ int image_wplanes(svdi_engine* e, SampleSource src, const GridGeom& g, const Sla
     e->pending_total = false;
     e->pending_need_s = sp.K > 1;
     e->pending_n = src.n;
+    e->pending_records = true;
     e->sz_off = (size_t)(sp.nslab * g.ntile * g.ntile2 + 1) * 4;
     e->sz_mom = plane_bytes * bslabs * (size_t)sp.K;
+    e->last_w = true;
     return SVDI_OK;
 }
 
@@ -1028,8 +1040,8 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
     }
 
     WPlanes wp{};
-    e->last_w = timed && !record && !dplan && allow_w && !use_tc && plan_wplanes(e, src, g.G, sp, r3min, r3max, mt3, wp);
-    if (e->last_w)
+    forget_w_call(e);
+    if (timed && !record && !dplan && allow_w && !use_tc && plan_wplanes(e, src, g.G, sp, r3min, r3max, mt3, wp))
         return image_wplanes(e, src, g, sp, wp, N, cell, d_out, vis_ready, alpha_max, slab_alpha, r3min, r3max, mt3);
 
     // the planes of the first slab batch and the image are cleared on the side stream, beside the binning
@@ -1225,6 +1237,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
     e->pending_total = false;
     e->pending_need_s = need_s;
     e->pending_n = n;
+    e->pending_records = true;
     if (multi_batch) {
         float mb = 0;
         cudaEventElapsedTime(&mb, e->ev[1], e->ev[2]);
@@ -1304,6 +1317,7 @@ int main_path_device(svdi_engine* e, const svdi_host_ms* d, size_t N, float cell
     cudaStream_t st = e->stream;
     const long long R = (long long)d->num_rows, C = (long long)d->num_channels;
     const long long n = (long long)d->num_samples;
+    forget_w_call(e);
     if (!fixed) SVDI_CUDA(cudaEventRecord(e->ev[0], st));
     SVDI_TRY(e->vr.ensure(n * 4));
     SVDI_TRY(e->vi.ensure(n * 4));
@@ -1378,6 +1392,7 @@ int archive_path(svdi_engine* e, const float* Visreal, const float* Visimag, con
     SVDI_TRY(check_archive_args(Visreal, Visimag, Bin, Vin, dirty_image, n, N, cell));
     cudaStream_t st = e->stream;
     SVDI_CUDA(cudaSetDevice(e->device));
+    forget_w_call(e);
     SVDI_CUDA(cudaEventRecord(e->ev[0], st));
     SVDI_TRY(upload_staged(e, e->vr, Visreal, n, st));
     SVDI_TRY(upload_staged(e, e->vi, Visimag, n, st));

@@ -143,6 +143,20 @@ def test_reading_buffers_keeps_the_route(cuda_device):
             assert api.kernel_launch_count() - n0 != before
 
 
+def test_failed_call_after_w_planes(cuda_device):
+    """A call that fails has overwritten the inputs that the last call's records and moments would be made from:
+    there are none then, rather than some of other inputs, and the next call is as before."""
+    s = _snap(256, 4, 3000)
+    bad = dataclasses.replace(s, uvw=np.full_like(s.uvw, np.nan))
+    with api.Engine(k_rule=api.KRULE_TARGET, target_error=1e-6, edge_mode=api.EDGE_STRICT) as e:
+        img = e.image(s)
+        with pytest.raises(api.SvdiError):
+            e.image(bad)
+        assert all(len(e.buffer(b)) == 0 for b in (api.BUF_OFFSETS, api.BUF_RECORDS, api.BUF_RECORDS_S, api.BUF_MOMENTS))
+        assert O.rel_rms(e.image(s), img) < 1e-6
+        assert len(e.buffer(api.BUF_RECORDS)) == e.stats()["num_gridded"] > 0
+
+
 def test_non_finite_visibility(cuda_device):
     s = _snap(256, 4, 3000)
     v = s.vis0_real.copy()
