@@ -17,6 +17,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <deque>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -218,6 +219,7 @@ struct svdi_engine {
     bool pending_stamps = false;            // stage times: the plan's stamps instead of the events
     long long pending_n = 0;
     std::map<std::tuple<long long, long long, int>, svdi::FftPlan> plans;
+    std::deque<std::tuple<long long, long long, int>> many_plans;  // row plans of many planes, oldest use first
     std::map<std::tuple<long long, long long, int, double>, std::vector<float>> corr_cache;
     std::tuple<long long, long long, int, double> corr_key{-1, -1, -1, 0.0};
     std::map<std::tuple<double, int, int>, std::vector<double>> cheb_cache;
@@ -459,28 +461,27 @@ int choose_slabs(svdi_engine* e, bool archive, double r3min, double r3max, doubl
 // CTA per block of adjacent columns, one launch over all planes); other smooth sizes use a
 // strided cuFFT column plan per plane. Grid sizes with a prime factor above 7 (cuFFT's Bluestein
 // path, which gave wrong in-place results for the interleaved column batches on B200) keep one 2-D
-// plan.
+// plan. batch = 0 makes the column part only, N = 0 the rows (or the 2-D transform) only: the parts that
+// many planes are transformed with (exec_fft_many).
 int make_fft_plan(long long G, long long N, int batch, cudaStream_t st, FftPlan& plan) {
     long long r = G;
     for (long long f : {2, 3, 5, 7})
         while (r % f == 0) r /= f;
     int n = (int)G;
     if (r == 1) {
-        SVDI_CUFFT(cufftPlanMany(&plan.rows, 1, &n, &n, 1, n, &n, 1, n, CUFFT_C2C, (int)(G * batch)));
-        if (col_fft_supported(G)) {
-            SVDI_TRY(make_col_fft(G, N * batch, plan.cp, &plan.d_tw, &plan.d_perm));
-            plan.mode = FftPlan::kRowsSharedCols;
-        } else {
+        if (batch) SVDI_CUFFT(cufftPlanMany(&plan.rows, 1, &n, &n, 1, n, &n, 1, n, CUFFT_C2C, (int)(G * batch)));
+        plan.mode = col_fft_supported(G) ? FftPlan::kRowsSharedCols : FftPlan::kRowsCufftCols;
+        if (N && plan.mode == FftPlan::kRowsSharedCols)
+            SVDI_TRY(make_col_fft(G, N * std::max(batch, 1), plan.cp, &plan.d_tw, &plan.d_perm));
+        else if (N)
             SVDI_CUFFT(cufftPlanMany(&plan.cols, 1, &n, &n, n, 1, &n, n, 1, CUFFT_C2C, (int)N));
-            plan.mode = FftPlan::kRowsCufftCols;
-        }
     } else {
         int dims[2] = {n, n};
-        SVDI_CUFFT(cufftPlanMany(&plan.rows, 2, dims, nullptr, 1, n * n, nullptr, 1, n * n, CUFFT_C2C, batch));
-        plan.cols = 0;
+        if (batch)
+            SVDI_CUFFT(cufftPlanMany(&plan.rows, 2, dims, nullptr, 1, n * n, nullptr, 1, n * n, CUFFT_C2C, batch));
         plan.mode = FftPlan::kFull2D;
     }
-    SVDI_CUFFT(cufftSetStream(plan.rows, st));
+    if (batch) SVDI_CUFFT(cufftSetStream(plan.rows, st));
     if (plan.cols) SVDI_CUFFT(cufftSetStream(plan.cols, st));
     plan.stream = st;
     plan.G = G;
@@ -501,8 +502,7 @@ int get_plan(svdi_engine* e, long long G, long long N, int batch, FftPlan& plan)
     return SVDI_OK;
 }
 
-int exec_fft(const FftPlan& plan, cufftComplex* planes, int nplanes) {
-    SVDI_CUFFT(cufftExecC2C(plan.rows, planes, planes, CUFFT_INVERSE));
+int exec_fft_cols(const FftPlan& plan, cufftComplex* planes, int nplanes) {
     if (plan.mode == FftPlan::kFull2D) return SVDI_OK;
     const long long c0 = plan.G / 2 - plan.N / 2;
     if (plan.mode == FftPlan::kRowsSharedCols)
@@ -513,6 +513,39 @@ int exec_fft(const FftPlan& plan, cufftComplex* planes, int nplanes) {
         SVDI_CUFFT(cufftExecC2C(plan.cols, col0, col0, CUFFT_INVERSE));
     }
     return SVDI_OK;
+}
+
+int exec_fft(const FftPlan& plan, cufftComplex* planes, int nplanes) {
+    SVDI_CUFFT(cufftExecC2C(plan.rows, planes, planes, CUFFT_INVERSE));
+    return exec_fft_cols(plan, planes, nplanes);
+}
+
+// The same for the many planes of wide fields. Their number follows the snapshot's w range, so a long-lived engine
+// meets ever new ones: the row plans (0.4 MB and more, 0.6 to 1 ms to make) of the last kManyPlans numbers are kept,
+// and the column part serves all of them. `evict`: no graph that uses older plans exists or is being recorded. Plans
+// of fixed sizes put together (64 + 32 + .. planes) need no new ones, but took 23 us more of a 3250 us call (46 planes
+// of 2304^2) and 8 ms more of an engine's first one.
+constexpr int kManyPlanes = 24;
+constexpr size_t kManyPlans = 32;
+int exec_fft_many(svdi_engine* e, long long G, long long N, cufftComplex* planes, int nplanes, bool evict) {
+    const auto key = std::make_tuple(G, 0LL, nplanes);
+    const auto used = std::find(e->many_plans.begin(), e->many_plans.end(), key);
+    if (used != e->many_plans.end()) e->many_plans.erase(used);
+    while (evict && !e->graph_bound && e->many_plans.size() >= kManyPlans) {
+        SVDI_CUDA(cudaStreamSynchronize(e->stream));
+        const auto old = e->plans.find(e->many_plans.front());
+        if (old != e->plans.end()) {
+            destroy_fft_plan(old->second);
+            e->plans.erase(old);
+        }
+        e->many_plans.pop_front();
+    }
+    FftPlan rows, cols;
+    SVDI_TRY(get_plan(e, G, 0, nplanes, rows));
+    e->many_plans.push_back(key);
+    SVDI_TRY(get_plan(e, G, N, 0, cols));
+    SVDI_CUFFT(cufftExecC2C(rows.rows, planes, planes, CUFFT_INVERSE));
+    return exec_fft_cols(cols, planes, nplanes);
 }
 
 // 1 / Phi(i), i = 0..N/2: inverse of the ES kernel's Fourier transform at image offset i, computed
@@ -625,7 +658,7 @@ size_t batch_slabs_for(svdi_engine* e, int nslab, int K, long long G) {
 }
 
 // Moment planes from which the error-target rule images through w planes instead (wplanes.cu).
-constexpr int kWPlanesMin = 24;
+constexpr int kWPlanesMin = kManyPlanes;
 
 // ES transform psi^(k) = integral of psi(x / (W / 2)) cos(2 pi k x) over the support, composite
 // Gauss-Legendre quadrature.
@@ -920,14 +953,12 @@ int image_wplanes(svdi_engine* e, SampleSource src, const GridGeom& g, const Sla
     float ms[3] = {0, 0, 0};  // gridding, FFT, recombination
     for (int lo = 0; lo < wp.P; lo += per) {
         const int hi = std::min(wp.P, lo + per);
-        FftPlan plan;
-        SVDI_TRY(get_plan(e, g.G, N, hi - lo, plan));
         SVDI_CUDA(cudaEventRecord(e->ev[3], st));
         SVDI_TRY(launch_grid_w(src, g, wp, e->poly, e->wpoly, e->rec.p, e->offsets.as<unsigned int>(),
                                e->chunk_key.as<unsigned int>(), lo, hi, e->planes.as<float2>(),
                                lo == 0 ? dropped : nullptr, st));
         SVDI_CUDA(cudaEventRecord(e->ev[4], st));
-        SVDI_TRY(exec_fft(plan, e->planes.as<cufftComplex>(), hi - lo));
+        SVDI_TRY(exec_fft_many(e, g.G, N, e->planes.as<cufftComplex>(), hi - lo, true));
         SVDI_CUDA(cudaEventRecord(e->ev[5], st));
         SVDI_TRY(launch_recombine_w(e->planes.as<float2>(), g, N, cell, e->vin64.as<double>(), wp, lo, hi,
                                     e->corr.as<float>(), 1.0 / (double)src.n, e->opt.reprojection, e->opt.presplat,
@@ -1116,7 +1147,8 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
         record->bslabs = bslabs;
     }
     FftPlan plan;
-    SVDI_TRY(get_plan(e, g.G, N, planes_per_batch, plan));
+    const bool many = planes_per_batch >= kManyPlanes;
+    if (!many) SVDI_TRY(get_plan(e, g.G, N, planes_per_batch, plan));
     SVDI_TRY(ensure_corr(e, N, g.G, g.W, o.beta));
     // slabs split over several batches: the signed sums of all batches before |.| (the reference
     // takes |.| per batch, SVDIntegratedImager.cu:1445, inside its batch loop at :1681)
@@ -1163,7 +1195,8 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
             e->sz_grid = plane_bytes * (size_t)(std::min(sp.nslab, (int)bslabs) * sp.K);
         }
         if (evented) SVDI_CUDA(cudaEventRecord(e->ev[4], st));
-        SVDI_TRY(exec_fft(plan, e->planes.as<cufftComplex>(), planes_per_batch));
+        if (many) SVDI_TRY(exec_fft_many(e, g.G, N, e->planes.as<cufftComplex>(), planes_per_batch, !record && !fixed));
+        else SVDI_TRY(exec_fft(plan, e->planes.as<cufftComplex>(), planes_per_batch));
         if (evented) SVDI_CUDA(cudaEventRecord(e->ev[5], st));
         // recombine the slabs of this batch (moment plane index relative to the batch)
         bp.nslab = s1 - s0;

@@ -157,6 +157,21 @@ def test_failed_call_after_w_planes(cuda_device):
         assert len(e.buffer(api.BUF_RECORDS)) == e.stats()["num_gridded"] > 0
 
 
+def test_many_w_ranges_on_one_engine(cuda_device):
+    """Snapshots of changing w range need another number of planes each (about 90 numbers here). The engine keeps
+    the row plans of the last 32: after 40 numbers a new plan takes an old one's place, up to the fragments of a few
+    2 MB allocations."""
+    import torch
+    s = _snap(512, 2, 4000)
+    free = []
+    with api.Engine(k_rule=api.KRULE_TARGET, target_error=1e-6, edge_mode=api.EDGE_STRICT) as e:
+        for f in np.linspace(1.0, 0.3, 96):  # all baselines shorter: the same rotation, a smaller w range
+            e.image(dataclasses.replace(s, uvw=s.uvw * np.float32(f)))
+            assert e.stats()["num_planes"] >= 24
+            free.append(torch.cuda.mem_get_info()[0])
+    assert free[39] - min(free[40:]) <= 8 << 20
+
+
 def test_non_finite_visibility(cuda_device):
     s = _snap(256, 4, 3000)
     v = s.vis0_real.copy()
