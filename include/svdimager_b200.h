@@ -102,7 +102,7 @@ int svdi_preprocess_measurement_set(const svdi_host_ms* host, svdi_device_buffer
 int svdi_fipipe_device(const svdi_device_buffers* dev, float* dirty_image, size_t image_size,
                        float cell_size);
 
-/* Replaces free_device_preprocess_buffers (SVDIntegratedImager.cu:855-865). */
+/* Replaces free_device_preprocess_buffers (SVDIntegratedImager.cu:855-865). Waits for the device. */
 void svdi_free_device_buffers(svdi_device_buffers* dev);
 
 /* Copies `bytes` from a device array of svdi_device_buffers (or any device pointer of this process)

@@ -1490,21 +1490,24 @@ std::unique_ptr<svdi_engine> take_idle_engine(int device) {
 }
 
 void give_idle_engine(std::unique_ptr<svdi_engine> e) {
+    // The caller's own work on the descriptor's arrays, on whatever stream, ends before another snapshot is written
+    // over them (destroying the engine waits for the device too).
+    int dev = 0;
+    const bool have = cudaGetDevice(&dev) == cudaSuccess;
+    const bool idle = cudaSetDevice(e->device) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess;
     // a new descriptor decides its slab batches by the memory that is free then, and starts without a plan
     e->bslab_cache.clear();
     e->spec_valid = false;
     e->have_last = false;
     e->last_w = false;
-    {
+    if (idle) {
         std::lock_guard<std::mutex> lk(g_idle_mu);
         size_t held = e->device_bytes();
         for (const auto& other : g_idle) held += other->device_bytes();
-        if (g_idle.size() < kIdleEngines && held <= kIdleBytes) {
-            g_idle.push_back(std::move(e));
-            return;
-        }
+        if (g_idle.size() < kIdleEngines && held <= kIdleBytes) g_idle.push_back(std::move(e));
     }
     e.reset();  // outside the lock: freeing device memory waits for the device
+    if (have) cudaSetDevice(dev);
 }
 
 int default_engine(svdi_engine** out) {

@@ -69,3 +69,30 @@ def test_threads(cuda_device, cases):
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+def test_freeing_waits_for_the_callers_streams(cuda_device, cases):
+    """Work that the caller has queued on a descriptor's arrays reads them, not the next snapshot's."""
+    import dataclasses
+    import torch
+
+    class View:
+        def __init__(self, ptr, n):
+            self.__cuda_array_interface__ = dict(shape=(n,), typestr="<f4", data=(ptr, False), version=3)
+
+    s, _ = cases[0]
+    other = dataclasses.replace(s, vis0_real=s.vis0_real + 1.0, vis3_real=s.vis3_real + 1.0)
+    api.preprocess_measurement_set_gpu(s).free()
+    b = api.preprocess_measurement_set_gpu(s)
+    ref = torch.as_tensor(View(b.buf.d_vis_real, s.num_samples), device="cuda").clone()
+    got = torch.zeros_like(ref)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(200_000_000)  # some 0.1 s
+        got.copy_(torch.as_tensor(View(b.buf.d_vis_real, s.num_samples), device="cuda"))
+    b.free()
+    c = api.preprocess_measurement_set_gpu(other)
+    torch.cuda.synchronize()
+    c.free()
+    assert torch.equal(got, ref)
