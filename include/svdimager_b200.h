@@ -102,8 +102,12 @@ int svdi_preprocess_measurement_set(const svdi_host_ms* host, svdi_device_buffer
 int svdi_fipipe_device(const svdi_device_buffers* dev, float* dirty_image, size_t image_size,
                        float cell_size);
 
-/* Replaces free_device_preprocess_buffers (SVDIntegratedImager.cu:855-865). Waits for the device. */
+/* Replaces free_device_preprocess_buffers (SVDIntegratedImager.cu:855-865). Waits for the device. The
+ * descriptor's engine is kept for the next svdi_preprocess_measurement_set: at most two idle engines and
+ * 1 GiB of device memory in all, with up to 48 MB of pinned host memory each. They go when an allocation
+ * of this library fails, or by svdi_release_idle_engines. */
 void svdi_free_device_buffers(svdi_device_buffers* dev);
+void svdi_release_idle_engines(void);
 
 /* Copies `bytes` from a device array of svdi_device_buffers (or any device pointer of this process)
  * into host memory and waits for the copy; for callers without their own CUDA runtime. No

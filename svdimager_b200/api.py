@@ -38,7 +38,7 @@ EXPORTED_SYMBOLS = (
     "svdi_server_submit", "svdi_server_wait", "svdi_server_poll", "svdi_server_stats",
     "svdi_server_destroy", "svdi_engine_dft_pixels", "svdi_batch_create", "svdi_batch_launch",
     "svdi_batch_check", "svdi_batch_plan", "svdi_batch_mode", "svdi_batch_destroy", "svdi_copy_to_host", "_Z6FIpipePfS_S_S_S_mmf",
-    "svdi_create", "svdi_submit", "svdi_poll", "svdi_wait", "svdi_destroy",
+    "svdi_release_idle_engines", "svdi_create", "svdi_submit", "svdi_poll", "svdi_wait", "svdi_destroy",
 )
 NOALLOC_MAX_KEYS = 16384
 
@@ -139,6 +139,7 @@ def lib():
         L.svdi_fipipe_device.argtypes = [ctypes.POINTER(DeviceBuffers), P, sz, f]
         L.svdi_free_device_buffers.argtypes = [ctypes.POINTER(DeviceBuffers)]
         L.svdi_free_device_buffers.restype = None
+        L.svdi_release_idle_engines.restype = None
         L.svdi_copy_to_host.argtypes = [P, P, sz]
         L.svdi_default_options.argtypes = [ctypes.POINTER(Options)]
         L.svdi_default_options.restype = None
@@ -431,6 +432,11 @@ def FIpipeDevice(buffers: PreprocessBuffers, image_size: int, cell_size: float) 
 
 def free_device_preprocess_buffers(buffers: PreprocessBuffers):
     buffers.free()
+
+
+def release_idle_engines():
+    """Free what freed descriptors keep for the next preprocess_measurement_set_gpu."""
+    lib().svdi_release_idle_engines()
 
 
 class Server:

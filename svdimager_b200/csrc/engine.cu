@@ -157,6 +157,15 @@ struct FftPlan {
     int batch = 0;
 };
 
+size_t fft_plan_bytes(const FftPlan& plan) {
+    size_t n = (size_t)2 << 20;
+    for (cufftHandle h : {plan.rows, plan.cols}) {
+        size_t work = 0;
+        if (h && cufftGetSize(h, &work) == CUFFT_SUCCESS) n += work;
+    }
+    return n;
+}
+
 void destroy_fft_plan(FftPlan& plan) {
     if (plan.rows) cufftDestroy(plan.rows);
     if (plan.cols) cufftDestroy(plan.cols);
@@ -253,9 +262,11 @@ struct svdi_engine {
                 &planes, &corr, &image, &cheb_err, &bin_out, &grid_keep, &tc_status, &kb_offsets, &acc, &chunk_key,
                 &keymax, &plan_buf, &scan_sums, &mma_slots, &probe, &remade};
     }
+    // buffers, the plans' tables and work areas, and 2 MB for what else cuFFT holds per plan
     size_t device_bytes() {
         size_t n = 0;
         for (const svdi::DevBuf* b : buffers()) n += b->cap;
+        for (const auto& kv : plans) n += svdi::fft_plan_bytes(kv.second);
         return n;
     }
     void bind_graph(bool on) {
@@ -497,7 +508,17 @@ int get_plan(svdi_engine* e, long long G, long long N, int batch, FftPlan& plan)
         plan = it->second;
         return SVDI_OK;
     }
-    SVDI_TRY(make_fft_plan(G, N, batch, e->stream, plan));
+    int rc = make_fft_plan(G, N, batch, e->stream, plan);
+    if (rc != SVDI_OK) {
+        destroy_fft_plan(plan);
+        if (drop_idle_engines()) {  // memory that only the idle pool holds
+            cudaGetLastError();
+            rc = make_fft_plan(G, N, batch, e->stream, plan);
+            if (rc == SVDI_OK) set_error("");
+            else destroy_fft_plan(plan);
+        }
+    }
+    SVDI_TRY(rc);
     e->plans[key] = plan;
     return SVDI_OK;
 }
@@ -1470,9 +1491,11 @@ std::map<int, std::unique_ptr<svdi_engine>> g_default_engines;
 // Idle engines of the two-step entry (svdi_preprocess_measurement_set ... svdi_free_device_buffers): the
 // entry used to make and destroy an engine per snapshot -- streams, some 25 allocations, a cuFFT plan --
 // which took 7 of the 8.5 ms of a 512^2 call with 130 k samples. A freed engine waits here for the next
-// call, at most kIdleEngines of them and kIdleBytes of their device memory in all; beyond that it is
-// destroyed as before, and a failing allocation of this library destroys them all and tries again. An engine
-// is owned by one descriptor at a time; the pool itself is guarded by a mutex.
+// call, at most kIdleEngines of them and kIdleBytes of their device memory in all (with each, its pinned 48 MB
+// staging ring and copy threads, if it has staged); beyond that it is destroyed as before. A failing allocation of
+// device memory in this library, its FFT plans included, destroys them all and tries again, and
+// svdi_release_idle_engines does so for the caller. An engine is owned by one descriptor at a time; the pool itself
+// is guarded by a mutex.
 constexpr size_t kIdleEngines = 2;
 constexpr size_t kIdleBytes = (size_t)1 << 30;
 std::mutex g_idle_mu;
@@ -1869,6 +1892,8 @@ int svdi_copy_to_host(void* host_dst, const void* device_src, size_t bytes) {
     SVDI_CUDA(cudaMemcpy(host_dst, device_src, bytes, cudaMemcpyDeviceToHost));
     return SVDI_OK;
 }
+
+void svdi_release_idle_engines(void) { drop_idle_engines(); }
 
 void svdi_free_device_buffers(svdi_device_buffers* dev) {
     if (!dev) return;
