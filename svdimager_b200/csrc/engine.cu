@@ -1518,8 +1518,10 @@ void give_idle_engine(std::unique_ptr<svdi_engine> e) {
     int dev = 0;
     const bool have = cudaGetDevice(&dev) == cudaSuccess;
     const bool idle = cudaSetDevice(e->device) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess;
-    // a new descriptor decides its slab batches by the memory that is free then, and starts without a plan
+    // a new descriptor decides its slab batches by the memory that is free then, and starts without a plan and
+    // without the truncation errors found for this one's w range
     e->bslab_cache.clear();
+    e->cheb_cache.clear();
     e->spec_valid = false;
     e->have_last = false;
     e->last_w = false;

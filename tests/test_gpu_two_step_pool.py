@@ -117,3 +117,15 @@ def test_freeing_waits_for_the_callers_streams(cuda_device, cases):
     torch.cuda.synchronize()
     c.free()
     assert torch.equal(got, ref)
+
+
+def test_taken_over_engines_keep_no_answers(cuda_device, cases):
+    """A snapshot imaged again on a taken-over engine launches what it launches on a new one."""
+    s, _ = cases[0]
+    counts = []
+    api.release_idle_engines()
+    for _ in range(3):
+        n0 = api.kernel_launch_count()
+        _two_step(s)
+        counts.append(api.kernel_launch_count() - n0)
+    assert counts[1:] == counts[:1] * 2, counts
