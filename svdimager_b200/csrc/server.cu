@@ -71,12 +71,17 @@ struct svdi_server {
 namespace svdi {
 namespace {
 
-// Device bytes one request needs in a slot: raw inputs, collapsed visibilities, binned records,
-// one moment plane per Chebyshev term (the estimate assumes `planes` planes) and the image.
-size_t request_bytes(const svdi_host_ms& ms, size_t N, double sigma, int planes) {
+// Device bytes one request needs in a slot: raw inputs, collapsed visibilities, binned records (the larger ones of
+// w planes where the error target may take those), one moment plane per Chebyshev term (the estimate assumes
+// `planes` planes), the image, and 64 MiB for what is left: the matrix gridder's sums of dense tiles (32 MiB at
+// most), key tables, FFT tables.
+size_t request_bytes(const svdi_host_ms& ms, size_t N, const svdi_options& o) {
     const size_t n = ms.num_samples;
-    const size_t G = (size_t)std::ceil(sigma * (double)N) + 8;
-    return n * (26 + 8 + 20) + ms.num_rows * 36 + (size_t)planes * G * G * 8 + N * N * 4 + (64u << 20);
+    const size_t G = (size_t)std::ceil(o.sigma * (double)N) + 8;
+    const bool w_planes = o.k_rule == SVDI_KRULE_TARGET && o.gridder == SVDI_GRIDDER_FP32;
+    const size_t records = w_planes ? n * w_record_bytes() + w_list_words(n) * 4 : n * 20;
+    const size_t planes = o.k_rule == SVDI_KRULE_BUCKET ? 8 : 2;
+    return n * (26 + 8) + records + ms.num_rows * 36 + planes * G * G * 8 + N * N * 4 + (64u << 20);
 }
 
 void worker_loop(svdi_server* s, int slot) {
@@ -210,7 +215,7 @@ int svdi_server_submit(svdi_server* s, const svdi_host_ms* ms, size_t N, float c
     r->N = N;
     r->cell = cell;
     r->out = out_image;
-    r->est_bytes = request_bytes(*ms, N, s->opt.sigma, s->opt.k_rule == SVDI_KRULE_BUCKET ? 8 : 2);
+    r->est_bytes = request_bytes(*ms, N, s->opt);
     if (r->est_bytes > s->budget) {
         set_error("request needs ~" + std::to_string(r->est_bytes >> 20) + " MiB of device memory, more than the "
                   "server's HBM budget of " + std::to_string(s->budget >> 20) + " MiB");

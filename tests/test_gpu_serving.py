@@ -103,6 +103,23 @@ def test_tight_budget_counts_resident_buffers_and_drains(alone, mix):
         assert 0 < peak <= budget
 
 
+def test_wide_field_requests_are_charged_what_they_hold(cuda_device):
+    """A wide field of 8.4 M samples under the error target images through w planes, whose records are twice as
+    large as the moments' ones: a slot's device memory stays within its charge. The small image keeps the planes
+    below 1 % of it; a small request before it loads what CUDA loads once."""
+    import torch
+    s = synth.make_snapshot("widefield")
+    first = synth.make_snapshot("widefield", nchan=4, n_rows_limit=3000)
+    opt = dict(k_rule=api.KRULE_TARGET, target_error=1e-6, edge_mode=api.EDGE_STRICT)
+    with api.Engine(**opt) as e:
+        e.image(first, 64, 0.3 / 64)
+    with api.Server(num_slots=1, **opt) as srv:
+        free = torch.cuda.mem_get_info()[0]
+        srv.wait(srv.submit(s, 64, 0.3 / 64), timeout_s=120)
+        held = free - torch.cuda.mem_get_info()[0]
+        assert held <= srv.stats()["hbm_in_use"]
+
+
 def test_malformed_requests_are_refused(cuda_device, mix):
     s, N, cell = mix[0]
     with api.Server(num_slots=1) as srv:
