@@ -176,10 +176,22 @@ def algorithmic_bytes(n_samples, n_rows, n_chan, planes, G, N):
     return 26 * n_samples + 24 * n_rows + 8 * n_chan + 32 * planes * G * G + 4 * N * N
 
 
-def grid_kernel_bytes(n_gridded, planes, G):
-    """Algorithmic bytes of the gridding stage: one 16 B record read per gridded sample and one
-    8 B write per moment-plane cell."""
-    return 16 * n_gridded + 8 * planes * G * G
+def grid_kernel_bytes(n_gridded, planes, G, record=16):
+    """Algorithmic bytes of the gridding stage: one record read per gridded sample (16 B; 32 B for
+    w planes) and one 8 B write per cell of the planes."""
+    return record * n_gridded + 8 * planes * G * G
+
+
+def gridding_stage(st, w_planes, gridder):
+    """(name, planes, algorithmic bytes) of the gridding stage of a call with statistics `st`."""
+    planes = w_planes or st["num_planes"]
+    if w_planes:
+        name = "k_grid_w (+ split and rare samples)"
+    elif st["used_tc"]:
+        name = ("k_grid_i8" if gridder == "tc_i8" else "k_grid_tc") + " (+ plane zeroing)"
+    else:
+        name = ("k_grid_mma" if st["tile"] == 8 else "k_grid_fp32") + " (+ plane zeroing)"
+    return name, planes, grid_kernel_bytes(st["num_gridded"], planes, st["grid_size"], 32 if w_planes else 16)
 
 
 def batching_phase(api, local, n_snapshots=256, launches=3, seed_offset=0):
@@ -279,7 +291,7 @@ def batching_phase(api, local, n_snapshots=256, launches=3, seed_offset=0):
 def widefield_phase(api, local, npix=256):
     """Configuration W: the 512-station layout at 30 deg elevation, 64 channels, 4096^2 image over
     a 0.3 rad field. ES support W and the Chebyshev error target are swept; each point reports the
-    device time, the moment planes used and the relative RMS error of the rotated-frame image
+    device time, the planes used (w planes or moment planes) and the relative RMS error of the rotated-frame image
     against the library's FP64 direct DFT at random pixels."""
     import torch
     from svdimager_b200 import synth
@@ -309,9 +321,9 @@ def widefield_phase(api, local, npix=256):
                 e.image_device(d, N, cell, img.data_ptr())
                 ms.append(e.stats()["ms_total"])
                 ms_grid.append(e.stats()["ms_grid"])
-            st = e.stats()
+            st, wp = e.stats(), e.w_planes()
         return {"support": W, "cheb_target": tgt, "w_slabs": st["num_slabs"],
-                "chebyshev_terms": st["num_terms"], "planes": st["num_planes"],
+                "chebyshev_terms": st["num_terms"], "planes": wp or st["num_planes"], "w_planes": wp,
                 "ms": round(float(np.median(ms)), 3), "ms_gridding": round(float(np.median(ms_grid)), 3),
                 "tensor_core": bool(st["used_tc"]), "rel_rms_vs_fp64_dft": err}
 
@@ -437,7 +449,7 @@ def run_ours(args):
     for _ in range(args.warmup):
         step()
     torch.cuda.synchronize(dev)
-    st = eng.stats()
+    st, w_planes = eng.stats(), eng.w_planes()
     lat = []
     if dist:
         dist.barrier()
@@ -514,26 +526,23 @@ def run_ours(args):
         return
 
     G = st["grid_size"]
-    planes = st["num_planes"]
+    grid_name, planes, grid_bytes = gridding_stage(st, w_planes, args.gridder)
     peak, peak_kind = peaks()
     stage_ms = {k: float(np.median(v)) for k, v in stage.items()}
     # dominant kernel stage of ours (cuFFT is a library call and reported beside it)
     ours = {k: v for k, v in stage_ms.items() if k != "ms_fft"}
     dom = max(ours, key=ours.get)
     if dom == "ms_grid":
-        alg = grid_kernel_bytes(st["num_gridded"], planes, G)
-        fp32 = "k_grid_mma" if st["tile"] == 8 else "k_grid_fp32"
-        name = (("k_grid_i8" if args.gridder == "tc_i8" else "k_grid_tc") if st["used_tc"] else fp32) \
-            + " (+ plane zeroing)"
+        alg, name = grid_bytes, grid_name
     elif dom == "ms_bin":
-        alg = (26 + 8) * snap.num_samples + 16 * st["num_gridded"]
-        name = "k_histogram_sep + k_scan + k_scatter_sep"
+        alg = (26 + 8) * snap.num_samples + (32 if w_planes else 16) * st["num_gridded"]
+        name = "k_bin_w + k_scan" if w_planes else "k_histogram_sep + k_scan + k_scatter_sep"
     elif dom == "ms_preprocess":
         alg = 26 * snap.num_samples + 8 * snap.num_samples + 36 * snap.num_rows
         name = "k_collapse + rotation"
     else:
         alg = 8 * planes * N * N + 4 * N * N
-        name = "k_recombine"
+        name = "k_recombine_w" if w_planes else "k_recombine"
     achieved = alg / (stage_ms[dom] * 1e-3) / 1e9
     # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch of each gridder on
     # this workload, from one-launch ncu --set full captures (fourth imaging call of this bench with
@@ -560,8 +569,9 @@ def run_ours(args):
             "workload": f"{args.config}: {snap.num_rows} baselines x {snap.num_channels} channels = "
                         f"{snap.num_samples} vis, one snapshot, {N}^2 image, cell {cell} rad",
             "gridder": GRIDDER_LABEL[args.gridder] if st["used_tc"] else (
+                "fp32 w planes" if w_planes else
                 "fp32 matrix-instruction (FP16 hi+lo products, FP32 sums)" if st["tile"] == 8 else "fp32 fixed-point"),
-            "grid": G, "planes": planes, "num_slabs": st["num_slabs"], "chebyshev_terms": st["num_terms"],
+            "grid": G, "planes": planes, "w_planes": w_planes, "num_slabs": st["num_slabs"], "chebyshev_terms": st["num_terms"],
             "support": 8, "beta": 15.3704324328, "oversampling": 1.5, "tile": st["tile"],
             "k_rule": "target 1e-6", "edges": "strict (samples whose footprint leaves the grid are dropped)",
             "gridded_samples": st["num_gridded"],
@@ -585,8 +595,11 @@ def run_ours(args):
         "roofline": {"bound": "hbm", "kernel": name, "achieved": round(achieved, 1), "peak": peak,
                      "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": traffic,
                      "peak_kind": peak_kind,
-                     "limiter": ("warp-instruction issue: weights, FP16 splits and operand loads of 64 cells "
-                                 "per sample, its DRAM traffic is small" if dom == "ms_grid" else None),
+                     "limiter": (None if dom != "ms_grid" else
+                                 "warp-instruction issue where samples are dense, else the writes of the planes"
+                                 if w_planes else
+                                 "warp-instruction issue: weights, FP16 splits and operand loads of 64 cells "
+                                 "per sample, its DRAM traffic is small"),
                      "snapshot_alg_bytes": algorithmic_bytes(snap.num_samples, snap.num_rows,
                                                              snap.num_channels, planes, G, N),
                      "snapshot_frac": round(algorithmic_bytes(snap.num_samples, snap.num_rows,

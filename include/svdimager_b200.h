@@ -210,6 +210,9 @@ typedef struct svdi_stats {
 } svdi_stats;
 
 int svdi_engine_last_stats(const svdi_engine* e, svdi_stats* out);
+/* w planes that the last call gridded and transformed in place of svdi_stats' num_planes moment planes
+ * (SVDI_KRULE_TARGET, wide fields); 0: the moment planes. Negative: an error status. */
+int svdi_engine_w_planes(const svdi_engine* e);
 
 /* FP64 direct DFT of the engine's last snapshot at pixels (px[i], py[i]) of its N x N image:
  * |sum_k Re(V_k e^{2 pi i r_k . t})| / |det V| / N_s over the samples the gridder kept (the same

@@ -33,7 +33,7 @@ EXPORTED_SYMBOLS = (
     "svdi_last_error", "svdi_fipipe", "svdi_preprocess_measurement_set", "svdi_fipipe_device",
     "svdi_free_device_buffers", "svdi_default_options", "svdi_engine_create", "svdi_engine_destroy",
     "svdi_engine_image_host", "svdi_engine_image_device", "svdi_engine_fipipe_host",
-    "svdi_engine_last_stats", "svdi_engine_buffer_size", "svdi_engine_copy_buffer",
+    "svdi_engine_last_stats", "svdi_engine_w_planes", "svdi_engine_buffer_size", "svdi_engine_copy_buffer",
     "svdi_kernel_launch_count", "svdi_bin_samples_noalloc", "svdi_server_create",
     "svdi_server_submit", "svdi_server_wait", "svdi_server_poll", "svdi_server_stats",
     "svdi_server_destroy", "svdi_engine_dft_pixels", "svdi_batch_create", "svdi_batch_launch",
@@ -150,6 +150,7 @@ def lib():
         L.svdi_engine_image_device.argtypes = [P, ctypes.POINTER(HostMS), sz, f, P, P]
         L.svdi_engine_fipipe_host.argtypes = [P, P, P, P, P, P, sz, sz, f]
         L.svdi_engine_last_stats.argtypes = [P, ctypes.POINTER(Stats)]
+        L.svdi_engine_w_planes.argtypes = [P]
         L.svdi_engine_buffer_size.argtypes = [P, i, ctypes.POINTER(sz)]
         L.svdi_engine_copy_buffer.argtypes = [P, i, P, sz]
         L.svdi_kernel_launch_count.restype = ctypes.c_uint64
@@ -311,6 +312,12 @@ class Engine:
         s = Stats()
         _check(lib().svdi_engine_last_stats(self._h, ctypes.byref(s)))
         return s.as_dict()
+
+    def w_planes(self) -> int:
+        """w planes of the last call, 0 when it imaged through its num_planes moment planes."""
+        n = lib().svdi_engine_w_planes(self._h)
+        _check(max(0, -n))
+        return n
 
     def dft_pixels(self, px, py) -> np.ndarray:
         """FP64 direct DFT of the last snapshot at pixels (px, py): the rotated-frame image value

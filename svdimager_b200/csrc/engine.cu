@@ -247,6 +247,7 @@ struct svdi_engine {
     double last_cell = 0.0;
     bool have_last = false;
     bool last_w = false;       // it went through w planes: no records or moments of it are held yet
+    int w_planes = 0;          // w planes of the last call that was imaged, 0 when through moments
     svdi::DevBuf probe, remade;
     // pageable host uploads and image downloads of the archive entry and the host-input call
     svdi::HostStager stager;
@@ -1012,6 +1013,7 @@ int image_wplanes(svdi_engine* e, SampleSource src, const GridGeom& g, const Sla
     e->sz_off = (size_t)(sp.nslab * g.ntile * g.ntile2 + 1) * 4;
     e->sz_mom = plane_bytes * bslabs * (size_t)sp.K;
     e->last_w = true;
+    e->w_planes = wp.P;
     return SVDI_OK;
 }
 
@@ -1264,6 +1266,7 @@ int image_core(svdi_engine* e, bool archive, SampleSource src, long long N, floa
         e->spec_sp = sp;
     }
     record_call(e, src, g, sp, N, cell);
+    e->w_planes = 0;
     if (!timed) {
         if (d_status_out) {
             if (use_tc)
@@ -1705,16 +1708,27 @@ int svdi_engine_last_stats(const svdi_engine* e, svdi_stats* out) {
     return SVDI_OK;
 }
 
+int svdi_engine_w_planes(const svdi_engine* e) {
+    if (!e) {
+        set_error("null engine");
+        return -SVDI_ERR_INVALID_ARGUMENT;
+    }
+    std::lock_guard<std::mutex> lk(const_cast<svdi_engine*>(e)->mu);
+    return e->w_planes;
+}
+
 // The records and moment planes of a last call that went through w planes: its Chebyshev form, run again on
 // the inputs that are still resident (into a scratch image).
 static int materialise_moments(svdi_engine* e, int which) {
     if (!e->last_w || which < SVDI_BUF_OFFSETS || which == SVDI_BUF_GRID) return SVDI_OK;
     const svdi_stats kept = e->last;
+    const int w_planes = e->w_planes;
     const size_t N = (size_t)e->last_N;
     SVDI_TRY(e->remade.ensure(N * N * sizeof(float)));
     const int rc = image_core(e, false, e->last_src, (long long)N, (float)e->last_cell, e->remade.as<float>(), nullptr,
                               nullptr, nullptr, nullptr, false, false);
     e->spec_valid = false;  // the next call of this shape goes through w planes like the one before
+    e->w_planes = w_planes;
     SVDI_TRY(rc);
     SVDI_TRY(finish_pending(e));
     e->last = kept;

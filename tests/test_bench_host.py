@@ -13,6 +13,18 @@ def test_algorithmic_bytes_of_the_precision_snapshot():
     assert bench.grid_kernel_bytes(7_017_770, 1, G) == 16 * 7_017_770 + 8 * G * G == 187_781_792
 
 
+def test_gridding_stage_of_w_planes_and_moments():
+    """A call through w planes is credited with the planes it gridded and its 32-byte records, not with the moment
+    planes that its statistics report."""
+    st = dict(num_planes=236, num_gridded=5_147_224, grid_size=6144, tile=8, used_tc=0)
+    G2 = 6144 ** 2
+    assert bench.gridding_stage(st, 116, "fp32") == ("k_grid_w (+ split and rare samples)", 116,
+                                                     32 * 5_147_224 + 8 * 116 * G2)
+    assert bench.gridding_stage(st, 0, "fp32") == ("k_grid_mma (+ plane zeroing)", 236, 16 * 5_147_224 + 8 * 236 * G2)
+    assert bench.gridding_stage(dict(st, tile=32), 0, "fp32")[0] == "k_grid_fp32 (+ plane zeroing)"
+    assert bench.gridding_stage(dict(st, used_tc=1), 0, "tc_i8")[0] == "k_grid_i8 (+ plane zeroing)"
+
+
 def test_clock_record_summary(tmp_path):
     rows = [
         "0, 1965, 1965, 812.4, 0x0000000000000000, Not Active, Not Active, Not Active, Not Active",

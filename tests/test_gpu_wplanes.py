@@ -143,6 +143,24 @@ def test_reading_buffers_keeps_the_route(cuda_device):
             assert api.kernel_launch_count() - n0 != before
 
 
+def test_reports_its_planes(cuda_device):
+    """w_planes() is the number of planes of the last call, buffers read or not; 0 for the moments."""
+    s = _snap(256, 4, 3000)
+    with api.Engine(k_rule=api.KRULE_TARGET, target_error=1e-6, edge_mode=api.EDGE_STRICT) as e:
+        assert e.w_planes() == 0
+        e.image(s)
+        n, st = e.w_planes(), e.stats()
+        # W = 10 planes and one per 1 / (3 max|t3|) of |r3|
+        hi = max(abs(st["r3_min"]), abs(st["r3_max"]))
+        assert n == int(hi * 3.0 * st["max_abs_t3"] * (1 + 1e-12)) + 10 < st["num_planes"]
+        e.buffer(api.BUF_RECORDS)
+        assert e.w_planes() == n
+        e.image(snapshot("small"))
+        assert e.w_planes() == 0
+        e.image(s)
+        assert e.w_planes() == n
+
+
 def test_failed_call_after_w_planes(cuda_device):
     """A call that fails has overwritten the inputs that the last call's records and moments would be made from:
     there are none then, rather than some of other inputs, and the next call is as before."""
