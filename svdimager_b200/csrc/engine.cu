@@ -1001,7 +1001,9 @@ int image_wplanes(svdi_engine* e, SampleSource src, const GridGeom& g, const Sla
     e->pending_times = !multi;
     e->pending_stamps = false;
     if (multi) {
-        e->last.ms_bin = 0;
+        float mb = 0;
+        cudaEventElapsedTime(&mb, e->ev[1], e->ev[2]);
+        e->last.ms_bin = mb;
         e->last.ms_grid = ms[0];
         e->last.ms_fft = ms[1];
         e->last.ms_image = ms[2];

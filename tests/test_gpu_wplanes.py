@@ -161,6 +161,18 @@ def test_reports_its_planes(cuda_device):
         assert e.w_planes() == n
 
 
+@pytest.mark.parametrize("batch", [0, 1])
+def test_stage_times(cuda_device, batch):
+    """Every stage of a call through w planes has its time, with the planes in one batch or several."""
+    s = _snap(256, 4, 3000)
+    with api.Engine(k_rule=api.KRULE_TARGET, target_error=1e-6, edge_mode=api.EDGE_STRICT, max_batch_slabs=batch) as e:
+        e.image(s)
+        st = e.stats()
+        assert e.w_planes() > 0
+        stages = [st["ms_" + k] for k in ("preprocess", "bin", "grid", "fft", "image")]
+        assert min(stages) > 0 and sum(stages) <= st["ms_total"] * 1.01, (stages, st["ms_total"])
+
+
 def test_failed_call_after_w_planes(cuda_device):
     """A call that fails has overwritten the inputs that the last call's records and moments would be made from:
     there are none then, rather than some of other inputs, and the next call is as before."""
