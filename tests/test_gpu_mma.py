@@ -108,3 +108,41 @@ def test_dense_tile_rounding(cuda_device, calls):
     finally:
         for e in engines.values():
             e.close()
+
+
+@pytest.mark.parametrize("N,nslab", [(2048, 3), (2048, 2), (777, 3)])
+def test_distant_keys(cuda_device, N, nslab):
+    """A compact array in several w-slabs: a few tiles of each slab hold records, the keys between them (147,456 of
+    a 3072^2 grid per slab) are empty. The planes against those of 32 x 32 tiles, each within GRID_TOL of the exact
+    ones; and a slab more costs a slab's gridding, not a walk over its keys: nslab times that of one slab, and 0.1 ms
+    for launches and noise."""
+    import dataclasses
+    from tests.conftest import snapshot
+    s = snapshot("small", image_size=N, cell_size=0.1 / N)
+    uvw = s.uvw * np.float32(0.01)
+    uvw[:, 2] = np.random.default_rng(2).uniform(-0.2, 0.2, len(uvw)) * uvw[:, 0].std()  # records in every slab
+    s = dataclasses.replace(s, uvw=uvw)
+    opt = dict(k_rule=api.KRULE_FIXED, fixed_k=1)
+
+    def grid_ms(e):
+        ms = []
+        for _ in range(9):
+            e.image(s)
+            ms.append(e.stats()["ms_grid"])
+        return float(np.median(ms)), e.stats()
+
+    with api.Engine(**opt) as e:
+        one, st = grid_ms(e)
+        assert st["num_slabs"] == 1
+    opt["target_alpha"] = st["alpha_max"] / (nslab - 0.5)
+    with api.Engine(**opt) as e:
+        ms, st = grid_ms(e)
+        assert st["num_slabs"] == nslab and st["tile"] == 8
+    planes = []
+    for tile in (0, 32):
+        with api.Engine(keep_grid=1, tile=tile, **opt) as e:
+            e.image(s)
+            planes.append(e.buffer(api.BUF_GRID).reshape(nslab, -1))
+    for a, b in zip(*planes):
+        assert np.linalg.norm(a - b) <= 2 * GRID_TOL * np.linalg.norm(b) > 0
+    assert ms <= nslab * one + 0.1, (ms, one)
