@@ -214,7 +214,7 @@ int launch_histogram(const SampleSource& src, const GridGeom& g, const SlabParam
                      unsigned int* d_counts, int n_keys, unsigned long long* d_dropped,
                      cudaStream_t st, const DevPlan* d_plan = nullptr);
 // d_kb_offsets (optional): exclusive scan of ceil(count / kb_size) per key, n_keys + 1 entries.
-// d_chunk_key (optional): for every chunk c of chunk_size records, the last key whose records
+// d_chunk_key (optional): for every chunk c of chunk_size records (a power of two), the last key whose records
 // start at or before c * chunk_size (ceil(total / chunk_size) entries, total = offsets[n_keys]).
 // d_sums (optional, scan_sums_words(n_keys) words of scratch): lets several blocks scan a large
 // number of keys; without it one block scans them all.
