@@ -368,18 +368,48 @@ __device__ inline void unit_of(long long u, const SepMap& m, int& rt, int& ch) {
     ch = (int)(u - (long long)rt * m.nch);
 }
 
-// Runs of equal keys on consecutive lanes (consecutive channels of one baseline mostly stay in a tile, and a key
-// that comes again later is another run): the first lane of this lane's run and the run's length. One shuffle
-// and one vote; a match over the warp costs several times that on the unit the atomics share.
-__device__ __forceinline__ void lane_run(int key, int lane, int& first, int& length) {
-    const int before = __shfl_up_sync(0xffffffffu, key, 1);
-    const unsigned int starts = __ballot_sync(0xffffffffu, lane == 0 || key != before);
-    first = 31 - __clz(starts & (0xffffffffu >> (31 - lane)));
-    const unsigned int after = starts & ~(0xffffffffu >> (31 - lane));
-    length = (after ? __ffs(after) - 1 : 32) - first;
-}
+// The lanes of a warp that place their records together. Runs of equal keys on consecutive lanes: consecutive
+// channels of one baseline mostly stay in a tile and do not come back to one. One shuffle and one vote; a match over
+// the warp costs several times that on the unit the atomics share (8.4 M samples of 64 channels: 195 instead of 185
+// us).
+template <bool ROWS>
+struct LaneGroup {
+    int first = 0, length = 0;
+    __device__ __forceinline__ void find(int key, int lane) {
+        const int before = __shfl_up_sync(0xffffffffu, key, 1);
+        const unsigned int starts = __ballot_sync(0xffffffffu, lane == 0 || key != before);
+        first = 31 - __clz(starts & (0xffffffffu >> (31 - lane)));
+        const unsigned int after = starts & ~(0xffffffffu >> (31 - lane));
+        length = (after ? __ffs(after) - 1 : 32) - first;
+    }
+    __device__ __forceinline__ int leader() const { return first; }
+    __device__ __forceinline__ unsigned int count() const { return (unsigned int)length; }
+    __device__ __forceinline__ unsigned int rank(int lane) const { return (unsigned int)(lane - first); }
+    __device__ __forceinline__ unsigned int lanes() const { return (0xffffffffu >> (32 - length)) << first; }
+};
+// Several rows per warp (fewer than 17 channels): keys may repeat apart, as in the few tiles of a compact array, where
+// each sample was an atomic of its own on one address (2 M samples of one channel in four tiles: binning 1.37 ms, with
+// the match 0.17; spread over the grid 127 and 134 us). So many runs are matched.
+template <>
+struct LaneGroup<true> {
+    unsigned int mask = 1;
+    __device__ __forceinline__ void find(int key, int lane) {
+        const int before = __shfl_up_sync(0xffffffffu, key, 1);
+        const unsigned int starts = __ballot_sync(0xffffffffu, lane == 0 || key != before);
+        if (__popc(starts) > 8) {
+            mask = __match_any_sync(0xffffffffu, key);
+            return;
+        }
+        const unsigned int upto = 0xffffffffu >> (31 - lane), after = starts & ~upto;
+        mask = (after ? (after & (0u - after)) - 1u : 0xffffffffu) & (0xffffffffu << (31 - __clz(starts & upto)));
+    }
+    __device__ __forceinline__ int leader() const { return __ffs(mask) - 1; }
+    __device__ __forceinline__ unsigned int count() const { return (unsigned int)__popc(mask); }
+    __device__ __forceinline__ unsigned int rank(int lane) const { return (unsigned int)__popc(mask & ((1u << lane) - 1u)); }
+    __device__ __forceinline__ unsigned int lanes() const { return mask; }
+};
 
-template <int UR>
+template <int UR, bool ROWS>
 __global__ void __launch_bounds__(kThreads) k_histogram_sep(SampleSource src, SepMap m, GridGeom g, SlabParams sp,
                                                            unsigned int* __restrict__ counts, int n_keys,
                                                            unsigned long long* __restrict__ dropped,
@@ -407,7 +437,7 @@ __global__ void __launch_bounds__(kThreads) k_histogram_sep(SampleSource src, Se
         const int c = ch * m.lpr + coff;
         const bool cvalid = c < m.C;
         const double sc = cvalid ? src.s[c] : 0.0;
-        // every lane takes every step (the match needs the whole warp); rows past the unit have no key
+        // every lane takes every step (the votes need the whole warp); rows past the unit have no key
         for (int i0 = 0; i0 < UR; i0 += rps) {
             const int i = i0 + sub;
             const long long row = (long long)rt * UR + i;
@@ -417,11 +447,11 @@ __global__ void __launch_bounds__(kThreads) k_histogram_sep(SampleSource src, Se
                 key = row_chan_key(sc, q[0], q[1], q[2], g, sp).key;
                 if (key < 0) ++ndrop;
             }
-            int first, length;
-            lane_run(key, lane, first, length);
-            if (key >= 0 && lane == first) {
-                if (use_smem) atomicAdd(&sh[key], (unsigned int)length);
-                else atomicAdd(&counts[key], (unsigned int)length);
+            LaneGroup<ROWS> group;
+            group.find(key, lane);
+            if (key >= 0 && lane == group.leader()) {
+                if (use_smem) atomicAdd(&sh[key], group.count());
+                else atomicAdd(&counts[key], group.count());
             }
         }
     }
@@ -437,7 +467,7 @@ __global__ void __launch_bounds__(kThreads) k_histogram_sep(SampleSource src, Se
 // Scatter for separable sources: per unit, the warp stages the unit's collapsed visibilities in
 // shared memory with row-contiguous loads, then writes each group's records to the slots one
 // global atomic on the key's cursor reserved.
-template <int UR>
+template <int UR, bool ROWS>
 __global__ void __launch_bounds__(kThreads, 4) k_scatter_sep(SampleSource src, SepMap m, GridGeom g, SlabParams sp,
                                                          unsigned int* __restrict__ cursor,
                                                          SampleRec* __restrict__ rec, float* __restrict__ rec_s,
@@ -483,13 +513,14 @@ __global__ void __launch_bounds__(kThreads, 4) k_scatter_sep(SampleSource src, S
         // latency of its cursor atomic is covered
         KeyRec last;
         last.key = -1;
-        int last_i = 0, last_first = 0, last_len = 0;
+        LaneGroup<ROWS> last_group;
+        int last_i = 0;
         unsigned int last_base = 0;
         for (int i0 = 0; i0 < UR + rps; i0 += rps) {
             KeyRec kr;
             kr.key = -2;
             const int i = i0 + sub;
-            int first = 0, length = 0;
+            LaneGroup<ROWS> group;
             unsigned int base = 0;
             if (i0 < UR) {
                 const long long row = row0 + i;
@@ -497,13 +528,13 @@ __global__ void __launch_bounds__(kThreads, 4) k_scatter_sep(SampleSource src, S
                     const double* q = src.q + row * 3;
                     kr = row_chan_key(sc, q[0], q[1], q[2], g, sp);
                 }
-                lane_run(kr.key, lane, first, length);
-                if (kr.key >= 0 && lane == first) base = atomicAdd(&cursor[kr.key], (unsigned int)length);
+                group.find(kr.key, lane);
+                if (kr.key >= 0 && lane == group.leader()) base = atomicAdd(&cursor[kr.key], group.count());
             }
             if (i0 > 0) {
-                const unsigned int b0 = __shfl_sync(0xffffffffu, last_base, last_first);
+                const unsigned int b0 = __shfl_sync(0xffffffffu, last_base, last_group.leader());
                 if (last.key >= 0) {
-                    const unsigned int pos = b0 + (unsigned int)(lane - last_first);
+                    const unsigned int pos = b0 + last_group.rank(lane);
                     const float2 v = my[coff * kVisPitch + last_i];
                     SampleRec r;
                     r.xq = last.xq;
@@ -515,17 +546,15 @@ __global__ void __launch_bounds__(kThreads, 4) k_scatter_sep(SampleSource src, S
                     nbad += nonfinite2(r.vre, r.vim);
                     const float m = fmaxf(fabsf(r.vre), fabsf(r.vim));
                     vm = fmaxf(vm, m);
-                    if (keymax) {  // the run's maximum, one atomic per run
-                        const unsigned int run = (0xffffffffu >> (32 - last_len)) << last_first;
-                        const unsigned int gm = __reduce_max_sync(run, __float_as_uint(m));
-                        if (lane == last_first && gm) atomicMax(&keymax[last.key], gm);
+                    if (keymax) {  // the group's maximum, one atomic per group
+                        const unsigned int gm = __reduce_max_sync(last_group.lanes(), __float_as_uint(m));
+                        if (lane == last_group.leader() && gm) atomicMax(&keymax[last.key], gm);
                     }
                 }
             }
             last = kr;
             last_i = i;
-            last_first = first;
-            last_len = length;
+            last_group = group;
             last_base = base;
         }
     }
@@ -566,9 +595,10 @@ int launch_histogram(const SampleSource& src, const GridGeom& g, const SlabParam
     const size_t smem = n_keys <= kSmemKeyLimit ? (size_t)n_keys * 4 : 0;
     if (use_sep(src)) {
         const int ur = unit_rows(src);
-        auto kern = ur == kUnitRows ? k_histogram_sep<kUnitRows> : k_histogram_sep<kUnitRowsSmall>;
-        SVDI_TRY(ensure_dynamic_smem((const void*)kern, smem));
         const SepMap m = sep_map(src, ur);
+        auto kern = m.lpr < 32 ? (ur == kUnitRows ? k_histogram_sep<kUnitRows, true> : k_histogram_sep<kUnitRowsSmall, true>)
+                               : (ur == kUnitRows ? k_histogram_sep<kUnitRows, false> : k_histogram_sep<kUnitRowsSmall, false>);
+        SVDI_TRY(ensure_dynamic_smem((const void*)kern, smem));
         const long long units = (long long)m.nrt * m.nch;
         long long blocks = (units + kThreads / 32 - 1) / (kThreads / 32);
         if (blocks > 4LL * current_sm_count()) blocks = 4LL * current_sm_count();   // a few units per warp: the shared histogram is flushed once
@@ -610,8 +640,9 @@ int launch_scatter(const SampleSource& src, const GridGeom& g, const SlabParams&
                    unsigned int* d_vmax, cudaStream_t st, unsigned int* d_keymax, const DevPlan* d_plan) {
     if (use_sep(src)) {
         const int ur = unit_rows(src);
-        auto kern = ur == kUnitRows ? k_scatter_sep<kUnitRows> : k_scatter_sep<kUnitRowsSmall>;
         const SepMap m = sep_map(src, ur);
+        auto kern = m.lpr < 32 ? (ur == kUnitRows ? k_scatter_sep<kUnitRows, true> : k_scatter_sep<kUnitRowsSmall, true>)
+                               : (ur == kUnitRows ? k_scatter_sep<kUnitRows, false> : k_scatter_sep<kUnitRowsSmall, false>);
         const long long units = (long long)m.nrt * m.nch;
         long long blocks = (units + kThreads / 32 - 1) / (kThreads / 32);
         if (blocks > 8LL * current_sm_count()) blocks = 8LL * current_sm_count();

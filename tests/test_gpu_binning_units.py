@@ -65,3 +65,43 @@ def test_dense_core_binning_time(cuda_device):
         spread = bin_ms(e, s)
         dense = bin_ms(e, dataclasses.replace(s, uvw=s.uvw * np.float32(1e-3)))
     assert dense <= 2 * spread, (dense, spread)
+
+
+@pytest.mark.parametrize("nchan,rows", [(1, 8128), (2, 8001), (3, 5000), (16, 1000), (17, 1000)])
+@pytest.mark.parametrize("scale", [1e-3, 0.02])
+def test_compact_array_bit_exact(cuda_device, nchan, rows, scale):
+    """Rows of a warp that share a tile without being neighbours, for one to all of a warp's lanes per row."""
+    import dataclasses
+    import numpy as np
+    s = snapshot("small", nchan=nchan, n_rows_limit=rows, image_size=256, cell_size=0.1 / 256)
+    s = dataclasses.replace(s, uvw=s.uvw * np.float32(scale))
+    with api.Engine() as e:
+        for _ in range(2):
+            e.image(s)
+        r = O.expand_coords(e.buffer(api.BUF_Q).reshape(-1, 3), e.buffer(api.BUF_S))
+        _check_binning(e, e.stats(), r, e.buffer(api.BUF_VIS_REAL), e.buffer(api.BUF_VIS_IMAG), s.cell_size, edge_mode=0)
+
+
+def test_few_channels_binning_time(cuda_device):
+    """1 M samples of one channel, all in a few tiles, are binned in at most 1.5 times what they take spread over
+    the grid (3 times where each sample is an atomic of its own on one address)."""
+    import dataclasses
+    import numpy as np
+    s = snapshot("precision", nchan=1, image_size=512, cell_size=0.1 / 512)
+    rng = np.random.default_rng(1)
+    uvw = np.concatenate([s.uvw] * 8) * rng.uniform(0.9, 1.0, (8 * s.num_rows, 1)).astype(np.float32)
+    many = {k: np.concatenate([v] * 8) for k, v in s.arrays().items() if k not in ("uvw", "frequencies_hz")}
+    s = dataclasses.replace(s, num_rows=len(uvw), uvw=uvw, **many)
+
+    def bin_ms(e, s):
+        ms = []
+        for _ in range(9):
+            e.image(s)
+            ms.append(e.stats()["ms_bin"])
+        return float(np.median(ms))
+
+    limit = 0.45 * 512 / 0.1 / (170e6 / 299792458.0)  # the longest baseline inside the grid
+    spread = dataclasses.replace(s, uvw=s.uvw * np.float32(limit / np.abs(uvw).max()))
+    with api.Engine(k_rule=api.KRULE_FIXED, fixed_k=1) as e:
+        wide, dense = bin_ms(e, spread), bin_ms(e, dataclasses.replace(spread, uvw=spread.uvw * np.float32(5e-3)))
+    assert dense <= 1.5 * wide, (dense, wide)
