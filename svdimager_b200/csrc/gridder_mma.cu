@@ -22,7 +22,7 @@
 // single warps from a counter; a batch of 32 records is staged lane-per-record (36 + 36 FMAs for the 16
 // taps: the even and odd parts of a piece's polynomial also give the mirrored piece), then 16-record
 // steps run for every tile segment the batch holds. Footprints that W x W taps cannot hold (exactly
-// integer positions, W + 1 cells; clipped at the low grid edge) go straight to the plane.
+// integer positions, W + 1 cells; clipped at the low grid edge) go straight to the plane, after the chunk's end.
 //
 // A tile's region and its right neighbour's share eight columns: a warp that moves on to that
 // neighbour (the next key) keeps them in its registers and reduces only the left half.
@@ -155,10 +155,11 @@ struct DenseSlots {
 constexpr int kSlotWords = 128;  // 16-byte words per slot: 16 x 16 complex cells
 
 template <int KC>
-struct WarpStage {
+struct alignas(16) WarpStage {  // one after another in shared memory, read 8 bytes at a time
     unsigned int a[KC][8 * kPitch];      // [term][row residue][record]: T_n(s) times the row weight
     unsigned int b[16 * kPitch];         // [b_row(column residue) + (re, im)][record]: column weight times v
     __half oa[32], ob[32];               // footprint origins (row, column) in the region
+    unsigned int rare;                   // batches of the chunk (8 at most) with rare records
 };
 
 // Column residues 0, 2, 4, 6 and then 1, 3, 5, 7, real and imaginary rows each: fragment tile (half,
@@ -236,13 +237,11 @@ __device__ __forceinline__ void products(const WarpStage<KC>& st, int k0, int k1
                                          __half2 row_res, __half2 res0, __half2 res1, unsigned int odd, float inv,
                                          float (&acc)[KC][4][4]) {
     BFrag b[NW];
-    unsigned int m0[NW], m1[NW];
 #pragma unroll
     for (int w = 0; w < NW; ++w) {
         const int k = w ? k1 : k0;
+        asm volatile("" ::: "memory");  // one window's loads after the other's: registers are short
         load_b(st, k, w ? k0 + 16 : lo, hi, gr, tq, res0, res1, odd, b[w]);
-        m0[w] = __hge2_mask(row_res, *reinterpret_cast<const __half2*>(&st.oa[k + 2 * tq]));
-        m1[w] = __hge2_mask(row_res, *reinterpret_cast<const __half2*>(&st.oa[k + 2 * tq + 8]));
     }
 #pragma unroll
     for (int t = 0; t < KC; ++t) {
@@ -254,7 +253,9 @@ __device__ __forceinline__ void products(const WarpStage<KC>& st, int k0, int k1
 #pragma unroll
         for (int w = 0; w < NW; ++w) {
             unsigned int ahi[4], alo[4];
-            load_a(st, t, w ? k1 : k0, gr, tq, m0[w], m1[w], ahi, alo);
+            const int k = (w ? k1 : k0) + 2 * tq;
+            load_a(st, t, w ? k1 : k0, gr, tq, __hge2_mask(row_res, *reinterpret_cast<const __half2*>(&st.oa[k])),
+                   __hge2_mask(row_res, *reinterpret_cast<const __half2*>(&st.oa[k + 8])), ahi, alo);
 #pragma unroll
             for (int j = 0; j < 4; ++j) mma_f16(c[j], alo, b[w].h[j][0], b[w].h[j][1]);
 #pragma unroll
@@ -305,6 +306,85 @@ __device__ __forceinline__ void products8(const WarpStage<KC>& st, int k0, int l
     }
 }
 
+// A record whose footprint W x W taps cannot hold: exactly integer positions (W + 1 cells), or clipped at the low
+// grid edge.
+template <int W>
+__device__ __forceinline__ bool is_rare(const SampleRec& r) {
+    return (r.xq & 0xFFFFFF) == 0 || (r.yq & 0xFFFFFF) == 0 || (r.xq >> 24) < W / 2 - 1 || (r.yq >> 24) < W / 2 - 1;
+}
+
+// The rare records of the batch [b0, b1), whose keys are `key` or later (returns the last one): exact ES formula,
+// lanes over cells, straight to the planes. Records at one position are summed first: autocorrelations and
+// baselines without coordinates all lie at the origin, where one after another they took 2 us each of their warp, on
+// the same 81 cells (2.1 M samples of 512 stations and their autocorrelations, 2 / 8 terms, 1024^2 image: call 812 /
+// 1250 -> 439 / 731 us). Run when the chunk's sums are out of the registers; in the segment loop it takes as many.
+template <int W, int KC>
+__device__ __forceinline__ int rare_records(const SampleRec* __restrict__ rec, const float* __restrict__ rec_s,
+                                            const unsigned int* __restrict__ offsets, unsigned int b0, unsigned int b1,
+                                            int key, int key_lo, int key_hi, int G, const FastDiv& by_slab,
+                                            const FastDiv& by_row, int K, float beta, float2* __restrict__ planes,
+                                            int term0) {
+    constexpr int HW = W / 2;
+    const int lane = threadIdx.x & 31;
+    const unsigned int mine = min(b0 + lane, b1 - 1);
+    const SampleRec own = rec[mine];
+    const float own_s = rec_s ? rec_s[mine] : 0.0f;
+    unsigned int rm = __ballot_sync(0xffffffffu, b0 + lane < b1 && is_rare<W>(own));
+    const long long GG = (long long)G * G;
+    while (rm) {
+        const int js = __ffs(rm) - 1;
+        const unsigned int p = b0 + js;
+        unsigned int ends;  // the window of 32 keys from `key`
+        while (!(ends = __ballot_sync(0xffffffffu, offsets[min(key + 1 + lane, key_hi)] > p))) {
+            key += 32;
+            ends = __ballot_sync(0xffffffffu, offsets[min(key + 32 * (lane + 1) * (lane + 1), key_hi)] > p);
+            const int f = __clz(__brev(ends));
+            key += 32 * f * f;
+        }
+        key += __ffs(ends) - 1;
+        const int n = key - key_lo, slab = div_by(n, by_slab), rem = n - slab * (int)by_slab.d;
+        const int t1 = div_by(rem, by_row), t2 = rem - t1 * (int)by_row.d;
+        float2* const plane = planes + ((long long)slab * K + term0) * GG;
+        const int xq = __shfl_sync(0xffffffffu, own.xq, js), yq = __shfl_sync(0xffffffffu, own.yq, js);
+        const float s = __shfl_sync(0xffffffffu, own_s, js);
+        const bool same = lane == js || ((rm >> lane & 1u) && own.xq == xq && own.yq == yq && own_s == s &&
+                                         b0 + lane < offsets[key + 1]);
+        rm &= ~__ballot_sync(0xffffffffu, same);
+        float vre = same ? own.vre : 0.0f, vim = same ? own.vim : 0.0f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            vre += __shfl_xor_sync(0xffffffffu, vre, o);
+            vim += __shfl_xor_sync(0xffffffffu, vim, o);
+        }
+        const int rcx = xq >> 24, rcy = yq >> 24, rfx = xq & 0xFFFFFF, rfy = yq & 0xFFFFFF;
+        const int lo_r = rfx ? rcx - (HW - 1) : rcx - HW, nr = rfx ? W : W + 1;
+        const int lo_c = rfy ? rcy - (HW - 1) : rcy - HW, nc = rfy ? W : W + 1;
+        const float px = (float)rfx * (1.0f / 16777216.0f), py = (float)rfy * (1.0f / 16777216.0f);
+        for (int c = lane; c < nr * nc; c += 32) {
+            const int i = c / nc, jj = c - i * nc;
+            const int row = t1 * kMmaTile + lo_r + i, col = t2 * kMmaTile + lo_c + jj;
+            if (row < 0 || col < 0 || row >= G || col >= G) continue;
+            const float x = ((float)(lo_r + i - rcx) - px) / (float)HW;
+            const float y = ((float)(lo_c + jj - rcy) - py) / (float)HW;
+            const float kv = es_exact(beta, x) * es_exact(beta, y) * (((row + col) & 1) ? -1.0f : 1.0f);
+            float2* d = plane + (long long)row * G + col;
+            float tm2 = 1.0f, tm1 = s;
+            for (int t = 0; t < term0; ++t) {
+                const float tt = 2.0f * s * tm1 - tm2;
+                tm2 = tm1;
+                tm1 = tt;
+            }
+            for (int t = 0; t < KC; ++t) {
+                red_add_v2(d + t * GG, kv * tm2 * vre, kv * tm2 * vim);
+                const float tt = 2.0f * s * tm1 - tm2;
+                tm2 = tm1;
+                tm1 = tt;
+            }
+        }
+    }
+    return key;
+}
+
 template <int W, int KC>
 __global__ void __launch_bounds__(32 * kWarps, min_ctas<KC>()) k_grid_mma(
     const SampleRec* __restrict__ rec, const float* __restrict__ rec_s, const unsigned int* __restrict__ offsets,
@@ -327,14 +407,6 @@ __global__ void __launch_bounds__(32 * kWarps, min_ctas<KC>()) k_grid_mma(
     const unsigned int ch_lo = rec_lo / chunk, n_ch = (rec_hi + chunk - 1) / chunk - ch_lo;
     const unsigned int n_work = n_ch * (unsigned int)groups;
 
-    float acc[KC][4][4];
-#pragma unroll
-    for (int t = 0; t < KC; ++t)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) acc[t][j][q] = 0.0f;
-
     // the chunk of work item i: the chunks are taken from both ends inwards, since the grid's outer
     // tiles hold few records each and take the longest per chunk
     auto chunk_of = [&](unsigned int i) {
@@ -342,7 +414,10 @@ __global__ void __launch_bounds__(32 * kWarps, min_ctas<KC>()) k_grid_mma(
         return ch_lo + ((ci & 1) ? n_ch - 1 - (ci >> 1) : (ci >> 1));
     };
     unsigned int item = 0, next = 0;
-    if (lane == 0) item = atomicAdd(work, 1u);
+    if (lane == 0) {
+        st.rare = 0u;
+        item = atomicAdd(work, 1u);
+    }
     item = __shfl_sync(0xffffffffu, item, 0);
     if (item >= n_work) return;
     unsigned int ch = chunk_of(item);
@@ -360,6 +435,13 @@ __global__ void __launch_bounds__(32 * kWarps, min_ctas<KC>()) k_grid_mma(
     }
     for (;;) {
         if (lane == 0) next = atomicAdd(work, 1u);  // its latency hides behind this chunk
+        float acc[KC][4][4];
+#pragma unroll
+        for (int t = 0; t < KC; ++t)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[t][j][q] = 0.0f;
         const int term0 = term_lo + (int)(item % (unsigned int)groups) * KC;
         const bool need_s = !(KC == 1 && term0 == 0);
         const unsigned int c_beg = max(rec_lo, ch * (unsigned int)chunk);
@@ -438,7 +520,7 @@ __global__ void __launch_bounds__(32 * kWarps, min_ctas<KC>()) k_grid_mma(
             const bool valid = b0 + lane < b1;
             const int fxq = r.xq & 0xFFFFFF, fyq = r.yq & 0xFFFFFF;
             const int r0 = (r.xq >> 24) - (HW - 1), c0 = (r.yq >> 24) - (HW - 1);
-            const bool rare = valid && (fxq == 0 || fyq == 0 || r0 < 0 || c0 < 0);
+            const bool rare = valid && is_rare<W>(r);
             const bool fast = valid && !rare;
             const unsigned int vbits =
                 fast ? (__float_as_uint(fmaxf(fabsf(r.vre), fabsf(r.vim))) & 0x7fffffffu) : 0u;
@@ -448,7 +530,7 @@ __global__ void __launch_bounds__(32 * kWarps, min_ctas<KC>()) k_grid_mma(
             const float scale = fast ? __int_as_float((se + 127) << 23) : 0.0f;
             // (1 + 2^-23) 2^-(14 + se): the last bit makes up for the products' truncation towards zero
             const float inv = __uint_as_float(((unsigned int)(127 - 14 - se) << 23) | 1u | neg);
-            const unsigned int rare_mask = __ballot_sync(0xffffffffu, rare);
+            if (rare) atomicOr(&st.rare, 1u << ((b0 - c_beg) / 32));
             if (vmax) {
                 const int oa = fast ? r0 : 0, ob = fast ? c0 : 0;
                 st.oa[lane] = __int2half_rn(oa);
@@ -555,40 +637,6 @@ __global__ void __launch_bounds__(32 * kWarps, min_ctas<KC>()) k_grid_mma(
                     else
                         products<2, KC>(st, k0, 16, lo, hi, gr, tq, row_res, res0, res1, odd, inv, acc);
                 }
-                // ---- rare records of the segment: exact ES formula, lanes over cells, straight to the plane
-                const unsigned int seg = (hi >= 32 ? 0xffffffffu : (1u << hi) - 1u) & ~((1u << lo) - 1u);
-                unsigned int rm = rare_mask & seg;
-                while (rm) {
-                    const int js = __ffs(rm) - 1;
-                    rm &= rm - 1;
-                    const SampleRec q = rec[b0 + js];
-                    const float s = need_s ? rec_s[b0 + js] : 0.0f;
-                    const int rcx = q.xq >> 24, rcy = q.yq >> 24, rfx = q.xq & 0xFFFFFF, rfy = q.yq & 0xFFFFFF;
-                    const int lo_r = rfx ? rcx - (HW - 1) : rcx - HW, nr = rfx ? W : W + 1;
-                    const int lo_c = rfy ? rcy - (HW - 1) : rcy - HW, nc = rfy ? W : W + 1;
-                    const float px = (float)rfx * (1.0f / 16777216.0f), py = (float)rfy * (1.0f / 16777216.0f);
-                    for (int c = lane; c < nr * nc; c += 32) {
-                        const int i = c / nc, jj = c - i * nc;
-                        const int row = t1 * kMmaTile + lo_r + i, col = t2 * kMmaTile + lo_c + jj;
-                        if (row < 0 || col < 0 || row >= G || col >= G) continue;
-                        const float x = ((float)(lo_r + i - rcx) - px) / (float)HW;
-                        const float y = ((float)(lo_c + jj - rcy) - py) / (float)HW;
-                        const float kv = es_exact(poly.beta, x) * es_exact(poly.beta, y) * (((row + col) & 1) ? -1.0f : 1.0f);
-                        float2* d = plane + (long long)row * G + col;
-                        float tm2 = 1.0f, tm1 = s;
-                        for (int t = 0; t < term0; ++t) {
-                            const float tt = 2.0f * s * tm1 - tm2;
-                            tm2 = tm1;
-                            tm1 = tt;
-                        }
-                        for (int t = 0; t < KC; ++t) {
-                            red_add_v2(d + t * ((long long)G * G), kv * tm2 * q.vre, kv * tm2 * q.vim);
-                            const float tt = 2.0f * s * tm1 - tm2;
-                            tm2 = tm1;
-                            tm1 = tt;
-                        }
-                    }
-                }
             }
             __syncwarp();
         }
@@ -627,6 +675,18 @@ __global__ void __launch_bounds__(32 * kWarps, min_ctas<KC>()) k_grid_mma(
                 }
         }
         if (to_plane) move_to(-1, min(kend, c_end) - kbeg);
+        unsigned int rare_batches = st.rare;
+        if (rare_batches) {
+            int rk = max(key_lo, (int)chunk_key[ch]);
+            __syncwarp();
+            if (lane == 0) st.rare = 0u;
+            __syncwarp();
+            for (; rare_batches; rare_batches &= rare_batches - 1) {
+                const unsigned int b0 = c_beg + 32 * (__ffs(rare_batches) - 1);
+                rk = rare_records<W, KC>(rec, need_s ? rec_s : nullptr, offsets, b0, min(b0 + 32u, c_end), rk, key_lo, key_hi,
+                                         G, by_slab, by_row, K, poly.beta, planes, term0);
+            }
+        }
         if (next >= n_work) break;
         item = next;
         ch = nch;

@@ -146,3 +146,53 @@ def test_distant_keys(cuda_device, N, nslab):
     for a, b in zip(*planes):
         assert np.linalg.norm(a - b) <= 2 * GRID_TOL * np.linalg.norm(b) > 0
     assert ms <= nslab * one + 0.1, (ms, one)
+
+
+@pytest.mark.parametrize("n,N,W,K", [(70, 48, 8, 1), (5000, 48, 8, 2), (5000, 61, 6, 3), (40_000, 64, 8, 8)])
+def test_samples_at_one_position(cuda_device, n, N, W, K):
+    """Many samples at the origin, among others on exact cells at the same place of neighbouring tiles and on the low
+    edge, in every batch and with different w: summed where position, tile and w agree."""
+    cell, G = 2e-3, (3 * N + 1) // 2
+    scale = float(np.float32(cell)) * G
+    rng = np.random.default_rng(n + K)
+    p = rng.uniform(-1.0, 1.0, (n, 2)) * 14.0
+    p[rng.random(n) < 0.5] = 0.0
+    other = rng.random(n) < 0.2
+    p[other] = 8.0 * rng.integers(-2, 3, (int(other.sum()), 2))
+    low = rng.random(n) < 0.05
+    p[low] = -(G // 2) + rng.integers(0, 3, (int(low.sum()), 2)) + 0.25
+    w = np.where(rng.random(n) < 0.7, 0.0, rng.choice([-30.0, 12.5, 40.0], n))
+    b = np.concatenate([p / scale, w[:, None]], axis=1).astype(np.float32)
+    vr, vi = (rng.normal(size=n).astype(np.float32) for _ in range(2))
+    opt = dict(coord_mode=api.COORD_REF32, keep_grid=1, k_rule=api.KRULE_FIXED, fixed_k=K, support=W, beta=W_BETA[W])
+    with api.Engine(api.archive_options(**opt)) as e:
+        e.fipipe(vr, vi, b, np.eye(3, dtype=np.float32), N, cell)
+        st = e.stats()
+        grid = e.buffer(api.BUF_GRID).reshape(K, G, G)
+    sc = O.SlabConfig(st["slab_r3_min"], st["r3_max"], st["max_abs_t3"], st["alpha_max"], 1, st["slab_width"],
+                      st["slab_half"], 1.0 / st["slab_half"], st["slab_alpha_max"], K)
+    ref = O.grid(b.astype(np.float64), vr, vi, scale, G, sc, 1.0, W=W, beta=W_BETA[W], coord_mode=1)
+    for k in range(K):
+        assert np.linalg.norm(grid[k] - ref[k]) <= GRID_TOL * np.linalg.norm(ref[k]), k
+
+
+@pytest.mark.parametrize("K", [1, 2, 8])
+def test_autocorrelations_time(cuda_device, K):
+    """A few per cent of autocorrelations (u = v = w = 0) cost a few per cent, not a chain of reductions on the origin's
+    cells: twice the gridding and 0.02 ms are allowed (one after another: 3 to 7 times)."""
+    import dataclasses
+    from tests.conftest import snapshot
+    s = snapshot("small", image_size=256, cell_size=0.1 / 256)
+    uvw = s.uvw.copy()
+    uvw[::32] = 0.0
+
+    def grid_ms(e, s):
+        ms = []
+        for _ in range(9):
+            e.image(s)
+            ms.append(e.stats()["ms_grid"])
+        return float(np.median(ms))
+
+    with api.Engine(k_rule=api.KRULE_FIXED, fixed_k=K) as e:
+        plain, autos = grid_ms(e, s), grid_ms(e, dataclasses.replace(s, uvw=uvw))
+    assert autos <= 2 * plain + 0.02, (autos, plain)
