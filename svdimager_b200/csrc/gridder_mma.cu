@@ -159,7 +159,7 @@ struct alignas(16) WarpStage {  // one after another in shared memory, read 8 by
     unsigned int a[KC][8 * kPitch];      // [term][row residue][record]: T_n(s) times the row weight
     unsigned int b[16 * kPitch];         // [b_row(column residue) + (re, im)][record]: column weight times v
     __half oa[32], ob[32];               // footprint origins (row, column) in the region
-    unsigned int rare;                   // batches of the chunk (8 at most) with rare records
+    unsigned int rare;                   // batches of the chunk (8 at most) with rare records (rare_records)
 };
 
 // Column residues 0, 2, 4, 6 and then 1, 3, 5, 7, real and imaginary rows each: fragment tile (half,
@@ -309,9 +309,18 @@ __device__ __forceinline__ void products8(const WarpStage<KC>& st, int k0, int l
 // A record whose footprint W x W taps cannot hold: exactly integer positions (W + 1 cells), or clipped at the low
 // grid edge.
 template <int W>
-__device__ __forceinline__ bool is_rare(const SampleRec& r) {
+__device__ __forceinline__ bool odd_footprint(const SampleRec& r) {
     return (r.xq & 0xFFFFFF) == 0 || (r.yq & 0xFFFFFF) == 0 || (r.xq >> 24) < W / 2 - 1 || (r.yq >> 24) < W / 2 - 1;
 }
+// The larger component's magnitude as bits (in the order of the magnitudes; 0x7f800000 and up: not finite).
+__device__ __forceinline__ unsigned int value_bits(const SampleRec& r) {
+    return max(__float_as_uint(r.vre) & 0x7fffffffu, __float_as_uint(r.vim) & 0x7fffffffu);
+}
+constexpr unsigned int kNotFinite = 0x7f800000u;
+// The batch's scale is its largest value's, and in a launch over several snapshots a batch may hold the records of
+// two. So that one snapshot's values cannot cost another's records their bits, a record 2^20 times smaller than the
+// largest, or not finite, is rare too (2^-19 of it, 22 bits of all others, is left to the split).
+constexpr unsigned int kScaleSpan = 20u << 23;
 
 // The rare records of the batch [b0, b1), whose keys are `key` or later (returns the last one): exact ES formula,
 // lanes over cells, straight to the planes. Records at one position are summed first: autocorrelations and
@@ -329,7 +338,11 @@ __device__ __forceinline__ int rare_records(const SampleRec* __restrict__ rec, c
     const unsigned int mine = min(b0 + lane, b1 - 1);
     const SampleRec own = rec[mine];
     const float own_s = rec_s ? rec_s[mine] : 0.0f;
-    unsigned int rm = __ballot_sync(0xffffffffu, b0 + lane < b1 && is_rare<W>(own));
+    const bool valid = b0 + lane < b1;
+    const unsigned int own_bits = valid ? value_bits(own) : 0u;
+    const bool plain = valid && !odd_footprint<W>(own) && own_bits < kNotFinite;
+    const unsigned int largest = __reduce_max_sync(0xffffffffu, plain ? own_bits : 0u);
+    unsigned int rm = __ballot_sync(0xffffffffu, valid && !(plain && (own_bits == 0u || own_bits + kScaleSpan >= largest)));
     const long long GG = (long long)G * G;
     while (rm) {
         const int js = __ffs(rm) - 1;
@@ -520,17 +533,17 @@ __global__ void __launch_bounds__(32 * kWarps, min_ctas<KC>()) k_grid_mma(
             const bool valid = b0 + lane < b1;
             const int fxq = r.xq & 0xFFFFFF, fyq = r.yq & 0xFFFFFF;
             const int r0 = (r.xq >> 24) - (HW - 1), c0 = (r.yq >> 24) - (HW - 1);
-            const bool rare = valid && is_rare<W>(r);
-            const bool fast = valid && !rare;
-            const unsigned int vbits =
-                fast ? (__float_as_uint(fmaxf(fabsf(r.vre), fabsf(r.vim))) & 0x7fffffffu) : 0u;
+            unsigned int vbits = valid ? value_bits(r) : 0u;
+            bool fast = valid && !odd_footprint<W>(r) && vbits < kNotFinite;
+            if (!fast) vbits = 0u;
             const unsigned int vmax = __reduce_max_sync(0xffffffffu, vbits);
+            fast = fast && (vbits == 0u || vbits + kScaleSpan >= vmax);
             // |v| 2^se < 2^14
             const int se = max(-110, min(110, 14 - ((int)(vmax >> 23) - 126)));
             const float scale = fast ? __int_as_float((se + 127) << 23) : 0.0f;
             // (1 + 2^-23) 2^-(14 + se): the last bit makes up for the products' truncation towards zero
             const float inv = __uint_as_float(((unsigned int)(127 - 14 - se) << 23) | 1u | neg);
-            if (rare) atomicOr(&st.rare, 1u << ((b0 - c_beg) / 32));
+            if (valid && !fast) atomicOr(&st.rare, 1u << ((b0 - c_beg) / 32));
             if (vmax) {
                 const int oa = fast ? r0 : 0, ob = fast ? c0 : 0;
                 st.oa[lane] = __int2half_rn(oa);
