@@ -222,22 +222,20 @@ __device__ __forceinline__ Runs block_runs(const unsigned int* __restrict__ offs
 // cleared here.
 __global__ void __launch_bounds__(256) k_split_w(const unsigned int* __restrict__ offsets, int G, int nt, int nplanes,
                                                  unsigned int* __restrict__ list, float2* __restrict__ planes) {
-    __shared__ unsigned int parts;
+    __shared__ unsigned int parts, at;
     const int nb = (G + kCells - 1) / kCells;
     for (int b = blockIdx.x; b < nb * nb; b += gridDim.x) {
         const int by = b / nb, bx = b - by * nb;
         if (threadIdx.x == 0) {
             parts = (block_runs(offsets, nt, by, bx).total() + kPart - 1) / kPart;
-            if (parts > 1) {
-                const unsigned int at = atomicAdd(list, parts - 1);
-                for (unsigned int k = 1; k < parts; ++k) {
-                    list[2 * (at + k)] = (unsigned int)b;
-                    list[2 * (at + k) + 1] = k;
-                }
-            }
+            if (parts > 1) at = atomicAdd(list, parts - 1);
         }
         __syncthreads();
         if (parts > 1) {
+            for (unsigned int k = 1 + threadIdx.x; k < parts; k += 256) {
+                list[2 * (at + k)] = (unsigned int)b;
+                list[2 * (at + k) + 1] = k;
+            }
             const int rows = min(kCells, G - by * kCells), cols = min(kCells, G - bx * kCells);
             float2* base = planes + (long long)by * kCells * G + bx * kCells;
             for (int i = threadIdx.x; i < nplanes * kCells * kCells; i += 256) {

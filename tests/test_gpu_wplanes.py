@@ -68,6 +68,18 @@ def test_matches_dft_and_chebyshev_form(cuda_device, N, nchan, rows, kw):
         assert O.rel_rms(at[f], dft[f]) < tol
 
 
+def test_blocks_of_many_parts(cuda_device):
+    """Nine tenths of 240 k samples in a few blocks of cells: each is shared by hundreds of CTAs, beside blocks of one
+    and of none."""
+    s = _snap(256, 8, 30000)
+    uvw = s.uvw.copy()
+    uvw[np.arange(len(uvw)) % 10 != 0] *= np.float32(0.02)
+    img, st, at, dft, ref, rst = _images(dataclasses.replace(s, uvw=uvw), edge_mode=api.EDGE_STRICT)
+    assert st["num_gridded"] == rst["num_gridded"]
+    f = np.isfinite(dft)
+    assert O.rel_rms(at[f], dft[f]) < IMG_TOL
+
+
 def test_one_signed_w_range(cuda_device):
     s = _snap(512, 4, 6000, shift=400.0)
     img, st, at, dft, ref, rst = _images(s, edge_mode=api.EDGE_STRICT)
