@@ -464,6 +464,9 @@ int choose_slabs(svdi_engine* e, bool archive, double r3min, double r3max, doubl
     return SVDI_OK;
 }
 
+// Planes of one transform from which its parts are planned apart (exec_fft_many).
+constexpr int kManyPlanes = 24;
+
 // The inverse 2-D FFT of `batch` moment planes of G x G, pruned to what the recombination reads:
 // every row (length G, contiguous) is transformed, then only the N columns it reads (the checkerboard
 // sign centres the transform, so pixel x reads column G / 2 + x - N / 2: one contiguous run) are
@@ -484,7 +487,7 @@ int make_fft_plan(long long G, long long N, int batch, cudaStream_t st, FftPlan&
         if (batch) SVDI_CUFFT(cufftPlanMany(&plan.rows, 1, &n, &n, 1, n, &n, 1, n, CUFFT_C2C, (int)(G * batch)));
         plan.mode = col_fft_supported(G) ? FftPlan::kRowsSharedCols : FftPlan::kRowsCufftCols;
         if (N && plan.mode == FftPlan::kRowsSharedCols)
-            SVDI_TRY(make_col_fft(G, N * std::max(batch, 1), plan.cp, &plan.d_tw, &plan.d_perm));
+            SVDI_TRY(make_col_fft(G, N * (batch ? batch : kManyPlanes), plan.cp, &plan.d_tw, &plan.d_perm));
         else if (N)
             SVDI_CUFFT(cufftPlanMany(&plan.cols, 1, &n, &n, n, 1, &n, n, 1, CUFFT_C2C, (int)N));
     } else {
@@ -547,7 +550,6 @@ int exec_fft(const FftPlan& plan, cufftComplex* planes, int nplanes) {
 // and the column part serves all of them. `evict`: no graph that uses older plans exists or is being recorded. Plans
 // of fixed sizes put together (64 + 32 + .. planes) need no new ones, but took 23 us more of a 3250 us call (46 planes
 // of 2304^2) and 8 ms more of an engine's first one.
-constexpr int kManyPlanes = 24;
 constexpr size_t kManyPlans = 32;
 int exec_fft_many(svdi_engine* e, long long G, long long N, cufftComplex* planes, int nplanes, bool evict) {
     const auto key = std::make_tuple(G, 0LL, nplanes);
