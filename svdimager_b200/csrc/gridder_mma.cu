@@ -31,9 +31,9 @@
 // the rest per tile), then the L2's reductions (16-byte reductions of 64-byte row pieces add 4.7 TB/s,
 // 8-byte ones of 32-byte pieces 3.3 TB/s: hence the column order of b_row). Gridding stage, B200, against the
 // fixed-point shared-memory gridder (gridder.cu, which keeps supports above 8 and the explicit tile
-// sizes 32 and 64): 6.5 M samples, 2 terms, 3072^2 grid 0.541 -> 0.315 ms; 1.04 M, 2 terms, 1536^2
-// 0.324 -> 0.080 ms; support 6 at 2048^2 0.590 -> 0.098 ms; 130 k samples, 8 terms, 384^2 0.119 ->
-// 0.043 ms; 0.64 M samples, 59 terms, 2304^2 7.7 -> 3.1 ms. Error against 64 bits over 143 random images:
+// sizes 32 and 64): 6.5 M samples, 2 terms, 3072^2 grid 0.541 -> 0.321 ms; 1.04 M, 2 terms, 1536^2
+// 0.324 -> 0.085 ms; support 6 at 2048^2 0.590 -> 0.094 ms; 130 k samples, 8 terms, 384^2 0.119 ->
+// 0.042 ms; 0.64 M samples, 59 terms, 2304^2 7.7 -> 3.1 ms. Error against 64 bits over 143 random images:
 // median 0.86, at most 1.03 of that gridder's.
 #include "svdi_internal.cuh"
 
@@ -145,7 +145,7 @@ __device__ __forceinline__ void taps(const float (&e)[4][5], const float (&o)[4]
 // group's last chunk adds the slot to the plane and leaves it and the group's arrival counter as zeros.
 // Error against 64 bits of dense-core images (0.3 to 0.6 M samples, chunks added singly / through slots): 1.1e-6
 // / 2.8e-7, 1.5e-6 / 5.3e-7, 5.1e-7 / 2.5e-7. Time: the wait for the arrival counter costs 2 us where all is
-// dense (130 k samples, 8 terms: 25 -> 27 us); fewer reductions of one address save 3 % at 6.5 M samples (0.331
+// dense (130 k samples in a few tiles, 8 terms: gridding 25 -> 27 us); fewer reductions of one address save 3 % at 6.5 M samples (0.331
 // -> 0.318 ms).
 struct DenseSlots {
     float4* sums;           // [group][term][kSlotWords]

@@ -98,7 +98,7 @@ struct DevPlan {
 // Stage times of a call with a device plan, taken by its kernels (%globaltimer, ns; the words follow the plan in
 // its buffer): starts of preprocessing, binning, gridding; gridding's end; recombination's start and end. An
 // event between two kernels costs 3 to 4 us of an otherwise idle device, where a kernel follows another in 1 us:
-// with five of them a 192^2 image of 130 k samples took 128 us instead of 115, 1024^2 of 1 M 267 instead of 253.
+// with five of them a 192^2 image of 24 k samples took 128 us instead of 115, 1024^2 of 1 M 267 instead of 253.
 enum { STAMP_PRE, STAMP_BIN, STAMP_GRID, STAMP_FFT, STAMP_IMAGE, STAMP_END, STAMP_COUNT };
 constexpr size_t kPlanBytes = (sizeof(DevPlan) + 15) / 16 * 16 + STAMP_COUNT * sizeof(unsigned long long);
 __host__ __device__ inline unsigned long long* plan_stamps(const DevPlan* plan) {
