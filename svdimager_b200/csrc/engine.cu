@@ -1521,10 +1521,14 @@ std::unique_ptr<svdi_engine> take_idle_engine(int device) {
 
 void give_idle_engine(std::unique_ptr<svdi_engine> e) {
     // The caller's own work on the descriptor's arrays, on whatever stream, ends before another snapshot is written
-    // over them (destroying the engine waits for the device too).
+    // over them: freeing memory waits for the device, as it does where the engine is destroyed (a device
+    // synchronisation would break a graph capture that another thread has in progress).
     int dev = 0;
     const bool have = cudaGetDevice(&dev) == cudaSuccess;
-    const bool idle = cudaSetDevice(e->device) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess;
+    void* marker = nullptr;
+    const bool idle = cudaSetDevice(e->device) == cudaSuccess && cudaMalloc(&marker, 256) == cudaSuccess &&
+                      cudaFree(marker) == cudaSuccess;
+    if (!idle) cudaGetLastError();
     // a new descriptor decides its slab batches by the memory that is free then, and starts without a plan and
     // without the truncation errors found for this one's w range
     e->bslab_cache.clear();

@@ -129,3 +129,44 @@ def test_taken_over_engines_keep_no_answers(cuda_device, cases):
         _two_step(s)
         counts.append(api.kernel_launch_count() - n0)
     assert counts[1:] == counts[:1] * 2, counts
+
+
+def test_freeing_beside_a_capture(cuda_device, cases):
+    """Another thread captures a CUDA graph while a descriptor is freed: the capture is not broken, and the engine
+    is still kept."""
+    import torch
+    s, ref = cases[1]
+    api.release_idle_engines()
+    b = api.preprocess_measurement_set_gpu(s)
+    ptr = b.buf.d_vis_real
+    x = torch.zeros(16, device="cuda")
+    started, freed = threading.Event(), threading.Event()
+    out = []
+
+    def capture():
+        g = torch.cuda.CUDAGraph()
+        try:
+            with torch.cuda.graph(g, capture_error_mode="thread_local"):
+                x.add_(1.0)
+                started.set()
+                freed.wait(20)
+                x.add_(1.0)
+            out.append(g)
+        except Exception as ex:  # noqa: BLE001
+            started.set()
+            out.append(ex)
+
+    t = threading.Thread(target=capture)
+    t.start()
+    started.wait(20)
+    b.free()
+    freed.set()
+    t.join()
+    assert isinstance(out[0], torch.cuda.CUDAGraph), out[0]
+    out[0].replay()
+    torch.cuda.synchronize()
+    assert torch.equal(x, torch.full_like(x, 2.0))
+    c = api.preprocess_measurement_set_gpu(s)
+    assert c.buf.d_vis_real == ptr  # the kept engine's arrays
+    assert O.rel_rms(api.FIpipeDevice(c, s.image_size, s.cell_size), ref) < 1e-6
+    c.free()
