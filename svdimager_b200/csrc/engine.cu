@@ -252,6 +252,7 @@ struct svdi_engine {
     // pageable host uploads and image downloads of the archive entry and the host-input call
     svdi::HostStager stager;
     bool batch_bound = false;  // it holds a batch
+    svdi_engine** batch_slot = nullptr;  // that batch's pointer to this engine, cleared when the engine goes first
     // A chained batch's graph runs on this engine's buffers: until the batch is destroyed, other calls of the
     // engine leave the allocations it refers to where they are (those they outgrow wait in `kept`).
     bool graph_bound = false;
@@ -279,7 +280,9 @@ struct svdi_engine {
     }
 
     ~svdi_engine() {
+        if (batch_slot) *batch_slot = nullptr;
         if (device >= 0) cudaSetDevice(device);
+        for (void* p : kept) cudaFree(p);
         for (auto& kv : plans) svdi::destroy_fft_plan(kv.second);
         for (auto& e : ev)
             if (e) cudaEventDestroy(e);
@@ -1988,6 +1991,7 @@ struct svdi_batch {
             std::lock_guard<std::mutex> lk(e->mu);
             e->bind_graph(false);
             e->batch_bound = false;
+            e->batch_slot = nullptr;
         }
     }
 };
@@ -2338,6 +2342,7 @@ int batch_create_one(svdi_engine* e, const svdi_host_ms* snapshots, size_t num_s
     const int wrc = wide_capture(b.get());
     if (wrc == SVDI_OK) {
         e->batch_bound = true;
+        e->batch_slot = &b->e;
         *out = b.release();
         return SVDI_OK;
     }
@@ -2368,6 +2373,7 @@ int batch_create_one(svdi_engine* e, const svdi_host_ms* snapshots, size_t num_s
     SVDI_CUDA(cudaGraphInstantiate(&b->exec, b->graph, 0));
     b->e = e;
     e->batch_bound = true;
+    e->batch_slot = &b->e;
     e->bind_graph(true);
     // the correction table is uploaded on the host's side, so the graph's own one goes with the batch
     std::swap(b->corr, e->corr);
@@ -2422,8 +2428,8 @@ int svdi_batch_create(svdi_engine* e, const svdi_host_ms* snapshots, size_t num_
 int svdi_batch_launch(svdi_batch* b, void* cuda_stream) {
     using namespace svdi;
     g_last_error.clear();
-    if (!b || !b->exec) {
-        set_error("null batch");
+    if (!b || !b->exec || !b->e) {
+        set_error(b && b->exec ? "the batch's engine is gone" : "null batch");
         return SVDI_ERR_INVALID_ARGUMENT;
     }
     SVDI_CUDA(cudaSetDevice(b->e->device));
@@ -2446,8 +2452,8 @@ int svdi_batch_launch(svdi_batch* b, void* cuda_stream) {
 int svdi_batch_check(svdi_batch* b) {
     using namespace svdi;
     g_last_error.clear();
-    if (!b) {
-        set_error("null batch");
+    if (!b || !b->e) {
+        set_error(b ? "the batch's engine is gone" : "null batch");
         return SVDI_ERR_INVALID_ARGUMENT;
     }
     SVDI_CUDA(cudaSetDevice(b->e->device));

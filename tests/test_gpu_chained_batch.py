@@ -43,3 +43,23 @@ def test_images_between_launches(cuda_device):
                 assert O.rel_rms(imgs.cpu().numpy(), first) < 1e-6
         e.image_device(descs[0], N, cell, one.data_ptr())  # after the batch: through w planes again
         assert O.rel_rms(one.cpu().numpy(), ref) < 1e-6
+
+
+@pytest.mark.parametrize("slabs", [0, 1])
+def test_engine_closed_before_its_batch(cuda_device, slabs):
+    """A batch that outlives its engine refuses to launch and can be destroyed (wide and chained)."""
+    import torch
+    N = 256
+    opt = dict(k_rule=api.KRULE_TARGET, target_error=1e-6, edge_mode=api.EDGE_STRICT, max_batch_slabs=slabs)
+    snaps = [snapshot("widefield", nchan=4, n_rows_limit=r, image_size=N, cell_size=0.3 / N) for r in (3000, 2500)]
+    keep, descs = _upload(snaps, torch)
+    imgs = torch.zeros((2, N, N), device="cuda")
+    e = api.Engine(**opt)
+    b = api.Batch(e, descs, N, 0.3 / N, imgs.data_ptr())
+    assert b.wide == (slabs == 0)
+    e.close()
+    for call in (b.launch, b.check):
+        with pytest.raises(api.SvdiError) as ei:
+            call()
+        assert ei.value.status == 1
+    b.close()
